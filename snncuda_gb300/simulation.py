@@ -12,6 +12,7 @@ std::runtime_error).
 
 from __future__ import annotations
 
+import array
 import ctypes
 import os
 import pathlib
@@ -500,9 +501,10 @@ class Readout:
     def _samples(samples):
         ptr = np.zeros(len(samples) + 1, np.uint64)
         ptr[1:] = np.cumsum([len(s) for s in samples])
-        n = np.ascontiguousarray([int(a) for s in samples for a, _ in s] or [0], np.uint32)
-        w = np.ascontiguousarray([float(b) for s in samples for _, b in s] or [0.0], np.float32)
-        return ptr, n, w
+        # array.array converts a list of Python numbers in half the time numpy takes
+        n = array.array("I", [int(a) for s in samples for a, _ in s] or [0])
+        w = array.array("f", [float(b) for s in samples for _, b in s] or [0.0])
+        return ptr, np.frombuffer(n, np.uint32), np.frombuffer(w, np.float32)
 
     def feedforward(self, samples, readouts):
         """(scores [samples, readouts] float32, spikes uint64, delivered per sample)."""
