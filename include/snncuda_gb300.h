@@ -238,16 +238,16 @@ int snncuda_sim_read_raster(snncuda_sim* sim, uint64_t first, uint64_t count, ui
  * (CudaBackend.cu).  snncuda_sim_autotune runs the simulation's next ticks
  * in timed probes of probe_ticks ticks (each probe first runs up to one
  * captured graph of ticks untimed) and keeps, per knob, the fastest of a few
- * candidates: blocks of the synapse-event kernel (events per warp), of the
- * per-target walk, of the grouping and of the temporal update, and the ticks
- * per captured graph; then it shrinks the wheel-slot capacity to twice the
+ * candidates: blocks of the synapse-event kernel, of the grouping and of the
+ * temporal update, and the ticks per captured graph; then it shrinks the wheel-slot capacity to twice the
  * largest per-tick due list seen plus 2^16 events when that saves a quarter
  * or more of it.  The probed ticks are ordinary ticks of the simulation and
  * launch shapes never change results.  Threads per block stay 256: the
  * kernels' shared-memory layouts are built for it, and blocks per SM (the
  * knobs above) are the occupancy lever. */
 typedef struct snncuda_tuning {
-    uint32_t grid_events, grid_walk, grid_bucket, grid_temporal;  /* blocks */
+    uint32_t grid_events, grid_walk, grid_bucket, grid_temporal;  /* blocks (grid_walk: without effect,
+                                       the synapse-event kernel walks its own targets) */
     uint32_t ticks_per_graph;
     uint32_t block_threads;
     uint64_t slot_event_capacity;   /* after tuning */

@@ -74,7 +74,7 @@ struct alignas(64) SynAB {
     SynB b;
 };
 
-// Per-event input of the neuron walk, written by k_events in due order inside
+// Per-event input of the neuron walk, in due order inside
 // every target's group: the weight after the event's pre-spike STDP (computed
 // as if the target had not fired earlier in the tick), compartment, receptor
 // and flags, the synapse and the due position.
@@ -113,7 +113,7 @@ struct alignas(64) NeuronRec {
     uint32_t last_fired1;  // last_fired_tick + 1, 0 = none
     uint32_t last_active;
     uint32_t flags;        // 4 x 2-bit tau code
-    // temporal pattern fields (written by k_temporal only)
+    // temporal pattern fields
     uint32_t match_count;
     uint32_t ws;           // temporal window_start_tick
     uint32_t len;          // spike_offsets.size()
@@ -214,7 +214,7 @@ struct Engine {
     uint32_t fire_cap;
     uint32_t fire_tiles_cap;
     float min_weight;
-    unsigned long long stage_wait_ns;  // limit of k_process's wait for its staged event inputs
+    unsigned long long stage_wait_ns;  // limit of a block's wait for a staging copy
 
     // network
     const unsigned long long* in_ptr;      // [N+1] target-major row pointers
@@ -247,11 +247,12 @@ struct Engine {
     // so the lines of grp_tmp being filled stay in L2 until
     // complete instead of going to DRAM half-written.
     uint32_t scatter_pass_events;
-    // 1: k_temporal and k_post run on the main stream in tick order instead
-    // of on the side stream beside k_events / k_process and beside the fire
-    // ordering (two random-access kernels side by side can take longer than
-    // one after the other).
+    // 1: k_post and k_temporal run on the main stream in tick order instead
+    // of on the side stream beside the fire ordering (two random-access
+    // kernels side by side can take longer than one after the other).
     uint32_t side_serial;
+    uint32_t inline_codes;                 // 1: inline_code_pattern holds for every target
+    uint32_t multi_refs;                   // 1: some target keeps several reference patterns (k_temporal runs)
     uint32_t* bcnt;                        // [grid_bucket][nbuckets] events of each (chunk, bucket)
     uint32_t* btot;                        // [nbuckets] events per bucket (zero between ticks)
     uint32_t* bstart;                      // [nbuckets + 1] first grouped position of each bucket
@@ -260,7 +261,7 @@ struct Engine {
     unsigned long long* grp;               // [slot_cap] due events grouped by target, due order inside
                                            // a target: (payload << 32) | (due index | ext << 31)
     BucketEntry* grp_tmp;                  // [slot_cap] the due events in bucket order (unsorted inside)
-    EvIn* evin;                            // [slot_cap] per-event inputs of k_process, grouped, due order
+    EvIn* evin;                            // [slot_cap] event inputs of buckets grouped in grp, due order
     SynPre* ev_a0;                         // [slot_cap] each synaptic event's changing fields before it
     uint32_t* fire_bits;                   // [slot_cap/32] bitmap of due positions that fired
     uint32_t* fire_at;                     // [slot_cap] firing neuron at a due position
@@ -281,12 +282,12 @@ struct Engine {
     Tables tab;
 
     // launch shapes (results do not depend on them; snncuda_sim_autotune
-    // picks grid_events, grid_walk, grid_bucket and grid_process)
+    // picks grid_events, grid_bucket and grid_process)
     uint32_t grid_wide;
     uint32_t grid_process;  // k_temporal blocks
-    uint32_t grid_walk;     // k_process blocks
+    uint32_t grid_walk;     // (a tuning field without effect: k_events walks its own targets)
     uint32_t grid_fire;
-    uint32_t grid_events;   // k_events blocks
+    uint32_t grid_events;   // k_events blocks at most (one per bucket)
 };
 
 constexpr uint32_t kMaxBuckets = 16384;   // target buckets of the grouping (shared-memory counters)
@@ -300,13 +301,28 @@ __host__ __device__ inline uint32_t bucket_shift_for(uint32_t N) {
     while (((static_cast<unsigned long long>(N) + (1ull << s) - 1) >> s) > kMaxBuckets) ++s;
     return s <= kMaxBucketShift ? s : 0;
 }
+// The tick's buckets may be more and narrower than bucket_shift_for's:
+// k_events takes a block per bucket, and 64 targets' events (about 12 per
+// target and tick on the dense workloads, 800 of the 1,280 a block's shared
+// memory holds) were the best fit there: 128 targets with twice the threads
+// took 273 us where 64 took 219 (recog_1m distributions at 200,000 neurons).
+// 32 targets where 64 would leave fewer than three blocks per SM.  Wider only
+// when there would be more than kMaxTickBuckets buckets (their counters fill
+// the placing blocks' shared memory).
+constexpr uint32_t kMaxTickBuckets = 32768;
+inline uint32_t tick_bucket_shift(uint32_t N, uint32_t sms) {
+    if (bucket_shift_for(N) == 0) return 0;
+    uint32_t s = (N >> 6) < 3 * sms ? 5 : 6;
+    while (((static_cast<unsigned long long>(N) + (1ull << s) - 1) >> s) > kMaxTickBuckets) ++s;
+    return s;
+}
 constexpr int kExpandFires = 8;          // fires per expansion block (one warp each)
 constexpr uint32_t kMaxClasses = 256;    // distinct delivery delays
 
 // Host-side launchers (kernels.cu).
 // `marks` (optional) holds 2 * kKernelCount events recorded around every
 // kernel (before, after) for profiling graphs.
-constexpr int kKernelCount = 10;
+constexpr int kKernelCount = 8;
 // The streams of a tick: k_temporal and k_post run on `side`, forked from
 // `main` with ev[0] / ev[2] and joined back with ev[1] / ev[3].
 struct TickStreams {
@@ -336,7 +352,7 @@ void launch_range_counts(const Engine& e, uint32_t n_begin, uint32_t n_end, unsi
 // (k_checksum); out must start at zero.
 void launch_checksum(const Engine& e, uint32_t n_begin, uint32_t n_end, unsigned long long tm_begin,
                      unsigned long long* out, cudaStream_t stream);
-// One-time kernel attributes (dynamic shared memory of k_process); call with
+// One-time kernel attributes (dynamic shared memory); call with
 // the device current before the first tick.
 void configure_kernels();
 // Builds the synapse records from SynA images (`a`, S entries): code-pattern

@@ -9,30 +9,27 @@
 //                   chunk of the due list (and copy far-future injections
 //                   that become reachable into the wheel)
 //  2. k_bscatter   bucket starts; place every event in its bucket
-//  3. k_bsort      per bucket: group by target, segment starts
-//  4. k_events     one warp per target with events: restore due order inside
-//                  its group, then per synapse (lanes in parallel) the event's
-//                  pre-spike STDP, pre-spike count and spike-code pattern
-//                  (SynapseDendriteProcessor.cpp:104-133, :318-365); writes
-//                  each event's input for the neuron walk
-//  5. k_process    one thread per touched target: the neuron's physics over
-//                  its events in due order (:175-229), redoing the STDP of
-//                  events that follow a fire of the target; fires into a
-//                  due-position bitmap
-//  6. k_fire_list  fires in due order (= reference fire order), raster
-//  7. k_fire_count events per (fire block, delay class); the last block scans
+//  3. k_events     a block per bucket: its events grouped by target in due
+//                   order in shared memory, then per synapse the event's
+//                   pre-spike STDP, pre-spike count and spike-code pattern
+//                   (SynapseDendriteProcessor.cpp:104-133, :318-365), per
+//                   target the neuron's physics over its events in due order
+//                   (:175-229), redoing the STDP of events that follow a fire
+//                   of the target, and its temporal pattern (:294-316); fires
+//                   into a due-position bitmap
+//  4. k_fire_list  fires in due order (= reference fire order), raster
+//  5. k_fire_count events per (fire block, delay class); the last block scans
 //                  destinations and finishes the tick
-//  8. k_expand     copy each fire's pre-expanded (synapse, offset) events into
+//  6. k_expand     copy each fire's pre-expanded (synapse, offset) events into
 //                  their delivery slots, order-preserving
 //
-// and two more, on a second stream (graph fork/join) beside the others, or
-// for networks of 2^26+ synapses on the main stream in tick order
-// (Engine::side_serial):
+// and two more, on a second stream (graph fork/join) beside 4-6, or for
+// networks of 2^26+ synapses on the main stream after 3 (Engine::side_serial):
 //
-//  9. k_temporal   the neuron temporal pattern of every touched target, once
-//                  per tick, beside 4-5 (or before 4)
-// 10. k_post       post-spike STDP over the in-rows of targets that fired
-//                  (:138-173), beside 6-8 (or after 5)
+//  7. k_post       post-spike STDP over the in-rows of targets that fired
+//                  (:138-173)
+//  8. k_temporal   the neuron temporal pattern of touched targets that keep
+//                  several reference patterns (networks that have any)
 //
 // Main-stream kernels that directly follow another are launched as
 // programmatic dependents (tick_enter), so each is scheduled while the one
@@ -40,13 +37,16 @@
 //
 // Every wait is a kernel boundary (a programmatic dependent's grid
 // dependency wait included), a "last block" hand-off (an atomic counter, no
-// spinning) or the time-bounded mbarrier wait of k_process's staging copy,
-// so no kernel here can hang.
+// spinning) or the time-bounded mbarrier wait of a staging copy, so no kernel
+// here can hang.
 // Float arithmetic uses explicitly rounded intrinsics so nothing is
 // contracted into an FMA: each operation rounds exactly as the reference's
 // separately evaluated float expressions.
 
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "engine.h"
 
@@ -54,18 +54,14 @@ namespace snngb {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr uint32_t kStageEvents = 3584;  // event inputs k_process stages per block (56 KB)
-constexpr uint32_t kLtpShared = 2560;    // longest LTP table k_process copies to shared memory (10 KB)
-constexpr size_t kProcessSmem = kStageEvents * sizeof(EvIn) + kLtpShared * sizeof(float);
 constexpr int kFireCountThreads = 1024;  // k_fire_count's last block scans up to 32 delay classes at once
 
-// Minimum resident blocks per SM requested for k_process and k_events
-// (register budget).
-#ifndef SNNGB_PROCESS_MIN_BLOCKS
-#define SNNGB_PROCESS_MIN_BLOCKS 3
+// Minimum resident blocks per SM requested for k_events (register budget).
+#ifndef SNNGB_EVENT_THREADS
+#define SNNGB_EVENT_THREADS 128
 #endif
 #ifndef SNNGB_EVENTS_MIN_BLOCKS
-#define SNNGB_EVENTS_MIN_BLOCKS 4
+#define SNNGB_EVENTS_MIN_BLOCKS 5
 #endif
 
 __device__ __forceinline__ float rec_gain(uint32_t r) { return r == 1 ? 0.55f : (r == 3 ? 0.65f : 1.0f); }
@@ -235,6 +231,17 @@ __device__ __forceinline__ bool cos_ge(unsigned long long dot, unsigned long lon
     return cos_ge_exact(dot, rn, cn, sim);
 }
 
+// cos_ge for sums that fit 32 bits: rn and cn share one reciprocal square root
+// (their product stays below 2^64; the estimate's relative error stays below
+// 1e-6).
+__device__ __forceinline__ bool cos_ge_u32(uint32_t dot, uint32_t rn, uint32_t cn, float sim) {
+    if (rn == 0 || cn == 0) return false;  // similarity 0.0f < sim
+    const float est = __fmul_rn(__uint2float_rn(dot), rsqrtf(__fmul_rn(__uint2float_rn(rn), __uint2float_rn(cn))));
+    if (est >= sim * 1.00002f) return true;
+    if (est <= sim * 0.99998f) return false;
+    return cos_ge_exact(dot, rn, cn, sim);
+}
+
 // (a + b) mod m for a < m and b <= m, without an integer division.
 __device__ __forceinline__ uint32_t wrap_add(uint32_t a, uint32_t b, uint32_t m) {
     const uint32_t x = a + b;
@@ -244,7 +251,7 @@ __device__ __forceinline__ uint32_t wrap_add(uint32_t a, uint32_t b, uint32_t m)
 struct NState {
     float cur[4];
     uint32_t upd[4];
-    uint32_t flags;  // tau codes (2 bits each); in k_temporal: last_match << 8
+    uint32_t flags;  // tau codes (2 bits each); in temporal_tick: last_match << 8
     float membrane;
     uint32_t spikes, last_fired1, last_active, match_count, ws, len;
     unsigned long long cn;
@@ -275,66 +282,46 @@ __device__ __forceinline__ float decay_factor(const Tables& tb, uint32_t code, u
 // pass.  Once no learned pattern is still being compared element by element
 // and a cached result already matches, every remaining append matches too
 // (the sums are frozen), which makes the common case O(1) per tick.
-// kOne: max_reference_patterns == 1, the single pattern lives in s.one.
-template <bool kOne>
-__device__ void temporal_tick(NState& s, const NeuronParam& p, uint32_t t, const Engine& e, int enabled,
-                              uint32_t k) {
+//
+// Targets that keep one reference pattern, a thread each: the pattern lives in
+// s.one.
+__device__ void temporal_tick(NState& s, const NeuronParam& p, uint32_t t, const Engine& e, int enabled, uint32_t k) {
     if (k == 0) return;
     if (!enabled) {
         s.flags &= ~(1u << 8);
         return;
     }
     unsigned long long* cand = e.cand + p.cand_base;
-    RefMeta* meta = e.refmeta + p.meta_base;
     unsigned long long* ring = e.ring + p.ring_base;
-    auto ref = [&](uint32_t r) -> RefMeta& {
-        if constexpr (kOne) {
-            return s.one;
-        } else {
-            return meta[wrap_add(s.ref_head, r, p.max_refs)];
-        }
-    };
+    RefMeta& m = s.one;
     if (s.len == 0 || t - s.ws > p.window) {
         s.ws = t;
         s.len = 0;
         s.nruns = 0;
         s.cn = 0;
-        for (uint32_t r = 0; r < s.ref_count; ++r) {
-            RefMeta& m = ref(r);
-            m.dot = 0;
-            m.rn = 0;
-            m.cn = 0;
-            m.cur_run = 0;
-            m.cur_pos = 0;
-            m.match = 2;
-        }
+        m.dot = 0;
+        m.rn = 0;
+        m.cn = 0;
+        m.cur_run = 0;
+        m.cur_pos = 0;
+        m.match = 2;
     }
     const uint32_t o = t - s.ws;
     const uint32_t oo = o * o;  // o < 2^16, so o * o fits 32 bits
+    auto matches = [&]() {
+        if (0.0f >= p.similarity) return true;
+        if (m.match == 2) m.match = cos_ge(m.dot, m.rn, m.cn, p.similarity) ? 1 : 0;
+        return m.match == 1;
+    };
     for (uint32_t j = 0; j < k; ++j) {
-        if (s.len >= 1 && s.ref_count > 0 && s.nruns > 0 && run_value(s.last_run) == o) {
-            bool frozen = true;
-            bool hit = 0.0f >= p.similarity;
-            for (uint32_t r = 0; r < s.ref_count; ++r) {
-                RefMeta& m = ref(r);
-                if (s.len + 1 <= m.len) {
-                    frozen = false;
-                    break;
-                }
-                if (!hit) {
-                    if (m.match == 2) m.match = cos_ge(m.dot, m.rn, m.cn, p.similarity) ? 1 : 0;
-                    hit = m.match == 1;
-                }
-            }
-            if (frozen && hit) {
-                const uint32_t n = k - j;
-                s.last_run += static_cast<unsigned long long>(n) << 16;
-                s.len += n;
-                s.cn += static_cast<unsigned long long>(oo) * n;
-                s.match_count += n;
-                s.flags |= (1u << 8);
-                return;
-            }
+        if (s.len >= 1 && s.ref_count > 0 && s.nruns > 0 && run_value(s.last_run) == o && s.len >= m.len && matches()) {
+            const uint32_t n = k - j;
+            s.last_run += static_cast<unsigned long long>(n) << 16;
+            s.len += n;
+            s.cn += static_cast<unsigned long long>(oo) * n;
+            s.match_count += n;
+            s.flags |= (1u << 8);
+            return;
         }
         // one append (spike_offsets.push_back, :309)
         if (s.nruns > 0 && run_value(s.last_run) == o) {
@@ -350,62 +337,40 @@ __device__ void temporal_tick(NState& s, const NeuronParam& p, uint32_t t, const
         }
         s.len += 1;
         s.cn += oo;
-        for (uint32_t r = 0; r < s.ref_count; ++r) {
-            RefMeta& m = ref(r);
-            if (s.len <= m.len) {
-                const unsigned long long run = ring[wrap_add(m.start, m.cur_run, p.ring_cap)];
-                const unsigned long long v = run_value(run);
-                if (++m.cur_pos == run_count(run)) {
-                    m.cur_run += 1;
-                    m.cur_pos = 0;
-                }
-                m.dot += static_cast<uint32_t>(v) * o;  // 16-bit values: 32-bit products
-                m.rn += static_cast<uint32_t>(v) * static_cast<uint32_t>(v);
-                m.cn += oo;
-                m.match = 2;
+        if (s.ref_count > 0 && s.len <= m.len) {
+            const unsigned long long run = ring[wrap_add(m.start, m.cur_run, p.ring_cap)];
+            const uint32_t v = run_value(run);
+            if (++m.cur_pos == run_count(run)) {
+                m.cur_run += 1;
+                m.cur_pos = 0;
             }
+            m.dot += v * o;  // 16-bit values: 32-bit products
+            m.rn += v * v;
+            m.cn += oo;
+            m.match = 2;
         }
-        bool match = false;
-        if (s.ref_count > 0 && s.len >= 2) {
-            if (0.0f >= p.similarity) {
-                match = true;
-            } else {
-                for (uint32_t r = 0; r < s.ref_count && !match; ++r) {
-                    RefMeta& m = ref(r);
-                    if (m.match == 2) m.match = cos_ge(m.dot, m.rn, m.cn, p.similarity) ? 1 : 0;
-                    match = m.match == 1;
-                }
-            }
-        }
-        if (match) {
+        if (s.ref_count > 0 && s.len >= 2 && matches()) {
             s.flags |= (1u << 8);
             s.match_count += 1;
             continue;
         }
         s.flags &= ~(1u << 8);
         if (s.len < 2) continue;
-        // learn_pattern (:31-41): FIFO with max_reference_patterns entries.
-        if (s.ref_count >= p.max_refs) {
-            s.ring_used -= ref(0).nruns;
-            s.ref_head = wrap_add(s.ref_head, 1, p.max_refs);
-            s.ref_count -= 1;
+        // learn_pattern (:31-41): the window takes the one pattern's place
+        if (s.ref_count > 0) {
+            s.ring_used -= m.nruns;
+            s.ref_count = 0;
         }
         if (s.ring_used + s.nruns > p.ring_cap) {
             raise_status(e, kStatusRingOverflow);
             return;
         }
+        s.snap_pending = true;
+        s.snap_nruns = s.nruns;
+        s.snap_last = s.last_run;
         const uint32_t start = s.ring_head;
-        if constexpr (kOne) {
-            s.snap_pending = true;
-            s.snap_nruns = s.nruns;
-            s.snap_last = s.last_run;
-        } else {
-            cand[s.nruns - 1] = s.last_run;
-            for (uint32_t i = 0; i < s.nruns; ++i) ring[wrap_add(start, i, p.ring_cap)] = cand[i];
-        }
         s.ring_head = wrap_add(start, s.nruns, p.ring_cap);
         s.ring_used += s.nruns;
-        RefMeta& m = ref(s.ref_count);
         m.dot = s.cn;
         m.rn = s.cn;
         m.cn = s.cn;
@@ -415,7 +380,7 @@ __device__ void temporal_tick(NState& s, const NeuronParam& p, uint32_t t, const
         m.cur_run = 0;
         m.cur_pos = 0;
         m.match = 2;
-        s.ref_count += 1;
+        s.ref_count = 1;
     }
 }
 
@@ -470,18 +435,14 @@ __device__ __forceinline__ bool process_input(NState& s, float threshold, uint32
 
 // StdpRule::weight_delta + apply (STDP.cpp:20-40) and the update bookkeeping
 // of SynapseDendriteProcessor.cpp:108-122 / :158-172.  `ltp` is the LTP delta
-// table (e.tab.ltp, or k_process's copy of it in shared memory).
-__device__ void stdp_apply(SynA& a, uint32_t pre, uint32_t post, const Engine& e, int stdp, const float* ltp) {
+// table.
+__device__ __forceinline__ void stdp_apply(SynA& a, uint32_t pre, uint32_t post, const Engine& e, int stdp, const float* ltp) {
     const float before = a.weight;
     float delta = 0.0f;
-    if (stdp && !((a.meta >> kMetaRuleOffBit) & 1u)) {
-        if (post > pre) {
-            const uint32_t dt = post - pre;
-            delta = ltp[dt < e.tab.stdp_len ? dt : e.tab.stdp_len - 1];
-        } else if (post < pre) {
-            const uint32_t dt = pre - post;
-            delta = e.tab.ltd[dt < e.tab.stdp_len ? dt : e.tab.stdp_len - 1];
-        }
+    if (stdp && !((a.meta >> kMetaRuleOffBit) & 1u) && post != pre) {
+        const float* table = post > pre ? ltp : e.tab.ltd;
+        const uint32_t dt = post > pre ? post - pre : pre - post;
+        delta = table[dt < e.tab.stdp_len ? dt : e.tab.stdp_len - 1];
     }
     float v = __fadd_rn(a.weight, delta);
     v = v < e.min_weight ? e.min_weight : (a.clamp_hi < v ? a.clamp_hi : v);
@@ -504,6 +465,14 @@ __device__ __forceinline__ bool post_catch_up(SynA& a, uint32_t t, uint32_t fire
     a.post_cnt = fires;
     return true;
 }
+
+// The parameters of a target that its events and its walk need.
+struct TargetParam {
+    float threshold;
+    uint32_t window;
+    float similarity;
+    uint32_t max_refs;
+};
 
 __device__ __forceinline__ void ring_set(unsigned long long& lo, unsigned long long& hi, uint32_t j,
                                          uint32_t v) {
@@ -554,61 +523,72 @@ __device__ __forceinline__ void store_pattern(uint16_t* pat, uint32_t stride, un
 // held in two 64-bit words.  `inline_pattern`: the target keeps one reference
 // pattern and codes have at most 4 offsets, so the single learned code
 // pattern is stored in ring_hi instead of the pattern pool.
-// Sum of the squares / of the products of four 16-bit lanes (offsets below
-// 2^16: every product fits 32 bits).
-__device__ __forceinline__ unsigned long long lanes_dot(unsigned long long a, unsigned long long b) {
-    const uint32_t a0 = static_cast<uint32_t>(a), a1 = static_cast<uint32_t>(a >> 32);
-    const uint32_t b0 = static_cast<uint32_t>(b), b1 = static_cast<uint32_t>(b >> 32);
-    return static_cast<unsigned long long>((a0 & 0xFFFFu) * (b0 & 0xFFFFu)) + ((a0 >> 16) * (b0 >> 16)) +
-           static_cast<unsigned long long>((a1 & 0xFFFFu) * (b1 & 0xFFFFu)) + ((a1 >> 16) * (b1 >> 16));
+// Four 16-bit offsets in two words.
+struct Lanes {
+    uint32_t a, b;
+};
+
+// Sum of the products of four 16-bit lanes.  kWide: offsets up to 65,535 (a
+// 64-bit sum); otherwise below 2^15, where four products fit 32 bits.
+template <bool kWide>
+__device__ __forceinline__ auto lanes_dot(Lanes x, Lanes y) {
+    using Sum = std::conditional_t<kWide, unsigned long long, uint32_t>;
+    return static_cast<Sum>((x.a & 0xFFFFu) * (y.a & 0xFFFFu)) + static_cast<Sum>((x.a >> 16) * (y.a >> 16)) +
+           static_cast<Sum>((x.b & 0xFFFFu) * (y.b & 0xFFFFu)) + static_cast<Sum>((x.b >> 16) * (y.b >> 16));
 }
 
-// code_update for inline_code_pattern (one reference pattern, at most 4
-// offsets): the window is the four 16-bit lanes of ring_lo, the learned
-// pattern those of ring_hi; lanes at or above `expected` are always zero, so
-// the sums run over all four lanes.
+// SynapseDendriteProcessor.cpp:318-365 for inline_code_pattern (one reference
+// pattern, at most 4 offsets): the window is the four 16-bit lanes of ring_lo,
+// the learned pattern those of ring_hi; lanes at or above `expected` are
+// always zero, so the sums run over all four lanes.
 __device__ __forceinline__ void code_update_inline(SynB& b, uint32_t window, float sim, uint32_t t) {
-    b.flags &= 0xF0u;  // last_code_match = false
-    if (b.code_len == 0 || t - b.code_ws > window) {
+    uint32_t flags = b.flags & 0xF0u;  // last_code_match = false
+    uint32_t len = b.code_len;
+    const uint32_t expected = flags >> 4;
+    if (len == 0 || t - b.code_ws > window) {
         b.code_ws = t;
-        b.code_len = 0;
+        len = 0;
     }
-    const uint32_t o = t - b.code_ws;
-    const uint32_t expected = b.flags >> 4;
-    if (b.code_len < expected) {
-        const int sh = 16 * b.code_len;
-        b.ring_lo = (b.ring_lo & ~(0xFFFFull << sh)) | (static_cast<unsigned long long>(o) << sh);
-        b.code_len += 1;
-        if (b.code_len < expected) return;
+    const uint32_t o = t - b.code_ws;  // at most `window`
+    Lanes x{static_cast<uint32_t>(b.ring_lo), static_cast<uint32_t>(b.ring_lo >> 32)};
+    uint32_t at = len;  // the new offset's lane
+    if (len < expected) {
+        ++len;
     } else {
-        const int sh = 16 * (expected - 1);
-        b.ring_lo = ((b.ring_lo >> 16) & ~(0xFFFFull << sh)) | (static_cast<unsigned long long>(o) << sh);
+        x.a = __byte_perm(x.a, x.b, 0x5432);
+        x.b >>= 16;
+        at = expected - 1;
     }
-    bool match = 0.0f >= sim;
-    if (!match && b.learned_count > 0)
-        match = cos_ge(lanes_dot(b.ring_hi, b.ring_lo), lanes_dot(b.ring_hi, b.ring_hi),
-                       lanes_dot(b.ring_lo, b.ring_lo), sim);
-    if (match) {
-        b.code_matches += 1;
-        b.flags |= 1u;
-        return;
+    const uint32_t put = (at & 1u) ? 0x5410u : 0x3254u;  // o into the upper or the lower half
+    x.a = at < 2 ? __byte_perm(x.a, o, put) : x.a;
+    x.b = at < 2 ? x.b : __byte_perm(x.b, o, put);
+    b.ring_lo = (static_cast<unsigned long long>(x.b) << 32) | x.a;
+    b.code_len = static_cast<uint8_t>(len);
+    if (len >= expected) {
+        bool match = 0.0f >= sim;
+        if (!match && b.learned_count > 0) {
+            const Lanes y{static_cast<uint32_t>(b.ring_hi), static_cast<uint32_t>(b.ring_hi >> 32)};
+            if (window < (1u << 15)) {
+                match = cos_ge_u32(lanes_dot<false>(y, x), lanes_dot<false>(y, y), lanes_dot<false>(x, x), sim);
+            } else {
+                match = cos_ge(lanes_dot<true>(y, x), lanes_dot<true>(y, y), lanes_dot<true>(x, x), sim);
+            }
+        }
+        if (match) {
+            b.code_matches += 1;
+            flags |= 1u;
+        } else {
+            b.ring_hi = b.ring_lo;
+            b.learned_count = 1;
+        }
     }
-    b.ring_hi = b.ring_lo;
-    b.learned_count = 1;
+    b.flags = static_cast<uint8_t>(flags);
 }
 
-__device__ void code_update(SynB& b, const NeuronParam& p, uint32_t t, uint16_t* lc, uint32_t stride, int enabled,
-                            bool inline_pattern) {
-    if (inline_pattern) {
-        if (enabled) {
-            code_update_inline(b, p.window, p.similarity, t);
-        } else {
-            b.flags &= 0xF0u;
-        }
-        return;
-    }
+// code_update for the pattern pool (`lc`: the synapse's learned patterns, up
+// to p.max_refs of `stride` offsets each).
+__device__ void code_update_pool(SynB& b, const TargetParam& p, uint32_t t, uint16_t* lc, uint32_t stride) {
     b.flags &= 0xF0u;  // last_code_match = false
-    if (!enabled) return;
     if (b.code_len == 0 || t - b.code_ws > p.window) {
         b.code_ws = t;
         b.code_len = 0;
@@ -618,9 +598,6 @@ __device__ void code_update(SynB& b, const NeuronParam& p, uint32_t t, uint16_t*
     if (b.code_len < expected) {
         ring_set(b.ring_lo, b.ring_hi, b.code_len, o);
         b.code_len += 1;
-    } else if (inline_pattern) {  // keep the last `expected` offsets (all in ring_lo)
-        b.ring_lo >>= 16;
-        ring_set(b.ring_lo, b.ring_hi, expected - 1, o);
     } else {
         b.ring_lo = (b.ring_lo >> 16) | (b.ring_hi << 48);
         b.ring_hi >>= 16;
@@ -630,20 +607,16 @@ __device__ void code_update(SynB& b, const NeuronParam& p, uint32_t t, uint16_t*
     bool match = 0.0f >= p.similarity;
     unsigned long long cn = 0;
     for (uint32_t j = 0; j < expected; ++j) {
-        const uint32_t v = ring_get(b.ring_lo, inline_pattern ? 0ull : b.ring_hi, j);
+        const uint32_t v = ring_get(b.ring_lo, b.ring_hi, j);
         cn += v * v;  // 16-bit offsets: 32-bit products, 64-bit sums
     }
     for (uint32_t i = 0; i < b.learned_count && !match; ++i) {
-        unsigned long long plo, phi = 0;
-        if (inline_pattern) {
-            plo = b.ring_hi;
-        } else {
-            load_pattern(lc + static_cast<size_t>(i) * stride, stride, plo, phi);
-        }
+        unsigned long long plo, phi;
+        load_pattern(lc + static_cast<size_t>(i) * stride, stride, plo, phi);
         unsigned long long dot = 0, rn = 0;
         for (uint32_t j = 0; j < expected; ++j) {
             const uint32_t pv = ring_get(plo, phi, j);
-            dot += pv * ring_get(b.ring_lo, inline_pattern ? 0ull : b.ring_hi, j);
+            dot += pv * ring_get(b.ring_lo, b.ring_hi, j);
             rn += pv * pv;
         }
         match = cos_ge(dot, rn, cn, p.similarity);
@@ -651,11 +624,6 @@ __device__ void code_update(SynB& b, const NeuronParam& p, uint32_t t, uint16_t*
     if (match) {
         b.code_matches += 1;
         b.flags |= 1u;
-        return;
-    }
-    if (inline_pattern) {
-        b.ring_hi = b.ring_lo;
-        b.learned_count = 1;
         return;
     }
     if (b.learned_count >= p.max_refs) {
@@ -668,13 +636,25 @@ __device__ void code_update(SynB& b, const NeuronParam& p, uint32_t t, uint16_t*
     b.learned_count += 1;
 }
 
+template <bool kInline>
+__device__ __forceinline__ void code_update(SynB& b, const TargetParam& p, uint32_t t, uint16_t* lc, uint32_t stride,
+                                            int enabled, bool inline_pattern) {
+    if (!enabled) {
+        b.flags &= 0xF0u;  // last_code_match = false
+    } else if (kInline || inline_pattern) {
+        code_update_inline(b, p.window, p.similarity, t);
+    } else {
+        code_update_pool(b, p, t, lc, stride);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
 
 // ---------------------------------------------------------------------------
 // grouping: the tick's due list regrouped by target (ascending), each
-// target's events in due order, in four kernels:
+// target's events in due order, in three or four kernels:
 //   k_bcount    a block per contiguous chunk of the due list: events per
 //               bucket of 2^bucket_shift consecutive targets, counted in
 //               shared memory; the block's row of counts goes to bcnt and is
@@ -685,26 +665,26 @@ __device__ void code_update(SynB& b, const NeuronParam& p, uint32_t t, uint16_t*
 //               inside a bucket arbitrary)
 //   k_bsort     a block per bucket: a counting sort of the bucket's events by
 //               target (in shared memory when the bucket fits), segment
-//               starts written; inside a target the order stays arbitrary
-//               (k_events ranks a target's events by due index, the grouping
-//               entry point sorts them with k_segsort)
+//               starts written; inside a target the order stays arbitrary,
+//               then k_segsort sorts it by due index (the grouping entry
+//               points only: the tick's k_events sorts its buckets itself)
 // Per event that is two or more reads of the due list (k_bscatter places a
 // long list in passes over disjoint bucket ranges, so the lines it fills stay
 // in L2 until complete), one scattered write, and a coalesced read and write
 // per bucket: no per-target global atomics.
 // ---------------------------------------------------------------------------
 
-// Block-wide exclusive scan of a[0 .. n) in shared memory (n <= 64 *
-// kThreads), in place; returns the total.  Every thread takes a run of
-// consecutive entries.
+// Block-wide exclusive scan of a[0 .. n) in shared memory, in place; returns
+// the total.  Every thread takes a run of consecutive entries.
+template <int kBlock>
 __device__ uint32_t block_scan_shared(uint32_t* a, uint32_t n) {
-    const uint32_t per = (n + kThreads - 1) / kThreads;
+    const uint32_t per = (n + kBlock - 1) / kBlock;
     const uint32_t b = threadIdx.x * per;
     const uint32_t en = b + per < n ? b + per : n;
     uint32_t sum = 0;
     for (uint32_t i = b; i < en; ++i) sum += a[i];
     uint32_t total;
-    uint32_t run = block_excl_scan(sum, &total);
+    uint32_t run = block_excl_scan_t<kBlock>(sum, &total);
     for (uint32_t i = b; i < en; ++i) {
         const uint32_t v = a[i];
         a[i] = run;
@@ -892,7 +872,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bcount(Engine e) {
         ext += lo >> 31;
     });
     // (if a drain failed the counts are partial and the tick is already
-    // flagged; the row is still written, and k_bscatter / k_bsort keep every
+    // flagged; the row is still written, and the kernels after it keep every
     // access in bounds whatever the counts)
     (void)ok;
     ext = __reduce_add_sync(0xffffffffu, ext);
@@ -944,7 +924,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bscatter(Engine e) {
         __syncthreads();
     }
     // this chunk's place in each bucket: behind the chunks that reserved
-    // before it (the cursors start at zero every tick; k_bsort clears them)
+    // before it (the cursors start at zero every tick; k_events clears them)
     const uint32_t* row = e.bcnt + static_cast<size_t>(blockIdx.x) * B;
     for (uint32_t b = threadIdx.x; b < B; b += blockDim.x) {
         const uint32_t c = row[b];
@@ -1069,7 +1049,7 @@ constexpr size_t kSortSmemBytes = kSortSmemEvents * sizeof(unsigned long long);
 
 // One block per bucket: a counting sort of the bucket's events by target.
 // The events of each target end up contiguous in grp (in arbitrary order;
-// k_events ranks them by due index) and the targets' segment starts are
+// k_segsort sorts them by due index) and the targets' segment starts are
 // written.  A bucket of at most kSortSmemEvents events is loaded once into
 // registers (every load in flight at once), counted, placed in shared memory
 // and written out coalesced; a larger one is counted and placed in grp
@@ -1114,7 +1094,7 @@ __global__ void __launch_bounds__(kThreads) k_bsort(Engine e) {
         for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) nz += s_cnt[j] != 0;
         nz = __reduce_add_sync(0xffffffffu, nz);
         if (lane == 0 && nz) atomicAdd(&e.ts->n_touched, nz);
-        block_scan_shared(s_cnt, nw);  // segment starts relative to lo
+        block_scan_shared<kThreads>(s_cnt, nw);  // segment starts relative to lo
         for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) e.seg_start[n0 + j] = lo + s_cnt[j];
         __syncthreads();
         if (threadIdx.x == 0) {  // the bucket's total and cursor start at zero next tick
@@ -1137,28 +1117,31 @@ __global__ void __launch_bounds__(kThreads) k_bsort(Engine e) {
     }
 }
 
-// Grouping entry point only: due order inside every target's group of grp
-// (one warp per target: up to 32 events bitonic-sorted in registers, longer
-// groups merge-sorted with grp_tmp as scratch).
+// One warp puts a target's group of `len` events in due order (up to 32
+// bitonic-sorted in registers, longer groups merge-sorted with tmp[0 .. len)
+// as scratch).
+__device__ __forceinline__ void sort_group(unsigned long long* g, unsigned long long* tmp, uint32_t len) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (len <= 1) return;
+    if (len <= 32) {
+        unsigned long long v = lane < len ? g[lane] : ~0ull;
+        uint32_t key = lane < len ? grp_key(v) : 0xFFFFFFFFu;
+        warp_bitonic(v, key);
+        if (lane < len) g[lane] = v;
+    } else {
+        warp_merge_sort(g, tmp, len);  // sorted into tmp
+        for (uint32_t k = lane; k < len; k += 32) g[k] = tmp[k];
+        __syncwarp();
+    }
+}
+
+// Grouping entry point only: due order inside every target's group of grp,
+// a warp per target.
 __global__ void __launch_bounds__(kThreads) k_segsort(Engine e) {
-    const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (blockDim.x / 32);
     for (uint32_t n = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); n < e.N; n += warps) {
         const uint32_t beg = e.seg_start[n];
-        const uint32_t len = e.seg_start[n + 1] - beg;
-        if (len <= 1) continue;
-        unsigned long long* g = e.grp + beg;
-        if (len <= 32) {
-            unsigned long long v = lane < static_cast<int>(len) ? g[lane] : ~0ull;
-            uint32_t key = lane < static_cast<int>(len) ? grp_key(v) : 0xFFFFFFFFu;
-            warp_bitonic(v, key);
-            if (lane < static_cast<int>(len)) g[lane] = v;
-        } else {
-            unsigned long long* tmp = reinterpret_cast<unsigned long long*>(e.grp_tmp) + beg;
-            warp_merge_sort(g, tmp, len);  // sorted into tmp
-            for (uint32_t k = lane; k < len; k += 32) g[k] = tmp[k];
-            __syncwarp();
-        }
+        sort_group(e.grp + beg, reinterpret_cast<unsigned long long*>(e.grp_tmp) + beg, e.seg_start[n + 1] - beg);
     }
 }
 
@@ -1167,8 +1150,9 @@ __global__ void __launch_bounds__(kThreads) k_segsort(Engine e) {
 // against the last post spike, last_pre, the pre-spike count, and the
 // spike-code pattern (:318-365).  None of it depends on the target's neuron
 // state; only the STDP part depends on whether the target fired earlier in the
-// tick, which k_process handles by redoing it (walk_fired_targets).
-__device__ __forceinline__ void pre_event(SynAB& r, const NeuronParam& p, uint32_t t, uint16_t* lc,
+// tick, which the walk handles by redoing it (walk_fired_targets).
+template <bool kInline>
+__device__ __forceinline__ void pre_event(SynAB& r, const TargetParam& p, uint32_t t, uint16_t* lc,
                                           const Engine& e, int stdp, int temporal, bool inl) {
     SynA& a = r.a;
     const uint32_t delay = a.meta & kMetaDelayMask;
@@ -1177,7 +1161,7 @@ __device__ __forceinline__ void pre_event(SynAB& r, const NeuronParam& p, uint32
         stdp_apply(a, pre_tick, a.last_post1 - 1, e, stdp, e.tab.ltp);
     a.last_pre1 = pre_tick + 1;
     r.b.pre_count += 1;
-    code_update(r.b, p, t, lc, e.code_stride, temporal, inl);
+    code_update<kInline>(r.b, p, t, lc, e.code_stride, temporal, inl);
 }
 
 __device__ __forceinline__ SynPre pre_fields(const SynA& a) {
@@ -1204,209 +1188,163 @@ __device__ __forceinline__ uint32_t ev_bits(const SynA& a) {
     return ((a.meta >> kMetaCompShift) & 3u) | (((a.meta >> kMetaRecShift) & 3u) << 2);
 }
 
-// All events of synapse tm in one target's group, in due order: `first` is
-// the group position of the first, `more(q)` says whether position q > first
-// is another one.  Snapshots each event's SynA, applies pre_event and writes
-// the event's input record.
-template <typename More, typename DueOf>
-__device__ __forceinline__ void synapse_events(const Engine& e, const NeuronParam& p, uint32_t beg, uint32_t first,
-                                               uint32_t last, uint32_t tm, uint32_t t, int stdp, int temporal,
-                                               More more, DueOf due_of) {
-    uint16_t* lc = e.lcode + p.lcode_base + static_cast<size_t>(tm - p.in_begin) * p.max_refs * e.code_stride;
-    const bool inl = inline_code_pattern(p.max_refs, e.code_stride);
-    SynAB r = e.syn[tm];
-    for (uint32_t q = first; q <= last; ++q) {
-        if (q != first && !more(q)) continue;
-        e.ev_a0[beg + q] = pre_fields(r.a);
-        pre_event(r, p, t, lc, e, stdp, temporal, inl);
-        EvIn in;
-        in.weight = r.a.weight;
-        in.bits = ev_bits(r.a) | (q != first ? kEvRepeat : 0u);
-        in.tm = tm;
-        in.due = due_of[q];
-        e.evin[beg + q] = in;
-    }
-    e.syn[tm] = r;
+// Starts bringing a line from DRAM into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// A synapse record moved with two 32-byte accesses (half the requests of
+// 16-byte ones; each half is one DRAM sector).
+__device__ __forceinline__ SynAB load_record(const SynAB* p) {
+    uint32_t v[16];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[8 * h]), "=r"(v[8 * h + 1]), "=r"(v[8 * h + 2]), "=r"(v[8 * h + 3]), "=r"(v[8 * h + 4]),
+                       "=r"(v[8 * h + 5]), "=r"(v[8 * h + 6]), "=r"(v[8 * h + 7])
+                     : "l"(reinterpret_cast<const char*>(p) + 32 * h)
+                     : "memory");
+    SynAB r;
+    r.a.weight = __uint_as_float(v[0]);
+    r.a.last_pre1 = v[1];
+    r.a.last_post1 = v[2];
+    r.a.meta = v[3];
+    r.a.clamp_hi = __uint_as_float(v[4]);
+    r.a.updates = v[5];
+    r.a.last_delta = __uint_as_float(v[6]);
+    r.a.post_cnt = v[7];
+    r.b.pre_count = v[8];
+    r.b.code_ws = v[9];
+    r.b.code_matches = v[10];
+    r.b.code_len = static_cast<uint8_t>(v[11]);
+    r.b.flags = static_cast<uint8_t>(v[11] >> 8);
+    r.b.learned_count = static_cast<uint16_t>(v[11] >> 16);
+    r.b.ring_lo = (static_cast<unsigned long long>(v[13]) << 32) | v[12];
+    r.b.ring_hi = (static_cast<unsigned long long>(v[15]) << 32) | v[14];
+    return r;
 }
 
-// Due position of entry q of a group sorted in memory.
-struct SortedDue {
-    const unsigned long long* s;
-    __device__ uint32_t operator[](uint32_t q) const { return static_cast<uint32_t>(s[q]) & ~kExternalBit; }
+__device__ __forceinline__ void store_record(SynAB* p, const SynAB& r) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(__float_as_uint(r.a.weight)),
+                 "r"(r.a.last_pre1), "r"(r.a.last_post1), "r"(r.a.meta), "r"(__float_as_uint(r.a.clamp_hi)),
+                 "r"(r.a.updates), "r"(__float_as_uint(r.a.last_delta)), "r"(r.a.post_cnt)
+                 : "memory");
+    const uint32_t bits = r.b.code_len | (static_cast<uint32_t>(r.b.flags) << 8) |
+                          (static_cast<uint32_t>(r.b.learned_count) << 16);
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(reinterpret_cast<char*>(p) + 32),
+                 "r"(r.b.pre_count), "r"(r.b.code_ws), "r"(r.b.code_matches), "r"(bits),
+                 "r"(static_cast<uint32_t>(r.b.ring_lo)), "r"(static_cast<uint32_t>(r.b.ring_lo >> 32)),
+                 "r"(static_cast<uint32_t>(r.b.ring_hi)), "r"(static_cast<uint32_t>(r.b.ring_hi >> 32))
+                 : "memory");
+}
+
+// The parameters of a bucket's targets: in shared memory, or (buckets wider
+// than kSharedParams targets: networks beyond 2^22 neurons) in the first 16
+// bytes of each NeuronParam.
+constexpr uint32_t kSharedParams = 256;
+
+__device__ __forceinline__ TargetParam load_param(const NeuronParam* p) {
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
+    return TargetParam{__uint_as_float(q.x), q.y, __uint_as_float(q.z), q.w};
+}
+
+struct BucketParams {
+    const TargetParam* shared;
+    const NeuronParam* global;  // the bucket's first target
+    bool in_shared;
+    __device__ __forceinline__ TargetParam operator[](uint32_t j) const {
+        return in_shared ? shared[j] : load_param(global + j);
+    }
 };
 
-// One target's group in k_events.  Groups of up to 32 events stay in lanes:
-// each event's position in due order is its rank among the group's due
-// indices, and the events of each synapse are found with one match; the
-// synapse's earliest event's lane then processes all of them in due order.
-// Longer groups are merge-sorted into grp_tmp and scanned.
-// A synapse with a single event in its target's group this tick: the unit
-// of work k_events queues so that all 32 lanes of a warp carry one.
-struct EvItem {
-    uint32_t tm, pos, due, n;
-};
+// Threads of a k_events block, the events it holds in shared memory, and the
+// most events of one target it ranks there (the rank compares every pair of a
+// target's events).
+constexpr int kEventThreads = SNNGB_EVENT_THREADS;
+constexpr uint32_t kBlockPerThread = 10;
+constexpr uint32_t kBlockEvents = kBlockPerThread * kEventThreads;
+constexpr uint32_t kRankEvents = 512;
+constexpr uint32_t kSharedSynapse = 0x8000u;  // beside an event's target: its synapse has other events in the tick
+static_assert((1u << kMaxBucketShift) <= kSharedSynapse, "targets of a bucket");
 
-// Pre-spike work of a queued event (one lane).
-__device__ __forceinline__ void synapse_item(const Engine& e, const EvItem& it, uint32_t t, int stdp, int temporal) {
-    const NeuronParam p = e.nparam[it.n];
-    const bool inl = inline_code_pattern(p.max_refs, e.code_stride);
-    uint16_t* lc =
-        inl ? nullptr : e.lcode + p.lcode_base + static_cast<size_t>(it.tm - p.in_begin) * p.max_refs * e.code_stride;
-    SynAB r = e.syn[it.tm];
-    e.ev_a0[it.pos] = pre_fields(r.a);
-    pre_event(r, p, t, lc, e, stdp, temporal, inl);
-    EvIn in;
-    in.weight = r.a.weight;
-    in.bits = ev_bits(r.a);
-    in.tm = it.tm;
-    in.due = it.due;
-    e.evin[it.pos] = in;
-    e.syn[it.tm] = r;
-}
-
-__device__ __forceinline__ void events_of_target(const Engine& e, uint32_t n, uint32_t beg, uint32_t len, uint32_t t,
-                                                 int stdp, int temporal, uint32_t* wdue, uint32_t* wrank,
-                                                 EvItem* queue, uint32_t& qn) {
-    const uint32_t lane = threadIdx.x & 31;
-    if (len <= 32) {
-        const bool valid = lane < len;
-        const unsigned long long v = valid ? e.grp[beg + lane] : 0ull;
-        const uint32_t lo = static_cast<uint32_t>(v);
-        const uint32_t key = lo & ~kExternalBit;
-        uint32_t rank = 0;
-        for (uint32_t i = 0; i < len; ++i) rank += __shfl_sync(0xffffffffu, key, i) < key;
-        const bool syn = valid && !(lo & kExternalBit);
-        const uint32_t tm = static_cast<uint32_t>(v >> 32);
-        const uint32_t same = __match_any_sync(0xffffffffu, syn ? tm : 0xFFFFFFFFu);
-        wdue[lane] = key;
-        wrank[lane] = rank;
-        __syncwarp();
-        if (valid && !syn) {
-            EvIn in;
-            in.weight = __uint_as_float(tm);
-            in.bits = kEvExternal;
-            in.tm = 0;
-            in.due = key;
-            e.evin[beg + rank] = in;
-        }
-        const bool single = syn && same == (1u << lane);
-        const uint32_t qmask = __ballot_sync(0xffffffffu, single);
-        if (single) {  // the common case: queued, processed 32 at a time
-            EvItem it;
-            it.tm = tm;
-            it.pos = beg + rank;
-            it.due = key;
-            it.n = n;
-            queue[qn + __popc(qmask & ((1u << lane) - 1u))] = it;
-        }
-        qn += __popc(qmask);
-        bool leader = syn && !single;
-        if (leader) {
-            for (uint32_t m = same; m; m &= m - 1) leader = leader && wrank[__ffs(m) - 1] >= rank;
-        }
-        if (leader) {
-            const NeuronParam p = e.nparam[n];
-            uint16_t* lc = e.lcode + p.lcode_base + static_cast<size_t>(tm - p.in_begin) * p.max_refs * e.code_stride;
-            const bool inl = inline_code_pattern(p.max_refs, e.code_stride);
-            SynAB r = e.syn[tm];
-            uint32_t rest = same, repeat = 0;
-            while (rest) {  // the synapse's events in due order (rank order)
-                uint32_t j = __ffs(rest) - 1, best = wrank[j];
-                for (uint32_t m = rest & (rest - 1); m; m &= m - 1) {
-                    const uint32_t c = __ffs(m) - 1;
-                    if (wrank[c] < best) {
-                        best = wrank[c];
-                        j = c;
-                    }
-                }
-                rest &= ~(1u << j);
-                e.ev_a0[beg + best] = pre_fields(r.a);
-                pre_event(r, p, t, lc, e, stdp, temporal, inl);
-                EvIn in;
-                in.weight = r.a.weight;
-                in.bits = ev_bits(r.a) | repeat;
-                in.tm = tm;
-                in.due = wdue[j];
-                e.evin[beg + best] = in;
-                repeat = kEvRepeat;
-            }
-            e.syn[tm] = r;
-        }
-        __syncwarp();
-        return;
+// A bucket's events grouped by target in due order, as the event and walk
+// phases of k_events see them.  Indices count from the bucket's first event.
+//
+// In shared memory.
+struct SharedEvents {
+    unsigned long long* word;  // payload << 32 | due index << 1 | external
+    float* w;                  // weight the event delivers
+    uint8_t* bits;             // EvIn::bits
+    __device__ __forceinline__ EvIn at(uint32_t i) const {
+        const unsigned long long v = word[i];
+        EvIn x;
+        x.weight = w[i];
+        x.bits = bits[i];
+        x.tm = static_cast<uint32_t>(v >> 32);
+        x.due = static_cast<uint32_t>(v) >> 1;
+        return x;
     }
-    // grp_tmp is free once the groups are built (16 bytes per event: room for
-    // two 8-byte words each)
-    unsigned long long* srt = reinterpret_cast<unsigned long long*>(e.grp_tmp) + beg;
-    warp_merge_sort(e.grp + beg, srt, len);
-    const NeuronParam p = e.nparam[n];
-    for (uint32_t j = lane; j < len; j += 32) {
-        const unsigned long long x = srt[j];
-        const uint32_t lo = static_cast<uint32_t>(x);
-        const uint32_t tm = static_cast<uint32_t>(x >> 32);
-        if (lo & kExternalBit) {
-            EvIn in;
-            in.weight = __uint_as_float(tm);
-            in.bits = kEvExternal;
-            in.tm = 0;
-            in.due = lo & ~kExternalBit;
-            e.evin[beg + j] = in;
-            continue;
-        }
-        auto same_syn = [&](uint32_t q) {
-            const unsigned long long y = srt[q];
-            return !(static_cast<uint32_t>(y) & kExternalBit) && static_cast<uint32_t>(y >> 32) == tm;
-        };
-        bool first = true;
-        for (uint32_t q = 0; q < j && first; ++q) first = !same_syn(q);
-        if (!first) continue;
-        synapse_events(e, p, beg, j, len - 1, tm, t, stdp, temporal, same_syn, SortedDue{srt});
-    }
-    __syncwarp();
-}
-
-// One warp per target with due events (events_of_target).  Synapses with a
-// single event this tick go to a per-warp queue in shared memory and are
-// processed 32 at a time, one per lane, whatever targets they belong to;
-// repeats and long groups are processed in place.
-__global__ void __launch_bounds__(kThreads, SNNGB_EVENTS_MIN_BLOCKS) k_events(Engine e) {
-    tick_enter();
-    __shared__ uint32_t s_due[kThreads], s_rank[kThreads];
-    __shared__ EvItem s_queue[kThreads / 32][64];
-    const uint32_t t = e.ts->tick;
-    const int stdp = e.ts->stdp_enabled;
-    const int temporal = e.ts->temporal_enabled;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t wbase = threadIdx.x & ~31u;
-    EvItem* queue = s_queue[threadIdx.x >> 5];
-    uint32_t qn = 0;  // warp-uniform
-    const uint32_t warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t n = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); n < e.N; n += warps) {
-        const uint32_t beg = e.seg_start[n];
-        const uint32_t end = e.seg_start[n + 1];
-        if (end == beg) continue;
-        events_of_target(e, n, beg, end - beg, t, stdp, temporal, s_due + wbase, s_rank + wbase, queue, qn);
-        if (qn >= 32) {
-            __syncwarp();
-            synapse_item(e, queue[qn - 32 + lane], t, stdp, temporal);
-            qn -= 32;
-            __syncwarp();
-        }
-    }
-    __syncwarp();
-    if (lane < qn) synapse_item(e, queue[lane], t, stdp, temporal);
-}
-
-// The block's event inputs: entries [lo, lo + cnt) of evin staged in shared
-// memory once `ready()` returns true; the rest read from global memory.
-struct Staged {
-    const EvIn* s;
-    uint32_t lo, cnt;
-    __device__ __forceinline__ EvIn at(const Engine& e, uint32_t g) const {
-        const uint32_t o = g - lo;
-        return o < cnt ? s[o] : e.evin[g];
+    __device__ __forceinline__ uint32_t bits_of(uint32_t i) const { return bits[i]; }
+    __device__ __forceinline__ float weight_of(uint32_t i) const { return w[i]; }
+    __device__ __forceinline__ bool external(uint32_t i) const { return static_cast<uint32_t>(word[i]) & 1u; }
+    __device__ __forceinline__ uint32_t payload(uint32_t i) const { return static_cast<uint32_t>(word[i] >> 32); }
+    __device__ __forceinline__ void put(uint32_t i, float weight, uint32_t b) const {
+        w[i] = weight;
+        bits[i] = static_cast<uint8_t>(b);
     }
 };
+
+// In global memory (a bucket with more events than a block holds, or a long
+// group): the grouped words of Engine::grp and one EvIn each.
+struct GlobalEvents {
+    const unsigned long long* word;  // payload << 32 | due index | external bit
+    EvIn* in;
+    __device__ __forceinline__ EvIn at(uint32_t i) const { return in[i]; }
+    __device__ __forceinline__ uint32_t bits_of(uint32_t i) const { return in[i].bits; }
+    __device__ __forceinline__ float weight_of(uint32_t i) const { return in[i].weight; }
+    __device__ __forceinline__ bool external(uint32_t i) const {
+        return static_cast<uint32_t>(word[i]) & kExternalBit;
+    }
+    __device__ __forceinline__ uint32_t payload(uint32_t i) const { return static_cast<uint32_t>(word[i] >> 32); }
+    __device__ __forceinline__ void put(uint32_t i, float weight, uint32_t b) const {
+        EvIn x;
+        x.weight = weight;
+        x.bits = b;
+        const unsigned long long v = word[i];
+        x.tm = static_cast<uint32_t>(v >> 32);
+        x.due = static_cast<uint32_t>(v) & ~kExternalBit;
+        in[i] = x;
+    }
+};
+
+// Event i's synapse record: the fields before the event (Engine::ev_a0), its
+// pre-spike work and its input for the walk.  `last` is the end of the
+// target's events if the synapse may have further ones there (they follow in
+// due order), else i + 1.
+template <bool kInline, typename Events>
+__device__ __forceinline__ void synapse_events(const Engine& e, const Events& ev, uint32_t lo, uint32_t i,
+                                               uint32_t last, const TargetParam& p, uint32_t n, uint32_t t, int stdp,
+                                               int temporal) {
+    const uint32_t tm = ev.payload(i);
+    const bool inl = kInline || inline_code_pattern(p.max_refs, e.code_stride);
+    uint16_t* lc = nullptr;
+    if (!inl) {
+        const NeuronParam& q = e.nparam[n];
+        lc = e.lcode + q.lcode_base + static_cast<size_t>(tm - q.in_begin) * p.max_refs * e.code_stride;
+    }
+    SynAB r = load_record(e.syn + tm);
+    // one body for the first and the further events, so that a warp's lanes
+    // go through it together whatever the distance to their next event
+    for (uint32_t q = i, repeat = 0;;) {
+        e.ev_a0[lo + q] = pre_fields(r.a);
+        pre_event<kInline>(r, p, t, lc, e, stdp, temporal, inl);
+        ev.put(q, r.a.weight, ev_bits(r.a) | repeat);
+        do {
+            ++q;
+        } while (q < last && (ev.payload(q) != tm || ev.external(q)));
+        if (q >= last) break;
+        repeat = kEvRepeat;
+    }
+    store_record(e.syn + tm, r);
+}
 
 // Applies to a synapse record the post-spike STDP owed for the target's fires
 // so far and the event's pre-spike STDP (the record is the synapse's state
@@ -1456,16 +1394,14 @@ __device__ __forceinline__ void record_fire(const Engine& e, const Walk& w, uint
     atomicAdd(&e.fire_tile[(due >> 5) / kThreads], 1u);
 }
 
-// Phase 1 of a target's walk: load the neuron (the physics fields only: the
-// temporal ones belong to k_temporal, which may be running at the same time)
-// and process its events in due order up to and including its first fire.
-// Every event before the first fire uses the weight k_events computed.
+// Phase 1 of a target's walk: load the neuron (its physics fields) and
+// process its events in due order up to and including its first fire.  Every
+// event before the first fire uses the weight its synapse's work computed.
 // Returns whether the target fired.
-template <typename Ready>
-__device__ __forceinline__ bool walk_to_first_fire(const Engine& e, Walk& w, uint32_t t, Staged& st, Ready ready) {
+template <typename Events>
+__device__ __forceinline__ bool walk_to_first_fire(const Engine& e, Walk& w, uint32_t t, const Events& ev) {
     NState& s = w.s;
     const NeuronRec* rec = e.nrec + w.n;
-    w.threshold = e.nparam[w.n].threshold;
     {
         const float4 c = reinterpret_cast<const float4*>(rec->cur)[0];
         const uint4 u = reinterpret_cast<const uint4*>(rec->upd)[0];
@@ -1486,12 +1422,11 @@ __device__ __forceinline__ bool walk_to_first_fire(const Engine& e, Walk& w, uin
     }
     w.fires = 0;
     w.first_fire = 0;
-    if (w.len > 0) decay_to(s, t, e);
-    if (!ready()) st.cnt = 0;
+    decay_to(s, t, e);
     for (uint32_t i = 0; i < w.len; ++i) {
-        const EvIn x = st.at(e, w.beg + i);
-        if (process_input(s, w.threshold, x.bits & 3u, (x.bits >> 2) & 3u, x.weight, t)) {
-            record_fire(e, w, x.due);
+        const uint32_t bits = ev.bits_of(w.beg + i);
+        if (process_input(s, w.threshold, bits & 3u, (bits >> 2) & 3u, ev.weight_of(w.beg + i), t)) {
+            record_fire(e, w, ev.at(w.beg + i).due);
             w.fires = 1;
             w.first_fire = i;
             w.i = i + 1;
@@ -1505,17 +1440,20 @@ __device__ __forceinline__ bool walk_to_first_fire(const Engine& e, Walk& w, uin
 // Phase 2, one warp: the rest of the walks of its lanes' fired targets, one
 // target at a time.  Every synaptic event after a fire redoes its STDP with
 // the target's fire count so far, starting from the synapse's state before
-// the event: k_events' snapshot, or, when the same synapse already had an
-// event after the first fire, the record that event left.  The warp redoes up
-// to 32 events at once (an event whose predecessor is in the same chunk waits
-// a round and takes its record by shuffle); the target's own lane then runs
-// the neuron physics over them in order.  If the target fires again inside the
+// the event: its snapshot, or, when the same synapse already had an event
+// after the first fire, the record that event left.  The warp redoes up to 32
+// events at once (an event whose predecessor is in the same chunk waits a
+// round and takes its record by shuffle); the target's own lane then runs the
+// neuron physics over them in order.  If the target fires again inside the
 // chunk, the events after that fire are redone with the new count; only the
 // records of events before it are stored (the last event of each synapse
-// stores).  The result is the sequential order's.
+// stores).  The result is the sequential order's.  `lo` is the bucket's first
+// event (Engine::ev_a0 counts from the tick's first one).
+template <typename Events>
 __device__ __forceinline__ void walk_fired_targets(const Engine& e, Walk& w, bool fired, uint32_t t, int stdp,
-                                                   Staged st, const float* ltp, float* s_wt) {
+                                                   const Events& ev, uint32_t lo, float* s_wt) {
     const uint32_t lane = threadIdx.x & 31;
+    const float* ltp = e.tab.ltp;
     unsigned pend = __ballot_sync(0xffffffffu, fired);
     while (pend) {
         const uint32_t L = __ffs(pend) - 1;
@@ -1529,13 +1467,13 @@ __device__ __forceinline__ void walk_fired_targets(const Engine& e, Walk& w, boo
             const uint32_t m = len - pos < 32 ? len - pos : 32;
             const uint32_t j = pos + lane;
             EvIn x{};
-            if (lane < m) x = st.at(e, beg + j);
+            if (lane < m) x = ev.at(beg + j);
             const bool syn = lane < m && !(x.bits & kEvExternal);
             // the synapse's latest earlier event after the first fire
             uint32_t pred = 0xFFFFFFFFu;
             if (syn && (x.bits & kEvRepeat)) {
                 for (uint32_t q = j; q-- > after;) {
-                    const EvIn y = st.at(e, beg + q);
+                    const EvIn y = ev.at(beg + q);
                     if (!(y.bits & kEvExternal) && y.tm == x.tm) {
                         pred = q;
                         break;
@@ -1547,7 +1485,7 @@ __device__ __forceinline__ void walk_fired_targets(const Engine& e, Walk& w, boo
             float wt = x.weight;
             bool done = !syn;
             if (syn && !wait) {
-                a = pred != 0xFFFFFFFFu ? e.syn[x.tm].a : before_event(e.syn[x.tm].a, e.ev_a0[beg + j]);
+                a = pred != 0xFFFFFFFFu ? e.syn[x.tm].a : before_event(e.syn[x.tm].a, e.ev_a0[lo + beg + j]);
                 wt = redo_pre_stdp(e, a, t, fires, stdp, ltp);
                 done = true;
             }
@@ -1566,7 +1504,7 @@ __device__ __forceinline__ void walk_fired_targets(const Engine& e, Walk& w, boo
             uint32_t next = pos + m;
             if (lane == L) {
                 for (uint32_t c = 0; c < m; ++c) {
-                    const EvIn y = st.at(e, beg + pos + c);
+                    const EvIn y = ev.at(beg + pos + c);
                     if (process_input(w.s, w.threshold, y.bits & 3u, (y.bits >> 2) & 3u, s_wt[c], t)) {
                         record_fire(e, w, y.due);
                         w.fires += 1;
@@ -1608,98 +1546,340 @@ __device__ __forceinline__ void finish_walk(const Engine& e, const Walk& w) {
     }
 }
 
-// One thread per touched target: the neuron's physics over its events in
-// due order.  Exact because every state an event reads or writes belongs to
-// its target (the target's neuron state and the target's incoming synapses);
-// post-spike STDP of a fire is applied lazily to synapses touched later in the
-// tick and in bulk by k_post for the rest.
-// A block's targets are consecutive touched targets, so their event inputs
-// are one contiguous range: one thread copies it into shared memory with a
-// bulk copy while every thread loads its neuron's records.
-__global__ void __launch_bounds__(kThreads, SNNGB_PROCESS_MIN_BLOCKS) k_process(Engine e) {
-    tick_enter();
-    extern __shared__ __align__(128) EvIn s_ev[];  // kStageEvents entries
-    __shared__ __align__(8) unsigned long long s_bar;
-    __shared__ uint32_t s_lo, s_cnt;
-    __shared__ float s_wt[kThreads / 32][32];  // per warp: weights of the events redone after a fire
-    const uint32_t t = e.ts->tick;
-    const uint32_t N = e.N;
-    const int stdp = e.ts->stdp_enabled;
-    if (threadIdx.x == 0) mbar_init(&s_bar, 1);
-    __syncthreads();
-    // the LTP table goes to shared memory (when it fits) during the first
-    // round's copy: the STDP redone after a fire then makes no dependent
-    // global load besides the snapshot
-    const bool ltp_shared = stdp && e.tab.stdp_len <= kLtpShared;
-    const float* ltp = ltp_shared ? reinterpret_cast<const float*>(s_ev + kStageEvents) : e.tab.ltp;
-    uint32_t parity = 0;
-    bool staging = true;  // false after a copy outlived its wait: shared memory is no longer used
-    // `per` consecutive targets per block and round (their events are one
-    // contiguous range of the grouped list): the grid has at least three
-    // blocks per SM, so one wave of equal blocks spreads over every SM (the
-    // block scheduler fills each SM to its occupancy limit)
-    const uint32_t per_even = (N + gridDim.x - 1) / gridDim.x;
-    const uint32_t per = per_even < blockDim.x ? per_even : blockDim.x;
-    for (uint32_t k0 = blockIdx.x * per; k0 < N; k0 += gridDim.x * per) {
-        if (threadIdx.x == 0) {
-            const uint32_t k1 = k0 + per < N ? k0 + per : N;
-            const uint32_t lo = e.seg_start[k0];
-            const uint32_t hi = e.seg_start[k1];
-            const uint32_t cnt = staging ? (hi - lo < kStageEvents ? hi - lo : kStageEvents) : 0u;
-            s_lo = lo;
-            s_cnt = cnt;
-            if (cnt > 0) bulk_load(s_ev, e.evin + lo, cnt * static_cast<uint32_t>(sizeof(EvIn)), &s_bar);
-        }
-        if (ltp_shared && k0 == blockIdx.x * per) {
-            float* s_ltp = reinterpret_cast<float*>(s_ev + kStageEvents);
-            for (uint32_t i = threadIdx.x; i < e.tab.stdp_len; i += blockDim.x) s_ltp[i] = e.tab.ltp[i];
-        }
-        __syncthreads();
-        const Staged st{s_ev, s_lo, s_cnt};
-        bool waited = st.cnt == 0;
-        bool ok = true;
-        auto ready = [&]() {
-            if (!waited) {
-                ok = mbar_wait(&s_bar, parity, e.stage_wait_ns);
-                waited = true;
-            }
-            return ok;
-        };
-        const uint32_t k = k0 + threadIdx.x;
+__device__ __noinline__ void temporal_target(const Engine& e, uint32_t n, uint32_t k, uint32_t t, int temporal);
+
+// The walks of a bucket's targets, a thread each.
+template <typename Events>
+__device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, uint32_t lo, uint32_t n0, uint32_t nw,
+                                            const uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
+                                            float* s_wt) {
+    for (uint32_t j0 = 0; j0 < nw; j0 += blockDim.x) {
+        const uint32_t j = j0 + threadIdx.x;
         Walk w;
         w.n = w.beg = w.len = w.i = w.fires = w.first_fire = 0;
-        if (threadIdx.x < per && k < N) {
-            w.n = k;
-            w.beg = e.seg_start[k];
-            w.len = e.seg_start[k + 1] - w.beg;
+        w.threshold = 0.0f;
+        if (j < nw) {
+            w.n = n0 + j;
+            w.beg = s_seg[j];
+            w.len = s_seg[j + 1] - w.beg;
+            w.threshold = par[j].threshold;
         }
-        const bool mine_target = w.len > 0;  // a target with due events
+        const bool mine = w.len > 0;  // a target with due events
         bool fired = false;
-        Staged mine = st;
-        if (mine_target) fired = walk_to_first_fire(e, w, t, mine, ready);
-        if (!ready()) mine.cnt = 0;
-        walk_fired_targets(e, w, fired, t, stdp, mine, ltp, s_wt[threadIdx.x >> 5]);
-        if (mine_target) finish_walk(e, w);
-        const bool failed = __syncthreads_or(!ok);
-        if (st.cnt > 0) {
-            if (failed) {
-                // the block read its inputs from global memory; wait once more
-                // for the copy before the buffer is reused or the block exits
-                if (threadIdx.x == 0) raise_status(e, kStatusStageTimeout);
-                if (!__syncthreads_and(mbar_wait(&s_bar, parity, kDrainWaitNs))) return;
-            }
-            parity ^= 1u;
-        }
-        if (failed) staging = false;
+        if (mine) fired = walk_to_first_fire(e, w, t, ev);
+        walk_fired_targets(e, w, fired, t, stdp, ev, lo, s_wt);
+        if (mine) finish_walk(e, w);
     }
 }
 
-// The temporal pattern update of every touched target (SynapseDendriteProcessor
-// .cpp:294-316), once per tick for all its k events (temporal_tick).  It reads
-// and writes only the neuron's temporal fields, which nothing else in the tick
-// touches, so it can run beside k_events / k_process.
-template <bool kOne>
-__device__ __forceinline__ void temporal_target(const Engine& e, uint32_t n, uint32_t k, uint32_t t, int temporal) {
+// A bucket with more events than the block's shared memory, or with a long
+// group: grouped in Engine::grp (a counting sort by target, then a warp per
+// target puts its events in due order), its event inputs in Engine::evin.
+template <bool kInline>
+__device__ __noinline__ void bucket_in_global(const Engine& e, uint32_t lo, uint32_t m, uint32_t n0, uint32_t nw,
+                                              uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
+                                              int temporal, float* s_wt) {
+    const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
+    unsigned long long* grp = e.grp + lo;
+    // s_seg[j + 1] holds target j's count, then its cursor, then its end
+    for (uint32_t j = threadIdx.x; j <= nw; j += blockDim.x) s_seg[j] = 0;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+        const uint32_t z = in[i].z;
+        if (z < nw) atomicAdd(&s_seg[z + 1], 1u);
+    }
+    __syncthreads();
+    block_scan_shared<kEventThreads>(s_seg + 1, nw);
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+        const uint4 q = in[i];
+        if (q.z < nw) grp[atomicAdd(&s_seg[q.z + 1], 1u)] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
+    }
+    __syncthreads();
+    // the bucket's own entries are placed: their memory is the merges' scratch
+    unsigned long long* tmp = reinterpret_cast<unsigned long long*>(e.grp_tmp + lo);
+    for (uint32_t j = threadIdx.x >> 5; j < nw; j += blockDim.x / 32) {
+        const uint32_t beg = s_seg[j], len = s_seg[j + 1] - beg;
+        sort_group(grp + beg, tmp + beg, len);
+    }
+    __syncthreads();
+    const GlobalEvents ev{grp, e.evin + lo};
+    const uint32_t total = s_seg[nw];
+    for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
+        if (ev.external(i)) {
+            ev.put(i, __uint_as_float(ev.payload(i)), kEvExternal);
+            continue;
+        }
+        uint32_t j = 0, above = nw;  // s_seg[j] <= i < s_seg[above]
+        while (above - j > 1) {
+            const uint32_t mid = (j + above) >> 1;
+            if (s_seg[mid] <= i) {
+                j = mid;
+            } else {
+                above = mid;
+            }
+        }
+        const uint32_t tm = ev.payload(i);
+        bool first = true;
+        for (uint32_t q = s_seg[j]; q < i && first; ++q) first = ev.external(q) || ev.payload(q) != tm;
+        if (first) synapse_events<kInline>(e, ev, lo, i, s_seg[j + 1], par[j], n0 + j, t, stdp, temporal);
+    }
+    for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) {
+        const uint32_t k = s_seg[j + 1] - s_seg[j];
+        if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
+    }
+    __syncthreads();
+    walk_bucket(e, ev, lo, n0, nw, s_seg, par, t, stdp, s_wt);
+}
+
+// Everything a tick does at its targets, a block per bucket of consecutive
+// targets (a bucket's events are one contiguous run of grp_tmp):
+//
+//   1. the bucket's entries come in with one bulk copy (bounded mbarrier
+//      wait) while the targets' parameters are loaded; every thread holds its
+//      share in registers;
+//   2. a counting sort by target into shared memory, then each event's place
+//      in due order is its rank among its target's events; the same
+//      comparison finds the synapses with several events;
+//   3. a thread per event, the warps taking 32 at a time as they get free: its
+//      synapse record (one 64-byte read and write, random), pre-spike STDP,
+//      spike code, the weight it delivers; a synapse with several events has
+//      one thread do them all (together with its like, so that the others'
+//      warps need not wait); beside them the neurons' temporal patterns, a
+//      thread per target;
+//   4. a thread per target: the neuron's physics over its events in due
+//      order, exact because everything an event reads or writes belongs to its
+//      target; post-spike STDP of a fire is applied lazily to synapses with
+//      later events in the tick and in bulk by k_post for the rest.
+//
+// The records' DRAM traffic (a 128-byte line in and one out per event: 39 ps
+// an event at the measured copy bandwidth) is the floor; the kernel is bound by
+// the length of its instruction streams before that (about 1,080 warp
+// instructions per 32 events, 35 % of the issue slots, 20 warps per SM at 96
+// registers; more blocks with fewer registers, and records loaded one round
+// ahead, measured the same or slower).  As four kernels (bucket sort, synapse
+// events by a warp per target, walk, temporal pattern) the events' words and
+// inputs went through global memory between them, 20 of 32 lanes idled, and
+// each waited for the slowest block of the one before.  Sum of the four ->
+// this one, per tick: 309 -> 197 us (2.5 M events, 200,000 neurons), 82 -> 36
+// us (250,000 events, 20,000 neurons).
+//
+// kInline: every synapse's learned code pattern is in its record
+// (inline_code_pattern holds for every target).
+template <bool kInline>
+__global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_events(const __grid_constant__ Engine e) {
+    tick_enter();
+    extern __shared__ __align__(128) unsigned char s_raw[];  // EventsLayout
+    __shared__ __align__(8) unsigned long long s_bar;
+    __shared__ float s_wt[kEventThreads / 32][32];  // per warp: weights of the events redone after a fire
+    __shared__ uint32_t s_repeats;                  // synapses with several events
+    __shared__ uint32_t s_next;                     // next task of the events phase
+    __shared__ uint32_t s_longest;                  // events of the busiest target
+    const uint32_t width = 1u << e.bucket_shift;
+    // the staged entries (16 bytes per event); once they are in registers, the
+    // words grouped by target (8) and the words in due order (8); once those
+    // are there, w and bits in place of the grouped words
+    uint4* s_in = reinterpret_cast<uint4*>(s_raw);
+    unsigned long long* s_word = reinterpret_cast<unsigned long long*>(s_raw);
+    const SharedEvents ev{s_word + kBlockEvents, reinterpret_cast<float*>(s_raw), s_raw + 4 * kBlockEvents};
+    uint16_t* s_tgt = reinterpret_cast<uint16_t*>(s_raw + sizeof(BucketEntry) * kBlockEvents);
+    uint16_t* s_list = s_tgt + kBlockEvents;  // first events of the synapses with several
+    TargetParam* s_par = reinterpret_cast<TargetParam*>(s_list + kBlockEvents);
+    const bool keep_params = width <= kSharedParams;
+    uint32_t* s_seg = reinterpret_cast<uint32_t*>(s_par + (keep_params ? width : 0u));  // [width + 2]
+    const uint32_t t = e.ts->tick;
+    const int stdp = e.ts->stdp_enabled;
+    const int temporal = e.ts->temporal_enabled;
+    if (threadIdx.x == 0) mbar_init(&s_bar, 1);
+    __syncthreads();
+    uint32_t parity = 0;
+    bool staging = true;  // false after a copy outlived its wait: no more copies
+    for (uint32_t b = blockIdx.x; b < e.nbuckets; b += gridDim.x) {
+        const uint32_t lo = e.bstart[b], m = e.bstart[b + 1] - lo;
+        const uint32_t n0 = b << e.bucket_shift;
+        const uint32_t nw = e.N - n0 < width ? e.N - n0 : width;
+        if (m == 0) {
+            if (e.multi_refs)
+                for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) e.seg_start[n0 + j] = lo;
+            continue;
+        }
+        const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
+        bool small = m <= kBlockEvents;
+        const bool staged = small && staging;
+        if (staged && threadIdx.x == 0) bulk_load(s_raw, in, m * static_cast<uint32_t>(sizeof(BucketEntry)), &s_bar);
+        const BucketParams par{s_par, e.nparam + n0, keep_params};
+        if (keep_params)
+            for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) s_par[j] = load_param(e.nparam + n0 + j);
+        for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) {
+            prefetch_l2(e.nrec + n0 + j);
+            prefetch_l2(e.ntp + n0 + j);
+        }
+        for (uint32_t j = threadIdx.x; j <= nw; j += kEventThreads) s_seg[j] = 0;
+        if (threadIdx.x == 0) {  // the bucket's total and cursor start at zero next tick
+            e.btot[b] = 0;
+            e.bcur[b] = 0;
+        }
+        bool ready = true;
+        if (staged && threadIdx.x == 0) ready = mbar_wait(&s_bar, parity, e.stage_wait_ns);
+        ready = __syncthreads_and(ready);
+        if (staged) {
+            if (!ready) {
+                // the copy is still in flight: wait for it once more before
+                // its buffer is used or the block exits
+                bool drained = true;
+                if (threadIdx.x == 0) {
+                    raise_status(e, kStatusStageTimeout);
+                    drained = mbar_wait(&s_bar, parity, kDrainWaitNs);
+                }
+                if (!__syncthreads_and(drained)) return;
+                staging = false;
+            }
+            parity ^= 1u;
+        }
+        if (small && !(staged && ready)) {  // no copy: the entries come in directly
+            for (uint32_t i = threadIdx.x; i < m; i += kEventThreads) s_in[i] = in[i];
+            __syncthreads();
+        }
+        if (small) {
+            // counting sort by target: an entry's place among its target's is
+            // the count before it
+            uint2 v[kBlockPerThread];
+            uint32_t at[kBlockPerThread];  // target | place << 16
+#pragma unroll
+            for (uint32_t k = 0; k < kBlockPerThread; ++k) {
+                const uint32_t i = threadIdx.x + k * kEventThreads;
+                at[k] = 0xFFFFu;
+                if (i >= m) continue;
+                const uint4 q = s_in[i];
+                if (!(q.x & kExternalBit)) prefetch_l2(e.syn + q.y);
+                v[k] = make_uint2(q.x, q.y);
+                if (q.z < nw) at[k] = q.z | (atomicAdd(&s_seg[q.z + 1], 1u) << 16);
+            }
+            __syncthreads();
+            // exclusive scan of the counts by one warp (a bucket has 32 to 64
+            // targets unless the network is huge): s_seg[j + 1], s_seg[j + 2]
+            // become the first and the end of target j's events
+            if (threadIdx.x < 32) {
+                uint32_t busy = 0, longest = 0, run = 0;
+                for (uint32_t j0 = 0; j0 < nw; j0 += 32) {
+                    const uint32_t j = j0 + threadIdx.x, c = j < nw ? s_seg[j + 1] : 0u;
+                    const uint32_t incl = warp_incl_scan(c);
+                    if (j < nw) s_seg[j + 1] = run + incl - c;
+                    run += __shfl_sync(0xffffffffu, incl, 31);
+                    busy += c != 0;
+                    longest = max(longest, c);
+                }
+                busy = __reduce_add_sync(0xffffffffu, busy);
+                longest = __reduce_max_sync(0xffffffffu, longest);
+                if (threadIdx.x == 0) {
+                    if (busy) atomicAdd(&e.ts->n_touched, busy);
+                    s_seg[nw + 1] = run;
+                    s_repeats = 0;
+                    s_next = 0;
+                    s_longest = longest;
+                }
+            }
+            __syncthreads();
+            small = s_longest <= kRankEvents;
+            if (small) {
+                const uint32_t total = s_seg[nw + 1];
+#pragma unroll
+                for (uint32_t k = 0; k < kBlockPerThread; ++k) {
+                    const uint32_t j = at[k] & 0xFFFFu;
+                    if (j == 0xFFFFu) continue;
+                    const uint32_t p = s_seg[j + 1] + (at[k] >> 16);
+                    s_word[p] = (static_cast<unsigned long long>(v[k].y) << 32) | __funnelshift_l(v[k].x, v[k].x, 1);
+                    s_tgt[p] = static_cast<uint16_t>(j);
+                }
+                __syncthreads();
+                // each event's rank in due order among its target's events
+                // (by position: the lanes of a warp read the same or the next
+                // group's words); of the synapses with several events, the
+                // first event goes on a list
+                for (uint32_t i = threadIdx.x; i < total; i += kEventThreads) {
+                    const unsigned long long v = s_word[i];
+                    const uint32_t j = s_tgt[i] & ~kSharedSynapse, s0 = s_seg[j + 1], s1 = s_seg[j + 2];
+                    const uint32_t due = static_cast<uint32_t>(v), pay = static_cast<uint32_t>(v >> 32);
+                    uint32_t p = s0, same = 0, before = 0;  // synaptic events with this payload, those due earlier
+                    for (uint32_t q = s0; q < s1; ++q) {
+                        const unsigned long long x = s_word[q];
+                        const uint32_t d = static_cast<uint32_t>(x);
+                        const bool hit = static_cast<uint32_t>(x >> 32) == pay && !(d & 1u);
+                        p += d < due;
+                        same += hit;
+                        before += hit && d < due;
+                    }
+                    ev.word[p] = v;
+                    if (same > 1 && !(due & 1u)) {
+                        s_tgt[p] = static_cast<uint16_t>(j | kSharedSynapse);
+                        if (before == 0) s_list[atomicAdd(&s_repeats, 1u)] = static_cast<uint16_t>(p);
+                    }
+                }
+                __syncthreads();
+                if (e.multi_refs)
+                    for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) e.seg_start[n0 + j] = lo + s_seg[j + 1];
+                // The warps share out the rest but the walk: the temporal
+                // patterns (they need only the targets' event counts) 32
+                // targets at a time from the first warps, the synapses with
+                // several events, then all other events.
+                const uint32_t lane = threadIdx.x & 31;
+                for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) {
+                    const uint32_t k = s_seg[j + 2] - s_seg[j + 1];
+                    if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
+                }
+                __syncwarp();
+                const uint32_t repeats = s_repeats, lists = (repeats + 31) / 32, tasks = lists + (total + 31) / 32;
+                for (;;) {
+                    uint32_t task = lane == 0 ? atomicAdd(&s_next, 1u) : 0u;
+                    task = __shfl_sync(0xffffffffu, task, 0);
+                    if (task >= tasks) break;
+                    uint32_t i = (task - lists) * 32 + lane, last = 0;
+                    bool run;
+                    if (task < lists) {
+                        const uint32_t k = task * 32 + lane;
+                        run = k < repeats;
+                        if (run) {
+                            i = s_list[k];
+                            last = s_seg[(s_tgt[i] & ~kSharedSynapse) + 2];
+                        }
+                    } else {
+                        run = i < total;
+                        if (run && ev.external(i)) {
+                            ev.put(i, __uint_as_float(ev.payload(i)), kEvExternal);
+                            run = false;
+                        }
+                        run = run && !(s_tgt[i] & kSharedSynapse);
+                        last = i + 1;
+                    }
+                    if (run) {
+                        const uint32_t j = s_tgt[i] & ~kSharedSynapse;
+                        synapse_events<kInline>(e, ev, lo, i, last, par[j], n0 + j, t, stdp, temporal);
+                    }
+                    __syncwarp();
+                }
+                __syncthreads();
+                walk_bucket(e, ev, lo, n0, nw, s_seg + 1, par, t, stdp, s_wt[threadIdx.x >> 5]);
+            }
+        }
+        if (!small) {
+            bucket_in_global<kInline>(e, lo, m, n0, nw, s_seg, par, t, stdp, temporal, s_wt[threadIdx.x >> 5]);
+            __syncthreads();
+            if (m > kBlockEvents) {
+                uint32_t busy = 0;
+                for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) busy += s_seg[j + 1] != s_seg[j];
+                busy = __reduce_add_sync(0xffffffffu, busy);
+                if ((threadIdx.x & 31) == 0 && busy) atomicAdd(&e.ts->n_touched, busy);
+            }
+            if (e.multi_refs)
+                for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) e.seg_start[n0 + j] = lo + s_seg[j];
+        }
+        __syncthreads();
+    }
+}
+
+// The temporal pattern of a touched target that keeps one reference pattern
+// (SynapseDendriteProcessor.cpp:294-316), once per tick for all its k events.
+// It reads and writes only the neuron's temporal fields.
+__device__ __noinline__ void temporal_target(const Engine& e, uint32_t n, uint32_t k, uint32_t t, int temporal) {
     const NeuronParam p = e.nparam[n];
     NeuronRec* rec = e.nrec + n;
     const NeuronTp q = e.ntp[n];
@@ -1715,12 +1895,13 @@ __device__ __forceinline__ void temporal_target(const Engine& e, uint32_t n, uin
     s.ring_head = q.ring_head;
     s.ring_used = q.ring_used;
     s.last_run = s.nruns > 0 ? e.cand[p.cand_base + s.nruns - 1] : 0ull;
-    if (kOne && s.ref_count > 0) s.one = e.refmeta[p.meta_base];
+    s.one = RefMeta{};
+    if (s.ref_count > 0) s.one = e.refmeta[p.meta_base];
     s.snap_pending = false;
-    temporal_tick<kOne>(s, p, t, e, temporal, k);
+    temporal_tick(s, p, t, e, temporal, k);
     if (s.nruns > 0) e.cand[p.cand_base + s.nruns - 1] = s.last_run;
-    if (kOne && s.ref_count > 0) e.refmeta[p.meta_base] = s.one;
-    if (kOne && s.snap_pending) {
+    if (s.ref_count > 0) e.refmeta[p.meta_base] = s.one;
+    if (s.snap_pending) {
         // runs 0 .. snap_nruns-2 are final in cand; the last one was saved
         unsigned long long* ring = e.ring + p.ring_base;
         const unsigned long long* cand = e.cand + p.cand_base;
@@ -1741,17 +1922,161 @@ __device__ __forceinline__ void temporal_target(const Engine& e, uint32_t n, uin
     e.ntp[n] = wq;
 }
 
+// The temporal pattern of the touched targets that keep several reference
+// patterns: kGroup lanes per target, a pattern per lane and round, so that
+// the patterns' sums and comparisons (up to 65,535 of them, each a 48-byte
+// entry) are in flight together.  A thread per target walked them one after
+// the other: 12 us of a 34-us tick with 2 patterns per neuron on a
+// 1,000-neuron network, and 30 us more with 43.  Runs after k_events, beside
+// the fire ordering, so it takes the tick from post_tick.
+template <int kGroup>
 __global__ void __launch_bounds__(kThreads) k_temporal(Engine e) {
-    const uint32_t t = e.ts->tick;
-    const int temporal = e.ts->temporal_enabled;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < e.N; n += gridDim.x * blockDim.x) {
-        const uint32_t len = e.seg_start[n + 1] - e.seg_start[n];
-        if (len == 0) continue;
-        if (e.nparam[n].max_refs == 1) {
-            temporal_target<true>(e, n, len, t, temporal);
-        } else {
-            temporal_target<false>(e, n, len, t, temporal);
+    const uint32_t t = e.ts->post_tick;
+    const int enabled = e.ts->temporal_enabled;
+    const uint32_t sub = threadIdx.x & (kGroup - 1);
+    const uint32_t mask = kGroup == 32 ? 0xffffffffu : ((1u << (kGroup & 31)) - 1u) << (threadIdx.x & 31 & ~(kGroup - 1));
+    const uint32_t groups = gridDim.x * blockDim.x / kGroup;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) / kGroup; n < e.N; n += groups) {
+        const uint32_t k = e.seg_start[n + 1] - e.seg_start[n];
+        if (k == 0) continue;
+        const NeuronParam p = e.nparam[n];
+        if (p.max_refs == 1) continue;  // done by k_events
+        NeuronRec* rec = e.nrec + n;
+        NeuronTp q = e.ntp[n];
+        if (!enabled) {
+            __syncwarp(mask);
+            if (sub == 0) e.ntp[n].last_match = 0;
+            continue;
         }
+        uint32_t match_count = rec->match_count, ws = rec->ws, len = rec->len;
+        unsigned long long* cand = e.cand + p.cand_base;
+        RefMeta* meta = e.refmeta + p.meta_base;
+        unsigned long long* ring = e.ring + p.ring_base;
+        unsigned long long last_run = q.nruns > 0 ? cand[q.nruns - 1] : 0ull;
+        __syncwarp(mask);  // the group has read its state
+        auto ref = [&](uint32_t r) -> RefMeta& { return meta[wrap_add(q.ref_head, r, p.max_refs)]; };
+        if (len == 0 || t - ws > p.window) {
+            ws = t;
+            len = 0;
+            q.nruns = 0;
+            q.cn = 0;
+            for (uint32_t r = sub; r < q.ref_count; r += kGroup) {
+                RefMeta& m = ref(r);
+                m.dot = 0;
+                m.rn = 0;
+                m.cn = 0;
+                m.cur_run = 0;
+                m.cur_pos = 0;
+                m.match = 2;
+            }
+        }
+        const uint32_t o = t - ws;
+        const uint32_t oo = o * o;
+        const bool always = 0.0f >= p.similarity;
+        for (uint32_t j = 0; j < k; ++j) {
+            // one append, and every pattern's comparison with the longer
+            // window; `frozen`: no pattern takes part in a further one
+            const bool grow = q.nruns > 0 && run_value(last_run) == o;
+            if (grow) {
+                last_run += (1ull << 16);
+            } else {
+                if (q.nruns > p.window) {  // cannot happen: at most window+1 distinct offsets
+                    if (sub == 0) raise_status(e, kStatusRunOverflow);
+                    break;
+                }
+                if (sub == 0 && q.nruns > 0) cand[q.nruns - 1] = last_run;
+                last_run = static_cast<unsigned long long>(o) | (1ull << 16);
+                q.nruns += 1;
+            }
+            len += 1;
+            q.cn += oo;
+            bool match = always && q.ref_count > 0 && len >= 2;
+            bool frozen = true;
+            for (uint32_t r0 = 0; r0 < q.ref_count; r0 += kGroup) {
+                bool hit = false, done = true;
+                if (r0 + sub < q.ref_count) {
+                    RefMeta& m = ref(r0 + sub);
+                    const uint32_t mlen = m.len;
+                    uint32_t state = m.match;
+                    done = len >= mlen;
+                    const bool advance = len <= mlen;
+                    if (advance || (state == 2 && !match && len >= 2)) {
+                        RefMeta x = m;
+                        if (advance) {
+                            const unsigned long long run = ring[wrap_add(x.start, x.cur_run, p.ring_cap)];
+                            const uint32_t v = run_value(run);
+                            if (++x.cur_pos == run_count(run)) {
+                                x.cur_run += 1;
+                                x.cur_pos = 0;
+                            }
+                            x.dot += v * o;  // 16-bit values: 32-bit products
+                            x.rn += v * v;
+                            x.cn += oo;
+                            x.match = 2;
+                        }
+                        if (!match && len >= 2) x.match = cos_ge(x.dot, x.rn, x.cn, p.similarity) ? 1 : 0;
+                        state = x.match;
+                        m = x;
+                    }
+                    hit = state == 1;
+                }
+                match = __any_sync(mask, hit && len >= 2) || match;
+                frozen = __all_sync(mask, done) && frozen;
+            }
+            if (match) {
+                q.last_match = 1;
+                match_count += 1;
+                if (frozen) {
+                    // the remaining appends change no pattern's sums: they match too
+                    const uint32_t rest = k - j - 1;
+                    last_run += static_cast<unsigned long long>(rest) << 16;
+                    len += rest;
+                    q.cn += static_cast<unsigned long long>(oo) * rest;
+                    match_count += rest;
+                    break;
+                }
+                continue;
+            }
+            q.last_match = 0;
+            if (len < 2) continue;
+            // learn_pattern (:31-41): FIFO with max_reference_patterns entries
+            if (q.ref_count >= p.max_refs) {
+                q.ring_used -= ref(0).nruns;
+                __syncwarp(mask);
+                q.ref_head = wrap_add(q.ref_head, 1, p.max_refs);
+                q.ref_count -= 1;
+            }
+            if (q.ring_used + q.nruns > p.ring_cap) {
+                if (sub == 0) raise_status(e, kStatusRingOverflow);
+                break;
+            }
+            if (sub == 0) cand[q.nruns - 1] = last_run;
+            __syncwarp(mask);
+            for (uint32_t i = sub; i < q.nruns; i += kGroup) ring[wrap_add(q.ring_head, i, p.ring_cap)] = cand[i];
+            if (sub == 0) {
+                RefMeta x;
+                x.dot = x.rn = x.cn = q.cn;
+                x.start = q.ring_head;
+                x.nruns = q.nruns;
+                x.len = len;
+                x.cur_run = 0;
+                x.cur_pos = 0;
+                x.match = 2;
+                ref(q.ref_count) = x;
+            }
+            q.ring_head = wrap_add(q.ring_head, q.nruns, p.ring_cap);
+            q.ring_used += q.nruns;
+            q.ref_count += 1;
+            __syncwarp(mask);
+        }
+        if (sub == 0) {
+            if (q.nruns > 0) cand[q.nruns - 1] = last_run;
+            rec->match_count = match_count;
+            rec->ws = ws;
+            rec->len = len;
+            e.ntp[n] = q;
+        }
+        __syncwarp(mask);
     }
 }
 
@@ -1791,7 +2116,7 @@ __global__ void k_post(Engine e) {
 }
 
 // Fires in due order, one thread per bitmap word (a tile is kThreads words).
-// k_process counted every tile's fires, so a block finds the first rank of
+// k_events counted every tile's fires, so a block finds the first rank of
 // its tile by adding the counts of the tiles before it.  A fire's rank r is
 // its position in the reference's fire order (due order,
 // NetworkPropagator.cpp:80-93); the fire list and the raster are written here
@@ -1841,7 +2166,7 @@ __global__ void k_fire_list(Engine e) {
 __global__ void __launch_bounds__(kFireCountThreads, 1) k_fire_count(Engine e) {
     tick_enter();
     const uint32_t t = e.ts->tick;
-    // the tick's fire count: the sum of k_process's per-tile counts
+    // the tick's fire count: the sum of k_events' per-tile counts
     const uint32_t tiles = ((e.ts->n_due + 31) / 32 + kThreads - 1) / kThreads;
     __shared__ uint32_t s_nf;
     if (threadIdx.x == 0) s_nf = 0;
@@ -2172,7 +2497,7 @@ static void launch_main(void (*kernel)(Engine), uint32_t grid, uint32_t block, s
     cudaLaunchKernelEx(&cfg, kernel, e);
 }
 
-// Dynamic shared memory of the grouping kernels.
+// Dynamic shared memory of the grouping kernels and of k_events.
 static size_t bucket_smem(const Engine& e) {
     return stream_buf_offset(e.nbuckets) + kStreamBufs * kStreamTile * sizeof(unsigned long long);
 }
@@ -2180,6 +2505,21 @@ static size_t bsort_smem(const Engine& e) {
     return kSortSmemBytes + (static_cast<size_t>(1) << e.bucket_shift) * sizeof(uint32_t);
 }
 static uint32_t bsort_grid(const Engine& e) { return e.nbuckets; }
+static size_t events_smem(uint32_t bucket_shift) {
+    const size_t width = static_cast<size_t>(1) << bucket_shift;
+    return kBlockEvents * (sizeof(BucketEntry) + 2 + 2) + (width <= kSharedParams ? width * sizeof(TargetParam) : 0) +
+           (width + 2) * sizeof(uint32_t);
+}
+
+// k_temporal's lanes per target: a whole warp while every target has one
+// resident at once, 8 lanes on larger networks.
+static void launch_temporal(const Engine& e, cudaStream_t stream) {
+    if (e.N <= e.grid_wide * 32u) {
+        k_temporal<32><<<(e.N + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, stream>>>(e);
+    } else {
+        k_temporal<8><<<e.grid_process, kThreads, 0, stream>>>(e);
+    }
+}
 
 void launch_tick(const Engine& e, const TickStreams& s, cudaEvent_t* marks) {
     const uint32_t wide = e.grid_wide;
@@ -2202,55 +2542,48 @@ void launch_tick(const Engine& e, const TickStreams& s, cudaEvent_t* marks) {
     // k_bcount follows a wait on the side stream: a full dependency
     mark(false); launch_main(k_bcount, e.grid_bucket, kBucketThreads, bucket_smem(e), stream, false, e); mark(true);
     mark(false); launch_main(k_bscatter, e.grid_bucket, kBucketThreads, bucket_smem(e), stream, dep, e); mark(true);
-    mark(false); launch_main(k_bsort, bsort_grid(e), kThreads, bsort_smem(e), stream, dep, e); mark(true);
+    mark(false);
+    launch_main(e.inline_codes ? k_events<true> : k_events<false>,
+                e.grid_events < e.nbuckets ? e.grid_events : e.nbuckets, kEventThreads,
+                events_smem(e.bucket_shift), stream, dep, e);
+    mark(true);
     if (e.side_serial) {
-        // everything in tick order on the main stream; k_temporal, k_events,
-        // k_post and the fire ordering take full dependencies (as
-        // programmatic dependents they made the tick 7 % slower on recog_1m:
-        // their blocks, launched early, held SM resources the kernel before
-        // them needed)
-        side_mark(8, false);
-        launch_main(k_temporal, e.grid_process, kThreads, 0, stream, false, e);
-        side_mark(8, true);
-        mark(false); launch_main(k_events, e.grid_events, kThreads, 0, stream, false, e); mark(true);
-        mark(false); launch_main(k_process, e.grid_walk, kThreads, kProcessSmem, stream, dep, e); mark(true);
-        side_mark(9, false);
-        launch_main(k_post, wide * 4, kThreads, 0, stream, false, e);
-        side_mark(9, true);
+        // everything in tick order on the main stream; k_post and the fire
+        // ordering take full dependencies (as programmatic dependents they
+        // made the tick 7 % slower on recog_1m: their blocks, launched early,
+        // held SM resources the kernel before them needed)
+        side_mark(6, false);
+        launch_main(k_post, wide * 2, kThreads, 0, stream, false, e);
+        side_mark(6, true);
+        side_mark(7, false);
+        if (e.multi_refs) launch_temporal(e, stream);
+        side_mark(7, true);
         mark(false); launch_main(k_fire_list, e.grid_fire, kThreads, 0, stream, false, e); mark(true);
         mark(false); launch_main(k_fire_count, e.grid_wide / 4 + 1, kFireCountThreads, 0, stream, false, e); mark(true);
         mark(false); launch_main(k_expand, e.grid_wide * 4, kThreads, 0, stream, dep, e); mark(true);
         return;
     }
-    // the temporal update forks off here and runs beside k_events / k_process
-    // (it needs only the segment starts)
+    // post-spike STDP of the fired targets and the temporal patterns of the
+    // targets with several reference patterns run beside the fire ordering
+    // and the expansion (which touch neither)
     cudaEventRecord(s.ev[0], stream);
     cudaStreamWaitEvent(s.side, s.ev[0], 0);
-    side_mark(8, false);
-    k_temporal<<<e.grid_process, kThreads, 0, s.side>>>(e);
-    side_mark(8, true);
+    side_mark(6, false);
+    k_post<<<wide, kThreads, 0, s.side>>>(e);
+    side_mark(6, true);
+    side_mark(7, false);
+    if (e.multi_refs) launch_temporal(e, s.side);
+    side_mark(7, true);
     cudaEventRecord(s.ev[1], s.side);
-    mark(false); launch_main(k_events, e.grid_events, kThreads, 0, stream, dep, e); mark(true);
-    mark(false); launch_main(k_process, e.grid_walk, kThreads, kProcessSmem, stream, dep, e); mark(true);
-    // post-spike STDP of the fired targets runs beside the fire ordering and
-    // the expansion (synapse records are not touched by those)
-    cudaEventRecord(s.ev[2], stream);
-    cudaStreamWaitEvent(s.side, s.ev[2], 0);
-    side_mark(9, false);
-    k_post<<<wide * 4, kThreads, 0, s.side>>>(e);
-    side_mark(9, true);
-    cudaEventRecord(s.ev[3], s.side);
     mark(false); launch_main(k_fire_list, e.grid_fire, kThreads, 0, stream, dep, e); mark(true);
-    cudaStreamWaitEvent(stream, s.ev[1], 0);  // k_temporal reads the tick counter k_fire_count advances
-    mark(false); launch_main(k_fire_count, e.grid_wide / 4 + 1, kFireCountThreads, 0, stream, false, e); mark(true);
+    mark(false); launch_main(k_fire_count, e.grid_wide / 4 + 1, kFireCountThreads, 0, stream, dep, e); mark(true);
     mark(false); launch_main(k_expand, e.grid_wide * 4, kThreads, 0, stream, dep, e); mark(true);
-    cudaStreamWaitEvent(stream, s.ev[3], 0);  // the next tick's k_events reads the synapse records
+    cudaStreamWaitEvent(stream, s.ev[1], 0);  // the next tick's k_events reads the records k_post updates
 }
 
 const char* kernel_name(int index) {
-    static const char* names[kKernelCount] = {"k_bcount",    "k_bscatter",  "k_bsort",    "k_events",
-                                              "k_process",   "k_fire_list", "k_fire_count", "k_expand",
-                                              "k_temporal",  "k_post"};
+    static const char* names[kKernelCount] = {"k_bcount",     "k_bscatter", "k_events", "k_fire_list",
+                                              "k_fire_count", "k_expand",   "k_post",   "k_temporal"};
     return index >= 0 && index < kKernelCount ? names[index] : "";
 }
 
@@ -2262,10 +2595,11 @@ void launch_group(const Engine& e, cudaStream_t stream) {
 }
 
 void configure_kernels() {
-    cudaFuncSetAttribute(k_process, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kProcessSmem));
+    const int events_bytes = static_cast<int>(std::max(events_smem(kMaxBucketShift), events_smem(8)));
+    cudaFuncSetAttribute(k_events<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
+    cudaFuncSetAttribute(k_events<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
     const int bucket_bytes =
-        static_cast<int>(stream_buf_offset(kMaxBuckets) + kStreamBufs * kStreamTile * sizeof(unsigned long long));
+        static_cast<int>(stream_buf_offset(kMaxTickBuckets) + kStreamBufs * kStreamTile * sizeof(unsigned long long));
     cudaFuncSetAttribute(k_bcount, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_bytes);
     cudaFuncSetAttribute(k_bscatter, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_bytes);
     cudaFuncSetAttribute(k_bsort, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -205,7 +205,7 @@ struct snncuda_sim {
     uint32_t ticks_per_graph{16};  // ticks captured in graph_many
     uint32_t sms{1};
 
-    // second stream of the tick graphs (k_temporal) and its fork/join events
+    // second stream of the tick graphs and its fork/join events
     cudaStream_t side{nullptr};
     cudaEvent_t tick_ev[4]{};
     // eviction: the device state held in host memory (evict_impl / restore_impl)
@@ -394,6 +394,7 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     std::vector<uint64_t>& in_ptr = pk.in_ptr;
     const uint32_t max_expected = pk.max_expected;
     e.code_stride = max_expected;
+    e.inline_codes = 1;
     sim->c_of_tm.resize(S);
     sim->tm_of_c.resize(S);
     if (S > 0) {
@@ -425,6 +426,8 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
         p.window = static_cast<uint32_t>(window);
         p.similarity = net->similarity_threshold[n];
         p.max_refs = static_cast<uint32_t>(refs);
+        if (refs > 1) e.multi_refs = 1;
+        if (!inline_code_pattern(p.max_refs, max_expected)) e.inline_codes = 0;
         const uint64_t full = refs * (window + 1);
         p.ring_cap = static_cast<uint32_t>(std::min<uint64_t>(full, std::max<uint64_t>(window + 1, run_budget)));
         p.in_begin = in_ptr[n];
@@ -468,7 +471,7 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     // ---- grouping buckets and launch shapes ----
     int sms = 0;
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sim->device), "device attribute");
-    e.bucket_shift = bucket_shift_for(N);
+    e.bucket_shift = tick_bucket_shift(N, static_cast<uint32_t>(std::max(1, sms)));
     if (e.bucket_shift == 0) throw_fail(SNNCUDA_ERR_UNSUPPORTED, "at most 2^28 neurons");
     e.nbuckets = static_cast<uint32_t>(std::max<uint64_t>(1, (static_cast<uint64_t>(N) + (1u << e.bucket_shift) - 1) >> e.bucket_shift));
     // counting and placing blocks: two per SM, fewer for small networks (one
@@ -563,19 +566,13 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     sim->in_ptr = std::move(in_ptr);
 
     e.grid_wide = static_cast<uint32_t>(std::max(1, sms * 2));
-    e.grid_events = e.grid_wide * 4;
+    e.grid_events = e.grid_wide * 8;
     sim->sms = static_cast<uint32_t>(std::max(1, sms));
     e.grid_process = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((N + 255) / 256, sms * 8ull)));
-    // k_process: at least three blocks per SM (of at least 64 targets) so its
-    // one wave covers every SM; at most eight per SM
-    e.grid_walk = static_cast<uint32_t>(std::max<uint64_t>(
-        1, std::min<uint64_t>(std::max<uint64_t>((N + 255) / 256, std::min<uint64_t>(sms * 3ull, (N + 63) / 64)),
-                              sms * 8ull)));
+    e.grid_walk = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((N + 63) / 64, sms * 8ull)));
     e.grid_fire = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(fire_tiles, sms * 8ull)));
-    // large networks: the temporal update and post-spike STDP in tick order
-    // (beside k_events they slowed it by more than their own time on a 1e9-
-    // synapse network, and by about their own time at 1e8 synapses; on a
-    // 2e7-synapse network the overlap still gains 15 %)
+    // large networks: post-spike STDP in tick order (two random-access
+    // kernels side by side slowed each other by more than the overlap gave)
     e.side_serial = e.S >= (1ull << 26) ? 1u : 0u;
     sim->ensure_far(1, 2);
     check(cudaStreamSynchronize(st), "create synchronize");
@@ -829,7 +826,7 @@ double probe_ms_per_tick(snncuda_sim* sim, uint64_t ticks) {
 }
 
 // Picks the launch shapes by timed probes of the next ticks (coordinate
-// descent over k_events, k_process, grouping and k_temporal blocks per SM
+// descent over k_events, grouping and k_temporal blocks per SM
 // and the ticks per captured graph), then sizes the wheel slots to twice the
 // largest due list seen plus 2^16 events when that is smaller than the
 // current capacity.
@@ -839,7 +836,6 @@ void autotune_impl(snncuda_sim* sim, uint64_t probe_ticks, snncuda_tuning* out) 
     run_complete(sim, true);
     Engine& e = sim->e;
     const uint32_t sms = sim->sms;
-    const uint32_t walk_max = static_cast<uint32_t>(std::max<uint64_t>(1, (static_cast<uint64_t>(sim->N) + 63) / 64));
     uint32_t probes = 0;
     double best = probe_ms_per_tick(sim, probe_ticks);
     ++probes;
@@ -850,8 +846,6 @@ void autotune_impl(snncuda_sim* sim, uint64_t probe_ticks, snncuda_tuning* out) 
     };
     std::vector<Knob> knobs = {
         {&e.grid_events, {sms * 4, sms * 8, sms * 16}},
-        {&e.grid_walk, {std::min(walk_max, sms * 2), std::min(walk_max, sms * 3), std::min(walk_max, sms * 4),
-                        std::min(walk_max, sms * 6)}},
         {&e.grid_bucket, {sms, sms * 2, sms * 4}},
         {&e.scatter_pass_events, {kScatterPassEvents / 2, kScatterPassEvents * 2, 0u}},
         {&e.side_serial, {0u, 1u}},

@@ -242,7 +242,7 @@ class Simulation:
         out = _abi.Profile()
         _check(self.lib, self.lib.snncuda_sim_profile(self.handle, int(inclusive_tick), ctypes.byref(out)))
         names = [self.lib.snncuda_kernel_name(k).decode() for k in range(_abi.KERNEL_COUNT)]
-        return {"ticks": int(out.ticks), "kernel_ms": dict(zip(names, list(out.kernel_ms))),
+        return {"ticks": int(out.ticks), "kernel_ms": {n: ms for n, ms in zip(names, list(out.kernel_ms)) if n},
                 "synaptic_events": int(out.synaptic_events), "external_events": int(out.external_events),
                 "fires": int(out.fires), "touched_targets": int(out.touched_targets)}
 
