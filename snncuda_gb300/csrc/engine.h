@@ -352,6 +352,40 @@ void launch_range_counts(const Engine& e, uint32_t n_begin, uint32_t n_end, unsi
 // (k_checksum); out must start at zero.
 void launch_checksum(const Engine& e, uint32_t n_begin, uint32_t n_end, unsigned long long tm_begin,
                      unsigned long long* out, cudaStream_t stream);
+// The readers' fields, one device array each (null: not wanted), in the types
+// of snncuda_neuron_state / snncuda_synapse_state.
+struct NeuronArrays {
+    float* membrane;
+    uint64_t* spikes;
+    int64_t* fired;
+    uint64_t* active;
+    float* current;    // 4 per neuron
+    uint64_t* update;  // 4 per neuron
+    float* tau;        // 4 per neuron
+    uint64_t* window;
+    uint64_t* offsets;
+    uint64_t* learned;
+    uint64_t* matches;
+    uint8_t* match;
+};
+struct SynapseArrays {
+    float* weight;
+    int64_t* pre;
+    int64_t* post;
+    uint64_t* pre_count;
+    uint64_t* updates;
+    float* delta;
+    uint64_t* window;
+    uint64_t* offsets;
+    uint64_t* learned;
+    uint64_t* matches;
+    uint8_t* match;
+};
+// Neurons [n0, n0 + count) into the arrays.
+void launch_unpack_neurons(const Engine& e, uint32_t n0, uint32_t count, const NeuronArrays& out, cudaStream_t stream);
+// The synapses in target-major slots order[0 .. count) into the arrays.
+void launch_unpack_synapses(const Engine& e, const uint32_t* order, uint64_t count, const SynapseArrays& out,
+                            cudaStream_t stream);
 // One-time kernel attributes (dynamic shared memory); call with
 // the device current before the first tick.
 void configure_kernels();

@@ -2360,10 +2360,14 @@ __global__ void k_range_counts(Engine e, uint32_t nb, uint32_t ne, unsigned long
         pre += e.syn[i].b.pre_count;
         code_matches += e.syn[i].b.code_matches;
     }
-    for (uint32_t slot = 0; slot < e.W; ++slot) {
+    // the wheel: blocks share out its slots (the loop over all of them in
+    // every block waited for W slot counts one after the other)
+    const uint32_t parts = gridDim.x > e.W ? gridDim.x / e.W : 1u;
+    for (uint32_t task = blockIdx.x; task < e.W * parts; task += gridDim.x) {
+        const uint32_t slot = task % e.W, part = task / e.W;
         const uint32_t cnt = e.slot_count[slot];
         const unsigned long long* ev = e.wheel + static_cast<size_t>(slot) * e.slot_cap;
-        for (unsigned long long i = first; i < cnt; i += stride) {
+        for (unsigned long long i = part * blockDim.x + threadIdx.x; i < cnt; i += parts * blockDim.x) {
             const uint32_t tgt = static_cast<uint32_t>(ev[i]) & ~kExternalBit;
             wheel += tgt >= nb && tgt < ne;
         }
@@ -2373,6 +2377,53 @@ __global__ void k_range_counts(Engine e, uint32_t nb, uint32_t ne, unsigned long
     if (wheel) atomicAdd(out + 2, wheel);
     if (matches) atomicAdd(out + 3, matches);
     if (code_matches) atomicAdd(out + 4, code_matches);
+}
+
+// Readers: a thread per neuron or synapse; the outputs are coalesced, the
+// synapse records come in Connectome order (one random 64-byte read each).
+__global__ void k_unpack_neurons(Engine e, uint32_t n0, uint32_t count, NeuronArrays o) {
+    constexpr float kTau[4] = {5.0f, 100.0f, 10.0f, 150.0f};  // receptor decay taus
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const NeuronRec r = e.nrec[n0 + i];
+        const NeuronTp q = e.ntp[n0 + i];
+        if (o.current) {
+            reinterpret_cast<float4*>(o.current)[i] = make_float4(r.cur[0], r.cur[1], r.cur[2], r.cur[3]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t code = (r.flags >> (2 * k)) & 3u;
+                o.tau[4ull * i + k] = code == 0 ? kTau[0] : (code == 1 ? kTau[1] : (code == 2 ? kTau[2] : kTau[3]));
+                o.update[4ull * i + k] = r.upd[k];
+            }
+        } else {
+            o.membrane[i] = r.membrane;
+            o.spikes[i] = r.spike_count;
+            o.fired[i] = static_cast<int64_t>(r.last_fired1) - 1;  // 0: none, reads -1
+            o.active[i] = r.last_active;
+            o.window[i] = r.ws;
+            o.offsets[i] = r.len;
+            o.learned[i] = q.ref_count;
+            o.matches[i] = r.match_count;
+            o.match[i] = static_cast<uint8_t>(q.last_match);
+        }
+    }
+}
+
+__global__ void k_unpack_synapses(Engine e, const uint32_t* order, unsigned long long count, SynapseArrays o) {
+    for (unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; i < count;
+         i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
+        const SynAB r = load_record(e.syn + order[i]);
+        o.weight[i] = r.a.weight;
+        o.pre[i] = static_cast<int64_t>(r.a.last_pre1) - 1;  // 0: none, reads -1
+        o.post[i] = static_cast<int64_t>(r.a.last_post1) - 1;
+        o.pre_count[i] = r.b.pre_count;
+        o.updates[i] = r.a.updates;
+        o.delta[i] = r.a.last_delta;
+        o.window[i] = r.b.code_ws;
+        o.offsets[i] = r.b.code_len;
+        o.learned[i] = r.b.learned_count;
+        o.matches[i] = r.b.code_matches;
+        o.match[i] = r.b.flags & 1u;
+    }
 }
 
 // 64-bit mix of one word into a running hash (multiply / xor-shift rounds).
@@ -2468,6 +2519,15 @@ __global__ void k_checksum(Engine e, uint32_t nb, uint32_t ne, unsigned long lon
 void launch_checksum(const Engine& e, uint32_t n_begin, uint32_t n_end, unsigned long long tm_begin,
                      unsigned long long* out, cudaStream_t stream) {
     k_checksum<<<e.grid_wide * 2, kThreads, 0, stream>>>(e, n_begin, n_end, tm_begin, out);
+}
+
+void launch_unpack_neurons(const Engine& e, uint32_t n0, uint32_t count, const NeuronArrays& out, cudaStream_t stream) {
+    k_unpack_neurons<<<e.grid_wide * 4, kThreads, 0, stream>>>(e, n0, count, out);
+}
+
+void launch_unpack_synapses(const Engine& e, const uint32_t* order, uint64_t count, const SynapseArrays& out,
+                            cudaStream_t stream) {
+    k_unpack_synapses<<<e.grid_wide * 4, kThreads, 0, stream>>>(e, order, count, out);
 }
 
 void launch_rule_off(const Engine& e, unsigned long long tm_begin, unsigned long long tm_end, cudaStream_t stream) {

@@ -18,6 +18,7 @@
 #include <map>
 #include <chrono>
 #include <deque>
+#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -26,6 +27,7 @@
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "engine.h"
@@ -188,15 +190,16 @@ struct snncuda_sim {
     unsigned long long* far_ev{nullptr};
     uint32_t* far_idx{nullptr};
     size_t far_ev_cap{0}, far_idx_cap{0};
-    // pinned host staging for injected events and their slot/tick indices
-    unsigned long long* host_ev{nullptr};
-    uint32_t* host_idx{nullptr};
-    size_t host_ev_cap{0}, host_idx_cap{0};
-    // injection staging
-    unsigned long long* inj_ev{nullptr};
-    uint32_t* inj_slot{nullptr};
-    uint32_t* inj_off{nullptr};
-    size_t inj_cap{0}, inj_groups_cap{0};
+    // pinned host staging of a run's injections, in use from a run's first
+    // copy until the run is complete
+    unsigned char* host_stage{nullptr};
+    size_t host_stage_cap{0};
+    bool stage_in_use{false};
+    // device staging of the injections placed at the start of a run: events,
+    // then the groups' slots and offsets
+    unsigned char* inj{nullptr};
+    size_t inj_cap{0};
+    uint32_t far_ticks_set{0};  // TickState::far_ticks on the device between runs
     // graphs
     cudaGraphExec_t graph_many{nullptr};
     cudaGraphExec_t graph_one{nullptr};
@@ -213,7 +216,11 @@ struct snncuda_sim {
     std::vector<std::vector<unsigned char>> evicted_data;  // per owned buffer
     uint64_t evictions{0};
     // asynchronous runs (run_enqueue / run_complete)
-    TickState* ts_pinned{nullptr};  // tick state copied back at the end of a run
+    // tick state and the wheel's slot counts, copied back at the end of a run
+    // (current until the next one starts)
+    TickState* ts_pinned{nullptr};
+    uint32_t* counts_pinned{nullptr};
+    bool pinned_current{false};
     cudaEvent_t run_done{nullptr};
     uint64_t run_target{0};         // inclusive tick of the run in flight
     bool run_in_flight{false};
@@ -223,6 +230,7 @@ struct snncuda_sim {
         for (cudaEvent_t ev : tick_ev)
             if (ev) cudaEventDestroy(ev);
         if (ts_pinned) cudaFreeHost(ts_pinned);
+        if (counts_pinned) cudaFreeHost(counts_pinned);
         if (graph_many) cudaGraphExecDestroy(graph_many);
         if (graph_one) cudaGraphExecDestroy(graph_one);
         if (graph_prof) cudaGraphExecDestroy(graph_prof);
@@ -236,29 +244,21 @@ struct snncuda_sim {
                 if (b.p) cudaFreeAsync(b.p, stream);
         if (far_ev) cudaFreeAsync(far_ev, stream);
         if (far_idx) cudaFreeAsync(far_idx, stream);
-        if (inj_ev) cudaFreeAsync(inj_ev, stream);
-        if (inj_slot) cudaFreeAsync(inj_slot, stream);
-        if (inj_off) cudaFreeAsync(inj_off, stream);
-        if (host_ev) cudaFreeHost(host_ev);
-        if (host_idx) cudaFreeHost(host_idx);
+        if (inj) cudaFreeAsync(inj, stream);
+        if (host_stage) cudaFreeHost(host_stage);
         if (side) cudaStreamDestroy(side);
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
 
-    // Pinned host buffers for the host->device copies of injected events.
-    void ensure_host(size_t events, size_t idx) {
-        if (events > host_ev_cap) {
-            if (host_ev) cudaFreeHost(host_ev);
-            host_ev = nullptr;
-            host_ev_cap = std::max<size_t>(events, 2 * host_ev_cap);
-            check(cudaMallocHost(&host_ev, host_ev_cap * sizeof(unsigned long long)), "pinned staging");
-        }
-        if (idx > host_idx_cap) {
-            if (host_idx) cudaFreeHost(host_idx);
-            host_idx = nullptr;
-            host_idx_cap = std::max<size_t>(idx, 2 * host_idx_cap);
-            check(cudaMallocHost(&host_idx, host_idx_cap * sizeof(uint32_t)), "pinned staging");
-        }
+    // Pinned host buffer for the host->device copies of a run's injections.
+    void ensure_host(size_t bytes) {
+        if (bytes <= host_stage_cap) return;
+        const size_t want = std::max(bytes, 2 * host_stage_cap);
+        if (host_stage) cudaFreeHost(host_stage);
+        host_stage = nullptr;
+        host_stage_cap = 0;
+        check(cudaMallocHost(reinterpret_cast<void**>(&host_stage), want), "pinned staging");
+        host_stage_cap = want;
     }
 
     void drop_graphs() {
@@ -302,23 +302,18 @@ struct snncuda_sim {
         e.far_idx = far_idx;
     }
 
-    void ensure_inject(size_t events, size_t groups) {
-        if (events > inj_cap) {
-            if (inj_ev) cudaFreeAsync(inj_ev, stream);
-            inj_ev = nullptr;
-            inj_cap = std::max<size_t>(events, 2 * inj_cap);
-            check(cudaMallocAsync(&inj_ev, inj_cap * sizeof(unsigned long long), stream), "inject events");
-        }
-        if (groups + 1 > inj_groups_cap) {
-            if (inj_slot) cudaFreeAsync(inj_slot, stream);
-            if (inj_off) cudaFreeAsync(inj_off, stream);
-            inj_slot = nullptr;
-            inj_off = nullptr;
-            inj_groups_cap = std::max<size_t>(groups + 1, 2 * inj_groups_cap);
-            check(cudaMallocAsync(&inj_slot, inj_groups_cap * sizeof(uint32_t), stream), "inject slots");
-            check(cudaMallocAsync(&inj_off, inj_groups_cap * sizeof(uint32_t), stream), "inject offsets");
-        }
+    void ensure_inject(size_t bytes) {
+        if (bytes <= inj_cap) return;
+        const size_t want = std::max(bytes, 2 * inj_cap);
+        if (inj) cudaFreeAsync(inj, stream);
+        inj = nullptr;
+        inj_cap = 0;
+        check(cudaMallocAsync(reinterpret_cast<void**>(&inj), want, stream), "inject staging");
+        inj_cap = want;
     }
+
+    // The tick state after the last run.
+    TickState current_ts() { return pinned_current ? *ts_pinned : read_ts(); }
 
     TickState read_ts() {
         TickState ts;
@@ -650,12 +645,11 @@ void evict_impl(snncuda_sim* sim) {
     for (DeviceBuffer& b : sim->owned)
         if (b.p) check(cudaFreeAsync(b.p, st), "eviction free");
     for (void** p : {reinterpret_cast<void**>(&sim->far_ev), reinterpret_cast<void**>(&sim->far_idx),
-                     reinterpret_cast<void**>(&sim->inj_ev), reinterpret_cast<void**>(&sim->inj_slot),
-                     reinterpret_cast<void**>(&sim->inj_off)}) {
+                     reinterpret_cast<void**>(&sim->inj)}) {
         if (*p) check(cudaFreeAsync(*p, st), "eviction free");
         *p = nullptr;
     }
-    sim->far_ev_cap = sim->far_idx_cap = sim->inj_cap = sim->inj_groups_cap = 0;
+    sim->far_ev_cap = sim->far_idx_cap = sim->inj_cap = 0;
     e.far_ev = nullptr;
     e.far_idx = nullptr;
     check(cudaStreamSynchronize(st), "eviction synchronize");
@@ -993,52 +987,59 @@ void run_enqueue(snncuda_sim* sim, uint64_t T, snncuda_profile* prof) {
     const size_t a_end = first_at_or_after(p + W);
     const size_t b_end = first_at_or_after(T + W);
     cudaStream_t st = sim->stream;
-    if (a_end > 0) {
-        // one group per delivery tick with injections (the queue is in tick
-        // order: each tick's injections are one run, found by binary search)
-        std::vector<uint32_t> slots, offs;
-        for (size_t b = 0; b < a_end;) {
-            const uint64_t tick = base[b].tick;
-            slots.push_back(static_cast<uint32_t>(tick & (W - 1)));
-            offs.push_back(static_cast<uint32_t>(b));
-            b = std::min(a_end, first_at_or_after(tick + 1));
-        }
-        offs.push_back(static_cast<uint32_t>(a_end));
-        sim->ensure_inject(a_end, slots.size());
-        sim->ensure_host(a_end, 2 * slots.size() + 1);
-        unsigned long long* hev = sim->host_ev;
+    // One pinned buffer holds everything the run copies to the device: the
+    // near events with their groups (one per delivery tick: the queue is in
+    // tick order, so each tick's injections are one run, found by binary
+    // search), then the far events with their tick index.  It is free again
+    // when the run is complete.
+    if (sim->stage_in_use) check(cudaStreamSynchronize(st), "staging");  // left by a run that failed to start
+    sim->stage_in_use = false;
+    sim->pinned_current = false;
+    std::vector<uint32_t> slots, offs;
+    for (size_t b = 0; b < a_end;) {
+        const uint64_t tick = base[b].tick;
+        slots.push_back(static_cast<uint32_t>(tick & (W - 1)));
+        offs.push_back(static_cast<uint32_t>(b));
+        b = std::min(a_end, first_at_or_after(tick + 1));
+    }
+    offs.push_back(static_cast<uint32_t>(a_end));
+    const uint32_t far_first = static_cast<uint32_t>(p + W);
+    const size_t far_n = b_end - a_end;
+    const uint32_t far_ticks = far_n > 0 ? static_cast<uint32_t>(T + W - 1 - (p + W) + 1) : 0u;  // deliveries p+W .. T+W-1
+    const size_t near_bytes = a_end > 0 ? a_end * 8 + (slots.size() + offs.size()) * 4 : 0;
+    const size_t far_at = (near_bytes + 7) & ~static_cast<size_t>(7);
+    const size_t far_bytes = far_n > 0 ? far_n * 8 + (static_cast<size_t>(far_ticks) + 1) * 4 : 0;
+    if (near_bytes + far_bytes > 0) {
+        sim->ensure_host(far_at + far_bytes);
+        auto* hev = reinterpret_cast<unsigned long long*>(sim->host_stage);
+        auto* fev = reinterpret_cast<unsigned long long*>(sim->host_stage + far_at);
         parallel_for(a_end, [&](size_t b, size_t en) {
             for (size_t i = b; i < en; ++i) hev[i] = base[i].event;
         });
-        std::copy(slots.begin(), slots.end(), sim->host_idx);
-        std::copy(offs.begin(), offs.end(), sim->host_idx + slots.size());
-        check(cudaMemcpyAsync(sim->inj_ev, sim->host_ev, a_end * 8, cudaMemcpyHostToDevice, st), "inject copy");
-        check(cudaMemcpyAsync(sim->inj_slot, sim->host_idx, slots.size() * 4, cudaMemcpyHostToDevice, st),
-              "inject copy");
-        check(cudaMemcpyAsync(sim->inj_off, sim->host_idx + slots.size(), offs.size() * 4, cudaMemcpyHostToDevice,
-                              st), "inject copy");
-        launch_inject(e, sim->inj_ev, sim->inj_slot, sim->inj_off, static_cast<uint32_t>(slots.size()), st);
-        check(cudaGetLastError(), "inject launch");
-        check(cudaStreamSynchronize(st), "inject synchronize");
-    }
-    uint32_t far_first = static_cast<uint32_t>(p + W);
-    uint32_t far_ticks = 0;
-    if (b_end > a_end) {
-        far_ticks = static_cast<uint32_t>(T + W - 1 - (p + W) + 1);  // deliveries p+W .. T+W-1
-        const size_t n = b_end - a_end;
-        sim->ensure_far(n, static_cast<size_t>(far_ticks) + 1);
-        sim->ensure_host(n, static_cast<size_t>(far_ticks) + 1);
-        uint32_t* idx = sim->host_idx;  // idx[j]: far injections due before far_first + j
-        for (uint32_t j = 0; j < far_ticks; ++j) idx[j] = static_cast<uint32_t>(first_at_or_after(far_first + j) - a_end);
-        idx[far_ticks] = static_cast<uint32_t>(n);
-        unsigned long long* hev = sim->host_ev;
-        parallel_for(n, [&](size_t b, size_t en) {
-            for (size_t i = b; i < en; ++i) hev[i] = base[a_end + i].event;
+        parallel_for(far_n, [&](size_t b, size_t en) {
+            for (size_t i = b; i < en; ++i) fev[i] = base[a_end + i].event;
         });
-        check(cudaMemcpyAsync(sim->far_ev, sim->host_ev, n * 8, cudaMemcpyHostToDevice, st), "far copy");
-        check(cudaMemcpyAsync(sim->far_idx, idx, (static_cast<size_t>(far_ticks) + 1) * 4, cudaMemcpyHostToDevice,
-                              st), "far copy");
-        check(cudaStreamSynchronize(st), "far copy");
+        sim->stage_in_use = true;
+        if (a_end > 0) {
+            sim->ensure_inject(near_bytes);
+            std::copy(slots.begin(), slots.end(), reinterpret_cast<uint32_t*>(hev + a_end));
+            std::copy(offs.begin(), offs.end(), reinterpret_cast<uint32_t*>(hev + a_end) + slots.size());
+            check(cudaMemcpyAsync(sim->inj, hev, near_bytes, cudaMemcpyHostToDevice, st), "inject copy");
+            const auto* ev = reinterpret_cast<const unsigned long long*>(sim->inj);
+            const auto* idx = reinterpret_cast<const uint32_t*>(ev + a_end);
+            launch_inject(e, ev, idx, idx + slots.size(), static_cast<uint32_t>(slots.size()), st);
+            check(cudaGetLastError(), "inject launch");
+        }
+        if (far_n > 0) {
+            sim->ensure_far(far_n, static_cast<size_t>(far_ticks) + 1);
+            uint32_t* idx = reinterpret_cast<uint32_t*>(fev + far_n);  // idx[j]: far injections due before far_first + j
+            for (uint32_t j = 0; j < far_ticks; ++j)
+                idx[j] = static_cast<uint32_t>(first_at_or_after(far_first + j) - a_end);
+            idx[far_ticks] = static_cast<uint32_t>(far_n);
+            check(cudaMemcpyAsync(sim->far_ev, fev, far_n * 8, cudaMemcpyHostToDevice, st), "far copy");
+            check(cudaMemcpyAsync(sim->far_idx, idx, (static_cast<size_t>(far_ticks) + 1) * 4, cudaMemcpyHostToDevice,
+                                  st), "far copy");
+        }
     }
     sim->pend_head += b_end;
     if (sim->pend_head == pend.size()) {
@@ -1055,10 +1056,15 @@ void run_enqueue(snncuda_sim* sim, uint64_t T, snncuda_profile* prof) {
         sim->pend_head = 0;
     }
     // run parameters live in device memory so the captured graphs stay valid
-    check(cudaMemcpyAsync(reinterpret_cast<char*>(e.ts) + offsetof(TickState, far_first_tick), &far_first, 4,
-                          cudaMemcpyHostToDevice, st), "run params");
-    check(cudaMemcpyAsync(reinterpret_cast<char*>(e.ts) + offsetof(TickState, far_ticks), &far_ticks, 4,
-                          cudaMemcpyHostToDevice, st), "run params");
+    auto set_far = [&](uint32_t n) {
+        if (n == 0 && sim->far_ticks_set == 0) return;
+        const uint32_t params[2] = {far_first, n};
+        static_assert(offsetof(TickState, far_ticks) == offsetof(TickState, far_first_tick) + 4, "copied together");
+        check(cudaMemcpyAsync(reinterpret_cast<char*>(e.ts) + offsetof(TickState, far_first_tick), params,
+                              sizeof(params), cudaMemcpyHostToDevice, st), "run params");
+        sim->far_ticks_set = n;
+    };
+    set_far(far_ticks);
     uint64_t ticks = T - p + 1;
     if (prof != nullptr) {
         const TickState before = sim->read_ts();
@@ -1091,12 +1097,16 @@ void run_enqueue(snncuda_sim* sim, uint64_t T, snncuda_profile* prof) {
         check(cudaGraphLaunch(sim->graph_one, st), "graph launch");
         ticks -= 1;
     }
-    const uint32_t zero = 0;
-    check(cudaMemcpyAsync(reinterpret_cast<char*>(e.ts) + offsetof(TickState, far_ticks), &zero, 4,
-                          cudaMemcpyHostToDevice, st), "run params");
-    if (sim->ts_pinned == nullptr) check(cudaMallocHost(&sim->ts_pinned, sizeof(TickState)), "pinned tick state");
+    set_far(0);
+    if (sim->ts_pinned == nullptr)
+        check(cudaMallocHost(reinterpret_cast<void**>(&sim->ts_pinned), sizeof(TickState)), "pinned tick state");
+    if (sim->counts_pinned == nullptr)
+        check(cudaMallocHost(reinterpret_cast<void**>(&sim->counts_pinned), e.W * sizeof(uint32_t)),
+              "pinned slot counts");
     if (sim->run_done == nullptr) check(cudaEventCreateWithFlags(&sim->run_done, cudaEventDisableTiming), "event");
     check(cudaMemcpyAsync(sim->ts_pinned, e.ts, sizeof(TickState), cudaMemcpyDeviceToHost, st), "read tick state");
+    check(cudaMemcpyAsync(sim->counts_pinned, e.slot_count, e.W * sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
+          "read slot counts");
     check(cudaEventRecord(sim->run_done, st), "event record");
     sim->run_target = T;
     sim->run_in_flight = true;
@@ -1114,6 +1124,8 @@ bool run_complete(snncuda_sim* sim, bool wait) {
         check(q, "run query");
     }
     sim->run_in_flight = false;
+    sim->stage_in_use = false;
+    sim->pinned_current = true;
     const TickState ts = *sim->ts_pinned;
     const uint64_t T = sim->run_target;
     sim->next_tick = T + 1;
@@ -1200,6 +1212,66 @@ HostState fetch_all(snncuda_sim* sim, bool temporal) {
         h.lcode = sim->d2h(e.lcode, lcode);
     }
     return h;
+}
+
+// Neurons or synapses from which a read unpacks the records on the device:
+// below, copying the records and filling the caller's arrays here is as quick
+// as a copy per array (64 bytes a record, under 1 MB).
+constexpr uint64_t kUnpackFrom = 8192;
+
+// The caller's arrays of one read and their places in the device buffer that
+// the unpacking kernel fills for up to `cap` records at a time.  The buffers
+// are a tick's scratch, whose contents nothing needs between ticks: three of
+// 16 bytes per slot event, so half as many records of 32 bytes in each.
+struct UnpackBuffers {
+    unsigned char* block[3];
+    uint64_t cap;
+    explicit UnpackBuffers(const Engine& e)
+        : block{reinterpret_cast<unsigned char*>(e.grp_tmp), reinterpret_cast<unsigned char*>(e.evin),
+                reinterpret_cast<unsigned char*>(e.ev_a0)},
+          cap(e.slot_cap / 2) {}
+    template <typename T>
+    T* at(int b, uint64_t bytes_per_record) const {
+        return reinterpret_cast<T*>(block[b] + bytes_per_record * cap);
+    }
+};
+static_assert(sizeof(BucketEntry) == 16 && sizeof(EvIn) == 16 && sizeof(SynPre) == 16, "UnpackBuffers' blocks");
+
+// Has the host map the pages of the caller's arrays, which the device is about
+// to overwrite whole: a copy that faults in fresh pages itself (arrays the
+// caller has just allocated) took 48 ms for 73 MB in 11 arrays; a write to
+// each page first makes it 4.4 ms, from 4 threads 3.0 (8: 3.0), 1.5 of them the
+// copies.
+void map_pages(std::initializer_list<std::pair<void*, uint64_t>> arrays) {
+    constexpr uint64_t kPage = 4096, kPerThread = 4u << 20;
+    uint64_t total = 0;
+    for (const auto& [p, bytes] : arrays) total += p ? bytes : 0;
+    const uint64_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const uint64_t threads = std::max<uint64_t>(1, std::min<uint64_t>({4, hw, total / kPerThread}));
+    auto touch = [&](uint64_t t) {
+        for (const auto& [p, bytes] : arrays) {
+            if (p == nullptr || bytes == 0) continue;
+            auto* c = static_cast<volatile unsigned char*>(p);
+            const uint64_t end = bytes * (t + 1) / threads;
+            for (uint64_t i = bytes * t / threads; i < end; i += kPage) c[i] = 0;
+            if (t + 1 == threads) c[bytes - 1] = 0;
+        }
+    };
+    std::vector<std::thread> pool;
+    uint64_t t = 1;
+    try {
+        for (; t < threads; ++t) pool.emplace_back(touch, t);
+    } catch (...) {
+        // a thread that could not start: its share is done here
+    }
+    touch(0);
+    for (; t < threads; ++t) touch(t);
+    for (std::thread& th : pool) th.join();
+}
+
+template <typename T>
+void copy_out(snncuda_sim* sim, T* dst, const void* src, uint64_t count) {
+    if (dst) check(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyDeviceToHost, sim->stream), "read state");
 }
 
 template <typename F>
@@ -1335,10 +1407,13 @@ int snncuda_sim_counters(snncuda_sim* sim, snncuda_counters* out) {
     if (sim == nullptr || out == nullptr) return set_error(SNNCUDA_ERR_INVALID_ARGUMENT, "null argument");
     return guarded([&] {
         resident(sim);
-        const TickState ts = sim->read_ts();
-        const std::vector<uint32_t> counts = sim->d2h(sim->e.slot_count, sim->e.W);
         uint64_t pending = sim->pending.size() - sim->pend_head;
-        for (uint32_t c : counts) pending += c;
+        if (sim->pinned_current) {
+            for (uint32_t i = 0; i < sim->e.W; ++i) pending += sim->counts_pinned[i];
+        } else {
+            for (uint32_t c : sim->d2h(sim->e.slot_count, sim->e.W)) pending += c;
+        }
+        const TickState ts = sim->current_ts();
         out->delivered_spikes = ts.delivered;
         out->fired_spikes = ts.fired;
         out->external_events = ts.external;
@@ -1358,8 +1433,57 @@ int snncuda_sim_idle(snncuda_sim* sim, int32_t* out) {
     return rc;
 }
 
+static void unpack_neurons(snncuda_sim* sim, uint32_t n0, uint32_t n1, const snncuda_neuron_state* o) {
+    const UnpackBuffers buf(sim->e);
+    const uint64_t n = n1 - n0;
+    map_pages({{o->membrane_potential, 4 * n}, {o->spike_count, 8 * n}, {o->last_fired_tick, 8 * n},
+               {o->last_active_tick, 8 * n}, {o->compartment_current, 16 * n}, {o->compartment_last_update, 32 * n},
+               {o->compartment_tau, 16 * n}, {o->window_start_tick, 8 * n}, {o->offset_count, 8 * n},
+               {o->learned_count, 8 * n}, {o->match_count, 8 * n}, {o->last_match, n}});
+    // 16 words of 4 bytes, 6 of 8 bytes and a byte per neuron, in two rounds
+    // of the buffers' 96 bytes: compartments first, then the rest
+    for (uint64_t i = 0; i < n; i += buf.cap) {
+        const uint64_t m = std::min<uint64_t>(buf.cap, n - i);
+        NeuronArrays d{};
+        d.current = buf.at<float>(0, 0);
+        d.tau = buf.at<float>(0, 16);
+        d.update = buf.at<uint64_t>(1, 0);
+        launch_unpack_neurons(sim->e, n0 + static_cast<uint32_t>(i), static_cast<uint32_t>(m), d, sim->stream);
+        check(cudaGetLastError(), "unpack launch");
+        copy_out(sim, o->compartment_current ? o->compartment_current + 4 * i : nullptr, d.current, 4 * m);
+        copy_out(sim, o->compartment_tau ? o->compartment_tau + 4 * i : nullptr, d.tau, 4 * m);
+        copy_out(sim, o->compartment_last_update ? o->compartment_last_update + 4 * i : nullptr, d.update, 4 * m);
+        d = NeuronArrays{};
+        d.spikes = buf.at<uint64_t>(0, 0);
+        d.fired = buf.at<int64_t>(0, 8);
+        d.active = buf.at<uint64_t>(0, 16);
+        d.window = buf.at<uint64_t>(0, 24);
+        d.offsets = buf.at<uint64_t>(1, 0);
+        d.learned = buf.at<uint64_t>(1, 8);
+        d.matches = buf.at<uint64_t>(1, 16);
+        d.membrane = buf.at<float>(1, 24);
+        d.match = buf.at<uint8_t>(1, 28);
+        launch_unpack_neurons(sim->e, n0 + static_cast<uint32_t>(i), static_cast<uint32_t>(m), d, sim->stream);
+        check(cudaGetLastError(), "unpack launch");
+        copy_out(sim, o->spike_count ? o->spike_count + i : nullptr, d.spikes, m);
+        copy_out(sim, o->last_fired_tick ? o->last_fired_tick + i : nullptr, d.fired, m);
+        copy_out(sim, o->last_active_tick ? o->last_active_tick + i : nullptr, d.active, m);
+        copy_out(sim, o->window_start_tick ? o->window_start_tick + i : nullptr, d.window, m);
+        copy_out(sim, o->offset_count ? o->offset_count + i : nullptr, d.offsets, m);
+        copy_out(sim, o->learned_count ? o->learned_count + i : nullptr, d.learned, m);
+        copy_out(sim, o->match_count ? o->match_count + i : nullptr, d.matches, m);
+        copy_out(sim, o->membrane_potential ? o->membrane_potential + i : nullptr, d.membrane, m);
+        copy_out(sim, o->last_match ? o->last_match + i : nullptr, d.match, m);
+    }
+    check(cudaStreamSynchronize(sim->stream), "read neurons");
+}
+
 // Neurons [n0, n1) into o[0 .. n1-n0).
 static void read_neurons_range(snncuda_sim* sim, uint32_t n0, uint32_t n1, const snncuda_neuron_state* o) {
+    if (n1 - n0 >= kUnpackFrom) {
+        unpack_neurons(sim, n0, n1, o);
+        return;
+    }
     const std::vector<NeuronRec> r = sim->d2h(sim->e.nrec + n0, n1 - n0);
     const std::vector<NeuronTp> q = sim->d2h(sim->e.ntp + n0, n1 - n0);
     for (uint32_t i = 0; i < n1 - n0; ++i) {
@@ -1388,10 +1512,59 @@ int snncuda_sim_read_neurons(snncuda_sim* sim, const snncuda_neuron_state* o) {
     });
 }
 
+// Synapses of Connectome indices [c0, c1) into o[0 .. c1-c0): a kernel gathers
+// the records in Connectome order into one array per field, which the copies
+// then move as they are (filling the caller's 11 arrays here took one thread
+// 52 ns a synapse, most of it cache misses of the order).
+static void unpack_synapses(snncuda_sim* sim, uint64_t c0, uint64_t c1, const snncuda_synapse_state* o) {
+    const UnpackBuffers buf(sim->e);
+    const uint64_t n = c1 - c0;
+    map_pages({{o->weight, 4 * n}, {o->last_pre_spike_tick, 8 * n}, {o->last_post_spike_tick, 8 * n},
+               {o->pre_spike_count, 8 * n}, {o->plasticity_update_count, 8 * n}, {o->last_weight_delta, 4 * n},
+               {o->code_window_start_tick, 8 * n}, {o->code_offset_count, 8 * n}, {o->learned_code_count, 8 * n},
+               {o->code_match_count, 8 * n}, {o->last_code_match, n}});
+    for (uint64_t i = 0; i < n; i += buf.cap) {
+        const uint64_t m = std::min<uint64_t>(buf.cap, n - i);
+        SynapseArrays d{};
+        d.pre = buf.at<int64_t>(0, 0);
+        d.post = buf.at<int64_t>(0, 8);
+        d.pre_count = buf.at<uint64_t>(0, 16);
+        d.updates = buf.at<uint64_t>(0, 24);
+        d.window = buf.at<uint64_t>(1, 0);
+        d.offsets = buf.at<uint64_t>(1, 8);
+        d.learned = buf.at<uint64_t>(1, 16);
+        d.matches = buf.at<uint64_t>(1, 24);
+        d.weight = buf.at<float>(2, 0);
+        d.delta = buf.at<float>(2, 4);
+        d.match = buf.at<uint8_t>(2, 12);
+        uint32_t* order = buf.at<uint32_t>(2, 8);
+        check(cudaMemcpyAsync(order, sim->tm_of_c.data() + c0 + i, m * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                              sim->stream), "synapse order");
+        launch_unpack_synapses(sim->e, order, m, d, sim->stream);
+        check(cudaGetLastError(), "unpack launch");
+        copy_out(sim, o->weight ? o->weight + i : nullptr, d.weight, m);
+        copy_out(sim, o->last_pre_spike_tick ? o->last_pre_spike_tick + i : nullptr, d.pre, m);
+        copy_out(sim, o->last_post_spike_tick ? o->last_post_spike_tick + i : nullptr, d.post, m);
+        copy_out(sim, o->pre_spike_count ? o->pre_spike_count + i : nullptr, d.pre_count, m);
+        copy_out(sim, o->plasticity_update_count ? o->plasticity_update_count + i : nullptr, d.updates, m);
+        copy_out(sim, o->last_weight_delta ? o->last_weight_delta + i : nullptr, d.delta, m);
+        copy_out(sim, o->code_window_start_tick ? o->code_window_start_tick + i : nullptr, d.window, m);
+        copy_out(sim, o->code_offset_count ? o->code_offset_count + i : nullptr, d.offsets, m);
+        copy_out(sim, o->learned_code_count ? o->learned_code_count + i : nullptr, d.learned, m);
+        copy_out(sim, o->code_match_count ? o->code_match_count + i : nullptr, d.matches, m);
+        copy_out(sim, o->last_code_match ? o->last_code_match + i : nullptr, d.match, m);
+    }
+    check(cudaStreamSynchronize(sim->stream), "read synapses");
+}
+
 // Synapses of Connectome indices [c0, c1), whose target-major slots are
 // [t0, t1), into o[0 .. c1-c0).
 static void read_synapses_range(snncuda_sim* sim, uint64_t c0, uint64_t c1, uint64_t t0, uint64_t t1,
                          const snncuda_synapse_state* o) {
+    if (c1 - c0 >= kUnpackFrom) {
+        unpack_synapses(sim, c0, c1, o);
+        return;
+    }
     const std::vector<SynAB> rec = sim->d2h(sim->e.syn + t0, t1 - t0);
     for (uint64_t tm = t0; tm < t1; ++tm) {
         const uint64_t i = sim->c_of_tm[tm] - c0;
@@ -1409,7 +1582,6 @@ static void read_synapses_range(snncuda_sim* sim, uint64_t c0, uint64_t c1, uint
         if (o->code_match_count) o->code_match_count[i] = b.code_matches;
         if (o->last_code_match) o->last_code_match[i] = b.flags & 1u;
     }
-    (void)c1;
 }
 
 int snncuda_sim_read_synapses(snncuda_sim* sim, const snncuda_synapse_state* o) {
@@ -1558,25 +1730,30 @@ const char* snncuda_kernel_name(int32_t index) { return kernel_name(index); }
 
 namespace {
 
-// Device checksums of a range of neurons and target-major synapses.
-void checksum_range(snncuda_sim* sim, uint32_t n0, uint32_t n1, uint64_t t0, uint64_t t1, uint64_t* neuron_sum,
-                    uint64_t* synapse_sum) {
+// A range of neurons and their incoming synapses (from target-major slot tm).
+struct CheckRange {
+    uint32_t n0, n1;
+    uint64_t tm;
+};
+
+// Device checksums of the ranges: out[2 i] of the neurons, out[2 i + 1] of the
+// synapses.
+std::vector<unsigned long long> checksum_ranges(snncuda_sim* sim, const std::vector<CheckRange>& ranges) {
     cudaStream_t st = sim->stream;
+    std::vector<unsigned long long> c(2 * ranges.size());
+    if (c.empty()) return c;
     unsigned long long* d = nullptr;
-    check(cudaMallocAsync(&d, 2 * sizeof(unsigned long long), st), "device allocation");
-    unsigned long long c[2] = {};
-    cudaError_t err = cudaMemsetAsync(d, 0, sizeof(c), st);
-    if (err == cudaSuccess) {
-        launch_checksum(sim->e, n0, n1, t0, d, st);
-        (void)t1;
+    check(cudaMallocAsync(&d, c.size() * sizeof(c[0]), st), "device allocation");
+    cudaError_t err = cudaMemsetAsync(d, 0, c.size() * sizeof(c[0]), st);
+    for (size_t i = 0; i < ranges.size() && err == cudaSuccess; ++i) {
+        launch_checksum(sim->e, ranges[i].n0, ranges[i].n1, ranges[i].tm, d + 2 * i, st);
         err = cudaGetLastError();
     }
-    if (err == cudaSuccess) err = cudaMemcpyAsync(c, d, sizeof(c), cudaMemcpyDeviceToHost, st);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(c.data(), d, c.size() * sizeof(c[0]), cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(d, st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(st);
     check(err, "state checksum");
-    if (neuron_sum) *neuron_sum = c[0];
-    if (synapse_sum) *synapse_sum = c[1];
+    return c;
 }
 
 }  // namespace
@@ -1585,7 +1762,9 @@ int snncuda_sim_state_checksum(snncuda_sim* sim, uint64_t* neuron_sum, uint64_t*
     if (sim == nullptr) return set_error(SNNCUDA_ERR_INVALID_ARGUMENT, "null sim");
     return guarded([&] {
         resident(sim);
-        checksum_range(sim, 0, sim->N, 0, sim->S, neuron_sum, synapse_sum);
+        const auto c = checksum_ranges(sim, {{0, sim->N, 0}});
+        if (neuron_sum) *neuron_sum = c[0];
+        if (synapse_sum) *synapse_sum = c[1];
     });
 }
 
@@ -1805,7 +1984,7 @@ int snncuda_sim_read_raster(snncuda_sim* sim, uint64_t first, uint64_t count, ui
     if (sim == nullptr) return set_error(SNNCUDA_ERR_INVALID_ARGUMENT, "null sim");
     return guarded([&] {
         resident(sim);
-        const TickState ts = sim->read_ts();
+        const TickState ts = sim->current_ts();
         const uint64_t have = std::min<uint64_t>(ts.raster_count, sim->e.raster_cap);
         if (first + count > have) throw_fail(SNNCUDA_ERR_INVALID_ARGUMENT, "raster range out of bounds");
         const std::vector<uint32_t> r = sim->d2h(sim->e.raster + 2 * first, 2 * count);
@@ -1935,7 +2114,7 @@ static snncuda_batch* batch_create_impl(uint32_t count, const snncuda_network* n
 // The network's fire records, in order, from the batch's raster.
 static void batch_raster(snncuda_batch* b, uint32_t i, std::vector<uint64_t>& ticks, std::vector<uint32_t>& neurons) {
     snncuda_sim* sim = b->sim;
-    const TickState ts = sim->read_ts();
+    const TickState ts = sim->current_ts();
     const uint64_t have = std::min<uint64_t>(ts.raster_count, sim->e.raster_cap);
     const std::vector<uint32_t> r = sim->d2h(sim->e.raster, 2 * have);
     ticks.clear();
@@ -2010,7 +2189,8 @@ int snncuda_batch_counters(snncuda_batch* b, uint32_t i, snncuda_counters* out) 
         check(cudaGetLastError(), "count launch");
         unsigned long long c[5];
         check(cudaMemcpyAsync(c, b->d_counts, sizeof(c), cudaMemcpyDeviceToHost, st), "counts");
-        const TickState ts = sim->read_ts();  // synchronizes the stream
+        check(cudaStreamSynchronize(st), "counts");
+        const TickState ts = sim->current_ts();
         uint64_t external = 0;
         for (uint64_t t : b->inj_ticks[i]) external += t < sim->next_tick;
         uint64_t pending = c[2];
@@ -2055,9 +2235,13 @@ int snncuda_batch_state_digests(snncuda_batch* b, uint64_t* neuron_digests, uint
 int snncuda_batch_state_checksums(snncuda_batch* b, uint64_t* neuron_sums, uint64_t* synapse_sums) {
     if (b == nullptr) return set_error(SNNCUDA_ERR_INVALID_ARGUMENT, "null batch");
     return guarded([&] {
-        for (uint32_t i = 0; i < b->count; ++i)
-            checksum_range(b->sim, b->nbase[i], b->nbase[i + 1], b->tm_begin(i), b->tm_end(i),
-                           neuron_sums ? neuron_sums + i : nullptr, synapse_sums ? synapse_sums + i : nullptr);
+        std::vector<CheckRange> ranges;
+        for (uint32_t i = 0; i < b->count; ++i) ranges.push_back({b->nbase[i], b->nbase[i + 1], b->tm_begin(i)});
+        const auto c = checksum_ranges(b->sim, ranges);
+        for (uint32_t i = 0; i < b->count; ++i) {
+            if (neuron_sums) neuron_sums[i] = c[2 * i];
+            if (synapse_sums) synapse_sums[i] = c[2 * i + 1];
+        }
     });
 }
 
