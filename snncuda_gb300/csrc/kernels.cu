@@ -2442,6 +2442,8 @@ __device__ __forceinline__ unsigned long long record_hash(unsigned long long ind
     return h;
 }
 
+constexpr int checksum_blocks(bool inline_codes) { return inline_codes ? 8 : 4; }  // per SM
+
 // Order-independent checksums of neurons [nb, ne) (NeuronRec + NeuronTp)
 // and of their incoming synapses: the sum over records of a hash of (index
 // within the range, the record's meaning).  A synapse contributes its SynA
@@ -2450,7 +2452,14 @@ __device__ __forceinline__ unsigned long long record_hash(unsigned long long ind
 // (inline in the record or in the pattern pool, which depends on the widest
 // code of the whole simulation), so a batch member and its solo run give
 // equal sums exactly when their states are equal (up to hash collisions).
-__global__ void k_checksum(Engine e, uint32_t nb, uint32_t ne, unsigned long long tb, unsigned long long* out) {
+//
+// Bound by the hash's instructions (about 19 words a record, a 64-bit multiply
+// each).  kInline (every learned code pattern in its record): a thread per
+// synapse over the whole range with eight blocks per SM, 5.4 -> 3.3 ms for 2e8
+// synapses (12.8 GB, 3.9 TB/s); a warp per target had four, ran a partial
+// round at the end of every target and chose the patterns' place per record.
+template <bool kInline>
+__global__ void __launch_bounds__(kThreads, checksum_blocks(kInline)) k_checksum(const __grid_constant__ Engine e, uint32_t nb, uint32_t ne, unsigned long long tb, unsigned long long* out) {
     const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
     const unsigned long long first = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
     unsigned long long hn = 0, hs = 0;
@@ -2470,38 +2479,60 @@ __global__ void k_checksum(Engine e, uint32_t nb, uint32_t ne, unsigned long lon
         }
         hn += record_hash<24>(n - nb, w);
     }
-    // synapses: a warp per target
-    const uint32_t lane = threadIdx.x & 31;
-    const unsigned long long warps = stride / 32;
-    for (unsigned long long n = nb + first / 32; n < ne; n += warps) {
-        const NeuronParam p = e.nparam[n];
-        const bool inl = inline_code_pattern(p.max_refs, e.code_stride);
-        for (unsigned long long i = e.in_ptr[n] + lane; i < e.in_ptr[n + 1]; i += 32) {
-            const SynAB rec = e.syn[i];
-            const SynA& a = rec.a;
-            const SynB& sb = rec.b;
-            unsigned long long h = mix64(0x6a09e667f3bcc908ull, i - tb);
-            h = mix64(h, __float_as_uint(a.weight));
-            h = mix64(h, a.last_pre1);
-            h = mix64(h, a.last_post1);
-            h = mix64(h, a.meta & ~(1u << kMetaRuleOffBit));
-            h = mix64(h, __float_as_uint(a.clamp_hi));
-            h = mix64(h, a.updates);
-            h = mix64(h, __float_as_uint(a.last_delta));
-            h = mix64(h, a.post_cnt);
-            h = mix64(h, sb.pre_count);
-            h = mix64(h, sb.code_ws);
-            h = mix64(h, sb.code_matches);
-            h = mix64(h, sb.code_len | (static_cast<uint32_t>(sb.flags) << 8) |
-                             (static_cast<uint32_t>(sb.learned_count) << 16));
-            for (uint32_t j = 0; j < sb.code_len; ++j) h = mix64(h, ring_get(sb.ring_lo, sb.ring_hi, j));
-            const uint32_t expected = (a.meta >> kMetaExpectedShift) & 15u;
-            const uint16_t* lc =
-                e.lcode + p.lcode_base + static_cast<size_t>(i - p.in_begin) * p.max_refs * e.code_stride;
-            for (uint32_t k = 0; k < sb.learned_count; ++k)
-                for (uint32_t j = 0; j < expected; ++j)
-                    h = mix64(h, inl ? ring_get(sb.ring_hi, 0ull, j) : lc[static_cast<size_t>(k) * e.code_stride + j]);
+    // a record's words but its learned code patterns
+    auto synapse_hash = [&](unsigned long long index, const SynAB& rec) {
+        const SynA& a = rec.a;
+        const SynB& sb = rec.b;
+        unsigned long long h = mix64(0x6a09e667f3bcc908ull, index);
+        h = mix64(h, __float_as_uint(a.weight));
+        h = mix64(h, a.last_pre1);
+        h = mix64(h, a.last_post1);
+        h = mix64(h, a.meta & ~(1u << kMetaRuleOffBit));
+        h = mix64(h, __float_as_uint(a.clamp_hi));
+        h = mix64(h, a.updates);
+        h = mix64(h, __float_as_uint(a.last_delta));
+        h = mix64(h, a.post_cnt);
+        h = mix64(h, sb.pre_count);
+        h = mix64(h, sb.code_ws);
+        h = mix64(h, sb.code_matches);
+        return mix64(h, sb.code_len | (static_cast<uint32_t>(sb.flags) << 8) |
+                            (static_cast<uint32_t>(sb.learned_count) << 16));
+    };
+    if constexpr (kInline) {
+        const unsigned long long te = e.in_ptr[ne];
+        for (unsigned long long i = tb + first; i < te; i += stride) {
+            const SynAB rec = load_record(e.syn + i);
+            unsigned long long h = synapse_hash(i - tb, rec);
+            const uint32_t expected = (rec.a.meta >> kMetaExpectedShift) & 15u;
+            const uint32_t learned = rec.b.learned_count ? expected : 0u;  // one pattern at most
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                if (j < rec.b.code_len) h = mix64(h, static_cast<uint32_t>(rec.b.ring_lo >> (16 * j)) & 0xFFFFu);
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                if (j < learned) h = mix64(h, static_cast<uint32_t>(rec.b.ring_hi >> (16 * j)) & 0xFFFFu);
             hs += h;
+        }
+    } else {
+        // a warp per target
+        const uint32_t lane = threadIdx.x & 31;
+        const unsigned long long warps = stride / 32;
+        for (unsigned long long n = nb + first / 32; n < ne; n += warps) {
+            const NeuronParam p = e.nparam[n];
+            const bool inl = inline_code_pattern(p.max_refs, e.code_stride);
+            for (unsigned long long i = e.in_ptr[n] + lane; i < e.in_ptr[n + 1]; i += 32) {
+                const SynAB rec = load_record(e.syn + i);
+                const SynB& sb = rec.b;
+                unsigned long long h = synapse_hash(i - tb, rec);
+                for (uint32_t j = 0; j < sb.code_len; ++j) h = mix64(h, ring_get(sb.ring_lo, sb.ring_hi, j));
+                const uint32_t expected = (rec.a.meta >> kMetaExpectedShift) & 15u;
+                const uint16_t* lc =
+                    e.lcode + p.lcode_base + static_cast<size_t>(i - p.in_begin) * p.max_refs * e.code_stride;
+                for (uint32_t k = 0; k < sb.learned_count; ++k)
+                    for (uint32_t j = 0; j < expected; ++j)
+                        h = mix64(h, inl ? ring_get(sb.ring_hi, 0ull, j) : lc[static_cast<size_t>(k) * e.code_stride + j]);
+                hs += h;
+            }
         }
     }
     for (int d = 16; d > 0; d >>= 1) {
@@ -2518,7 +2549,12 @@ __global__ void k_checksum(Engine e, uint32_t nb, uint32_t ne, unsigned long lon
 
 void launch_checksum(const Engine& e, uint32_t n_begin, uint32_t n_end, unsigned long long tm_begin,
                      unsigned long long* out, cudaStream_t stream) {
-    k_checksum<<<e.grid_wide * 2, kThreads, 0, stream>>>(e, n_begin, n_end, tm_begin, out);
+    const uint32_t grid = e.grid_wide / 2 * checksum_blocks(e.inline_codes);
+    if (e.inline_codes) {
+        k_checksum<true><<<grid, kThreads, 0, stream>>>(e, n_begin, n_end, tm_begin, out);
+    } else {
+        k_checksum<false><<<grid, kThreads, 0, stream>>>(e, n_begin, n_end, tm_begin, out);
+    }
 }
 
 void launch_unpack_neurons(const Engine& e, uint32_t n0, uint32_t count, const NeuronArrays& out, cudaStream_t stream) {
