@@ -1374,201 +1374,195 @@ __device__ __forceinline__ SynA shfl_syn(const SynA& a, uint32_t src) {
     return r;
 }
 
-// One target's walk (the reference's sequential per-event loop,
-// NetworkPropagator.cpp:80-131, restricted to that target): its neuron state
-// and how far the walk has got.
-struct Walk {
-    NState s;
-    float threshold;
-    uint32_t n, beg, len;
-    uint32_t i;           // next event
-    uint32_t fires;       // target fires so far this tick
-    uint32_t first_fire;  // event of the first fire
-};
-
-// A fire at due position `due`: its bit in the fire bitmap, the neuron, and
-// one more fire in the bitmap tile (kThreads words) for k_fire_list.
-__device__ __forceinline__ void record_fire(const Engine& e, const Walk& w, uint32_t due) {
-    atomicOr(&e.fire_bits[due >> 5], 1u << (due & 31));
-    e.fire_at[due] = w.n;
-    atomicAdd(&e.fire_tile[(due >> 5) / kThreads], 1u);
+// The physics fields of a neuron's state.
+__device__ __forceinline__ void load_physics(NState& s, const NeuronRec* rec) {
+    const float4 c = reinterpret_cast<const float4*>(rec->cur)[0];
+    const uint4 u = reinterpret_cast<const uint4*>(rec->upd)[0];
+    const uint4 m = *reinterpret_cast<const uint4*>(&rec->membrane);
+    s.cur[0] = c.x;
+    s.cur[1] = c.y;
+    s.cur[2] = c.z;
+    s.cur[3] = c.w;
+    s.upd[0] = u.x;
+    s.upd[1] = u.y;
+    s.upd[2] = u.z;
+    s.upd[3] = u.w;
+    s.membrane = __uint_as_float(m.x);
+    s.spikes = m.y;
+    s.last_fired1 = m.z;
+    s.last_active = m.w;
+    s.flags = rec->flags;
 }
 
-// Phase 1 of a target's walk: load the neuron (its physics fields) and
-// process its events in due order up to and including its first fire.  Every
-// event before the first fire uses the weight its synapse's work computed.
-// Returns whether the target fired.
-template <typename Events>
-__device__ __forceinline__ bool walk_to_first_fire(const Engine& e, Walk& w, uint32_t t, const Events& ev) {
-    NState& s = w.s;
-    const NeuronRec* rec = e.nrec + w.n;
-    {
-        const float4 c = reinterpret_cast<const float4*>(rec->cur)[0];
-        const uint4 u = reinterpret_cast<const uint4*>(rec->upd)[0];
-        const uint4 m = *reinterpret_cast<const uint4*>(&rec->membrane);
-        s.cur[0] = c.x;
-        s.cur[1] = c.y;
-        s.cur[2] = c.z;
-        s.cur[3] = c.w;
-        s.upd[0] = u.x;
-        s.upd[1] = u.y;
-        s.upd[2] = u.z;
-        s.upd[3] = u.w;
-        s.membrane = __uint_as_float(m.x);
-        s.spikes = m.y;
-        s.last_fired1 = m.z;
-        s.last_active = m.w;
-        s.flags = rec->flags;
-    }
-    w.fires = 0;
-    w.first_fire = 0;
-    decay_to(s, t, e);
-    for (uint32_t i = 0; i < w.len; ++i) {
-        const uint32_t bits = ev.bits_of(w.beg + i);
-        if (process_input(s, w.threshold, bits & 3u, (bits >> 2) & 3u, ev.weight_of(w.beg + i), t)) {
-            record_fire(e, w, ev.at(w.beg + i).due);
-            w.fires = 1;
-            w.first_fire = i;
-            w.i = i + 1;
-            return true;
-        }
-    }
-    w.i = w.len;
-    return false;
-}
-
-// Phase 2, one warp: the rest of the walks of its lanes' fired targets, one
-// target at a time.  Every synaptic event after a fire redoes its STDP with
-// the target's fire count so far, starting from the synapse's state before
-// the event: its snapshot, or, when the same synapse already had an event
-// after the first fire, the record that event left.  The warp redoes up to 32
-// events at once (an event whose predecessor is in the same chunk waits a
-// round and takes its record by shuffle); the target's own lane then runs the
-// neuron physics over them in order.  If the target fires again inside the
-// chunk, the events after that fire are redone with the new count; only the
-// records of events before it are stored (the last event of each synapse
-// stores).  The result is the sequential order's.  `lo` is the bucket's first
-// event (Engine::ev_a0 counts from the tick's first one).
-template <typename Events>
-__device__ __forceinline__ void walk_fired_targets(const Engine& e, Walk& w, bool fired, uint32_t t, int stdp,
-                                                   const Events& ev, uint32_t lo, float* s_wt) {
-    const uint32_t lane = threadIdx.x & 31;
-    const float* ltp = e.tab.ltp;
-    unsigned pend = __ballot_sync(0xffffffffu, fired);
-    while (pend) {
-        const uint32_t L = __ffs(pend) - 1;
-        pend &= pend - 1;
-        const uint32_t beg = __shfl_sync(0xffffffffu, w.beg, L);
-        const uint32_t len = __shfl_sync(0xffffffffu, w.len, L);
-        const uint32_t after = __shfl_sync(0xffffffffu, w.first_fire, L) + 1;  // first event after the first fire
-        uint32_t pos = __shfl_sync(0xffffffffu, w.i, L);
-        uint32_t fires = __shfl_sync(0xffffffffu, w.fires, L);
-        while (pos < len) {
-            const uint32_t m = len - pos < 32 ? len - pos : 32;
-            const uint32_t j = pos + lane;
-            EvIn x{};
-            if (lane < m) x = ev.at(beg + j);
-            const bool syn = lane < m && !(x.bits & kEvExternal);
-            // the synapse's latest earlier event after the first fire
-            uint32_t pred = 0xFFFFFFFFu;
-            if (syn && (x.bits & kEvRepeat)) {
-                for (uint32_t q = j; q-- > after;) {
-                    const EvIn y = ev.at(beg + q);
-                    if (!(y.bits & kEvExternal) && y.tm == x.tm) {
-                        pred = q;
-                        break;
-                    }
-                }
-            }
-            const bool wait = pred != 0xFFFFFFFFu && pred >= pos;  // predecessor in this chunk
-            SynA a{};
-            float wt = x.weight;
-            bool done = !syn;
-            if (syn && !wait) {
-                a = pred != 0xFFFFFFFFu ? e.syn[x.tm].a : before_event(e.syn[x.tm].a, e.ev_a0[lo + beg + j]);
-                wt = redo_pre_stdp(e, a, t, fires, stdp, ltp);
-                done = true;
-            }
-            while (!__all_sync(0xffffffffu, done)) {
-                const uint32_t src = wait ? pred - pos : lane;
-                const SynA pa = shfl_syn(a, src);
-                const bool pdone = __shfl_sync(0xffffffffu, done, src);
-                if (!done && pdone) {
-                    a = pa;
-                    wt = redo_pre_stdp(e, a, t, fires, stdp, ltp);
-                    done = true;
-                }
-            }
-            if (lane < m) s_wt[lane] = wt;
-            __syncwarp();
-            uint32_t next = pos + m;
-            if (lane == L) {
-                for (uint32_t c = 0; c < m; ++c) {
-                    const EvIn y = ev.at(beg + pos + c);
-                    if (process_input(w.s, w.threshold, y.bits & 3u, (y.bits >> 2) & 3u, s_wt[c], t)) {
-                        record_fire(e, w, y.due);
-                        w.fires += 1;
-                        if (c + 1 < m) {
-                            next = pos + c + 1;
-                            break;
-                        }
-                    }
-                }
-                w.i = next;
-            }
-            next = __shfl_sync(0xffffffffu, next, L);
-            // store the records of the events before `next`, the last one of
-            // each synapse
-            const bool store = syn && j < next;
-            const unsigned long long key = store ? x.tm : (1ull << 32) | lane;
-            const unsigned same = __match_any_sync(0xffffffffu, key);
-            if (store && lane == 31u - __clz(same)) e.syn[x.tm].a = a;
-            pos = next;
-            fires = __shfl_sync(0xffffffffu, w.fires, L);
-            __syncwarp();
-        }
-    }
-}
-
-// Stores a finished walk's neuron state and lists the target if it fired.
-__device__ __forceinline__ void finish_walk(const Engine& e, const Walk& w) {
-    const NState& s = w.s;
-    NeuronRec* rec = e.nrec + w.n;
+__device__ __forceinline__ void store_physics(const NState& s, NeuronRec* rec) {
     reinterpret_cast<float4*>(rec->cur)[0] = make_float4(s.cur[0], s.cur[1], s.cur[2], s.cur[3]);
     reinterpret_cast<uint4*>(rec->upd)[0] = make_uint4(s.upd[0], s.upd[1], s.upd[2], s.upd[3]);
     *reinterpret_cast<uint4*>(&rec->membrane) =
         make_uint4(__float_as_uint(s.membrane), s.spikes, s.last_fired1, s.last_active);
     rec->flags = s.flags;
-    if (w.fires > 0) {
-        const uint32_t j = atomicAdd(&e.ts->n_fired_targets, 1u);
-        e.fired_tgt[j] = w.n;
-        e.fired_cnt[j] = w.fires;
-    }
 }
 
-__device__ __noinline__ void temporal_target(const Engine& e, uint32_t n, uint32_t k, uint32_t t, int temporal);
+// A fire of neuron n at due position `due`: its bit in the fire bitmap, the
+// neuron, and one more fire in the bitmap tile (kThreads words) for
+// k_fire_list.
+__device__ __forceinline__ void record_fire(const Engine& e, uint32_t n, uint32_t due) {
+    atomicOr(&e.fire_bits[due >> 5], 1u << (due & 31));
+    e.fire_at[due] = n;
+    atomicAdd(&e.fire_tile[(due >> 5) / kThreads], 1u);
+}
 
-// The walks of a bucket's targets, a thread each.
+// Lists a target that fired `fires` times this tick (k_post).
+__device__ __forceinline__ void record_fired_target(const Engine& e, uint32_t n, uint32_t fires) {
+    const uint32_t j = atomicAdd(&e.ts->n_fired_targets, 1u);
+    e.fired_tgt[j] = n;
+    e.fired_cnt[j] = fires;
+}
+
+// A target whose walk goes on after its first fire.
+struct Refire {
+    uint32_t j;     // target within the bucket
+    uint32_t next;  // its event after the fire
+};
+
+// The rest of a fired target's walk, one warp.  Every synaptic event after a
+// fire redoes its STDP with the target's fire count so far, starting from the
+// synapse's state before the event: its snapshot, or, when the same synapse
+// already had an event after the first fire, the record that event left.  The
+// warp redoes up to 32 events at once (an event whose predecessor is in the
+// same chunk waits a round and takes its record by shuffle); then the neuron
+// physics run over them in order (in lane 0: state `s`).  If the target fires
+// again inside the chunk, the events after that fire are redone with the new
+// count; only the records of events before it are stored (the last event of
+// each synapse stores).  The result is the sequential order's.  `beg`: the
+// target's first event in the bucket, `lo`: the bucket's first event in the
+// tick (Engine::ev_a0 counts from there).  Returns the target's fires.
+template <typename Events>
+__device__ __forceinline__ uint32_t walk_after_fire(const Engine& e, NState& s, float threshold, uint32_t n,
+                                                    uint32_t beg, uint32_t len, uint32_t after, uint32_t t, int stdp,
+                                                    const Events& ev, uint32_t lo, float* s_wt) {
+    const uint32_t lane = threadIdx.x & 31;
+    const float* ltp = e.tab.ltp;
+    uint32_t pos = after, fires = 1;
+    while (pos < len) {
+        const uint32_t m = len - pos < 32 ? len - pos : 32;
+        const uint32_t j = pos + lane;
+        EvIn x{};
+        if (lane < m) x = ev.at(beg + j);
+        const bool syn = lane < m && !(x.bits & kEvExternal);
+        // the synapse's latest earlier event after the first fire
+        uint32_t pred = 0xFFFFFFFFu;
+        if (syn && (x.bits & kEvRepeat)) {
+            for (uint32_t q = j; q-- > after;) {
+                const EvIn y = ev.at(beg + q);
+                if (!(y.bits & kEvExternal) && y.tm == x.tm) {
+                    pred = q;
+                    break;
+                }
+            }
+        }
+        const bool wait = pred != 0xFFFFFFFFu && pred >= pos;  // predecessor in this chunk
+        SynA a{};
+        float wt = x.weight;
+        bool done = !syn;
+        if (syn && !wait) {
+            a = pred != 0xFFFFFFFFu ? e.syn[x.tm].a : before_event(e.syn[x.tm].a, e.ev_a0[lo + beg + j]);
+            wt = redo_pre_stdp(e, a, t, fires, stdp, ltp);
+            done = true;
+        }
+        while (!__all_sync(0xffffffffu, done)) {
+            const uint32_t src = wait ? pred - pos : lane;
+            const SynA pa = shfl_syn(a, src);
+            const bool pdone = __shfl_sync(0xffffffffu, done, src);
+            if (!done && pdone) {
+                a = pa;
+                wt = redo_pre_stdp(e, a, t, fires, stdp, ltp);
+                done = true;
+            }
+        }
+        if (lane < m) s_wt[lane] = wt;
+        __syncwarp();
+        uint32_t next = pos + m;
+        if (lane == 0) {
+            for (uint32_t c = 0; c < m; ++c) {
+                const uint32_t bits = ev.bits_of(beg + pos + c);
+                if (process_input(s, threshold, bits & 3u, (bits >> 2) & 3u, s_wt[c], t)) {
+                    record_fire(e, n, ev.at(beg + pos + c).due);
+                    fires += 1;
+                    if (c + 1 < m) {
+                        next = pos + c + 1;
+                        break;
+                    }
+                }
+            }
+        }
+        next = __shfl_sync(0xffffffffu, next, 0);
+        // store the records of the events before `next`, the last one of
+        // each synapse
+        const bool store = syn && j < next;
+        const unsigned long long key = store ? x.tm : (1ull << 32) | lane;
+        const unsigned same = __match_any_sync(0xffffffffu, key);
+        if (store && lane == 31u - __clz(same)) e.syn[x.tm].a = a;
+        pos = next;
+        fires = __shfl_sync(0xffffffffu, fires, 0);
+        __syncwarp();
+    }
+    return fires;
+}
+
+__device__ __forceinline__ void temporal_target(const Engine& e, uint32_t n, uint32_t k, uint32_t t, int temporal);
+
+// The walks of a bucket's targets (the reference's sequential per-event loop,
+// NetworkPropagator.cpp:80-131, restricted to each target).  A thread per
+// target processes its events in due order up to and including its first fire
+// (every event before it uses the weight its synapse's work computed).  The
+// few targets with events after their first fire are then shared out to the
+// block's warps (one warp did its own 32 targets' one after the other: up to
+// 20 us with three or four of them, where the walk itself takes 4; sharing them
+// took the kernel from 36 to 32 us at 250,000 events, 197 to 187 at 2.5 M).
 template <typename Events>
 __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, uint32_t lo, uint32_t n0, uint32_t nw,
                                             const uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
-                                            float* s_wt) {
-    for (uint32_t j0 = 0; j0 < nw; j0 += blockDim.x) {
+                                            float* s_wt, Refire* s_refire, uint32_t* s_refires) {
+    for (uint32_t j0 = 0; j0 < nw; j0 += kEventThreads) {
+        if (threadIdx.x == 0) *s_refires = 0;
+        __syncthreads();
         const uint32_t j = j0 + threadIdx.x;
-        Walk w;
-        w.n = w.beg = w.len = w.i = w.fires = w.first_fire = 0;
-        w.threshold = 0.0f;
-        if (j < nw) {
-            w.n = n0 + j;
-            w.beg = s_seg[j];
-            w.len = s_seg[j + 1] - w.beg;
-            w.threshold = par[j].threshold;
+        const uint32_t beg = j < nw ? s_seg[j] : 0u, len = j < nw ? s_seg[j + 1] - beg : 0u;
+        if (len > 0) {
+            NeuronRec* rec = e.nrec + n0 + j;
+            const float threshold = par[j].threshold;
+            NState s;
+            load_physics(s, rec);
+            decay_to(s, t, e);
+            for (uint32_t i = 0; i < len; ++i) {
+                const uint32_t bits = ev.bits_of(beg + i);
+                if (process_input(s, threshold, bits & 3u, (bits >> 2) & 3u, ev.weight_of(beg + i), t)) {
+                    record_fire(e, n0 + j, ev.at(beg + i).due);
+                    if (i + 1 < len) {
+                        s_refire[atomicAdd(s_refires, 1u)] = Refire{j, i + 1};
+                    } else {
+                        record_fired_target(e, n0 + j, 1);
+                    }
+                    break;
+                }
+            }
+            store_physics(s, rec);
         }
-        const bool mine = w.len > 0;  // a target with due events
-        bool fired = false;
-        if (mine) fired = walk_to_first_fire(e, w, t, ev);
-        walk_fired_targets(e, w, fired, t, stdp, ev, lo, s_wt);
-        if (mine) finish_walk(e, w);
+        __syncthreads();
+        const uint32_t refires = *s_refires, warp = threadIdx.x >> 5;
+        for (uint32_t k = warp; k < refires; k += kEventThreads / 32) {
+            const Refire f = s_refire[k];
+            const uint32_t n = n0 + f.j, first = s_seg[f.j];
+            NState s;
+            load_physics(s, e.nrec + n);
+            const uint32_t fires = walk_after_fire(e, s, par[f.j].threshold, n, first, s_seg[f.j + 1] - first, f.next, t,
+                                                   stdp, ev, lo, s_wt + 32 * warp);
+            if ((threadIdx.x & 31) == 0) {
+                store_physics(s, e.nrec + n);
+                record_fired_target(e, n, fires);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1578,7 +1572,7 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
 template <bool kInline>
 __device__ __noinline__ void bucket_in_global(const Engine& e, uint32_t lo, uint32_t m, uint32_t n0, uint32_t nw,
                                               uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
-                                              int temporal, float* s_wt) {
+                                              int temporal, float* s_wt, Refire* s_refire, uint32_t* s_refires) {
     const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
     unsigned long long* grp = e.grp + lo;
     // s_seg[j + 1] holds target j's count, then its cursor, then its end
@@ -1628,7 +1622,7 @@ __device__ __noinline__ void bucket_in_global(const Engine& e, uint32_t lo, uint
         if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
     }
     __syncthreads();
-    walk_bucket(e, ev, lo, n0, nw, s_seg, par, t, stdp, s_wt);
+    walk_bucket(e, ev, lo, n0, nw, s_seg, par, t, stdp, s_wt, s_refire, s_refires);
 }
 
 // Everything a tick does at its targets, a block per bucket of consecutive
@@ -1660,7 +1654,7 @@ __device__ __noinline__ void bucket_in_global(const Engine& e, uint32_t lo, uint
 // events by a warp per target, walk, temporal pattern) the events' words and
 // inputs went through global memory between them, 20 of 32 lanes idled, and
 // each waited for the slowest block of the one before.  Sum of the four ->
-// this one, per tick: 309 -> 197 us (2.5 M events, 200,000 neurons), 82 -> 36
+// this one, per tick: 309 -> 187 us (2.5 M events, 200,000 neurons), 82 -> 32
 // us (250,000 events, 20,000 neurons).
 //
 // kInline: every synapse's learned code pattern is in its record
@@ -1673,6 +1667,8 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
     __shared__ float s_wt[kEventThreads / 32][32];  // per warp: weights of the events redone after a fire
     __shared__ uint32_t s_repeats;                  // synapses with several events
     __shared__ uint32_t s_next;                     // next task of the events phase
+    __shared__ Refire s_refire[kEventThreads];      // targets that go on after their first fire
+    __shared__ uint32_t s_refires;
     __shared__ uint32_t s_longest;                  // events of the busiest target
     const uint32_t width = 1u << e.bucket_shift;
     // the staged entries (16 bytes per event); once they are in registers, the
@@ -1857,11 +1853,12 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
                     __syncwarp();
                 }
                 __syncthreads();
-                walk_bucket(e, ev, lo, n0, nw, s_seg + 1, par, t, stdp, s_wt[threadIdx.x >> 5]);
+                walk_bucket(e, ev, lo, n0, nw, s_seg + 1, par, t, stdp, &s_wt[0][0], s_refire, &s_refires);
             }
         }
         if (!small) {
-            bucket_in_global<kInline>(e, lo, m, n0, nw, s_seg, par, t, stdp, temporal, s_wt[threadIdx.x >> 5]);
+            bucket_in_global<kInline>(e, lo, m, n0, nw, s_seg, par, t, stdp, temporal, &s_wt[0][0], s_refire,
+                                      &s_refires);
             __syncthreads();
             if (m > kBlockEvents) {
                 uint32_t busy = 0;
