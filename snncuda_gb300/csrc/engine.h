@@ -334,9 +334,11 @@ void launch_tick(const Engine& e, const TickStreams& s, cudaEvent_t* marks = nul
 const char* kernel_name(int index);
 void launch_inject(const Engine& e, const unsigned long long* ev, const uint32_t* slot_of_group,
                    const uint32_t* group_off, uint32_t groups, cudaStream_t stream);
-// Groups the W == 1 "wheel" of e (a caller's event buffer) by target: the
-// tick's four grouping kernels.
-void launch_group(const Engine& e, cudaStream_t stream);
+// Groups the W == 1 "wheel" of e (a caller's buffer of `count` events) by
+// target: the tick's counting and placing kernels, then k_group.
+void launch_group(const Engine& e, uint32_t count, cudaStream_t stream);
+// The kernel attributes launch_group needs (as configure_kernels).
+void configure_group();
 // Batched form: one handle simulates several networks side by side.
 // Sets kMetaRuleOffBit on target-major synapses [tm_begin, tm_end).
 void launch_rule_off(const Engine& e, unsigned long long tm_begin, unsigned long long tm_end, cudaStream_t stream);

@@ -663,11 +663,10 @@ __device__ __forceinline__ void code_update(SynB& b, const TargetParam& p, uint3
 //               totals itself), one reservation per (chunk, bucket), then
 //               every event goes to its bucket's range of grp_tmp (order
 //               inside a bucket arbitrary)
-//   k_bsort     a block per bucket: a counting sort of the bucket's events by
-//               target (in shared memory when the bucket fits), segment
-//               starts written; inside a target the order stays arbitrary,
-//               then k_segsort sorts it by due index (the grouping entry
-//               points only: the tick's k_events sorts its buckets itself)
+//   k_group     a block per bucket: the bucket's events by target in due order,
+//               and the segment starts (the grouping entry points only: the
+//               tick's k_events sorts its buckets itself); of buckets too
+//               large for its shared memory, k_group_rest sorts the segments
 // Per event that is two or more reads of the due list (k_bscatter places a
 // long list in passes over disjoint bucket ranges, so the lines it fills stay
 // in L2 until complete), one scattered write, and a coalesced read and write
@@ -1041,80 +1040,113 @@ __device__ void warp_merge_sort(unsigned long long* a, unsigned long long* b, ui
 
 
 
-// Events k_bsort places in shared memory before writing them out; each
-// thread holds its share of such a bucket in registers.
-constexpr uint32_t kSortSmemEvents = 4096;
-constexpr uint32_t kSortPerThread = kSortSmemEvents / kThreads;
-constexpr size_t kSortSmemBytes = kSortSmemEvents * sizeof(unsigned long long);
+// The lanes of a whole warp with the same 8-bit digit as this one (`in`: the
+// lane has one); eight ballots, where a match instruction over mostly
+// different digits kept the SM's match unit busy five times as long.
+__device__ __forceinline__ uint32_t same_digit(uint32_t digit, bool in) {
+    const uint32_t active = __ballot_sync(0xffffffffu, in);
+    uint32_t same = active;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = (digit >> b) & 1u;
+        const uint32_t ones = __ballot_sync(0xffffffffu, one);
+        same &= one ? ones : ~ones;
+    }
+    return same;
+}
 
-// One block per bucket: a counting sort of the bucket's events by target.
-// The events of each target end up contiguous in grp (in arbitrary order;
-// k_segsort sorts them by due index) and the targets' segment starts are
-// written.  A bucket of at most kSortSmemEvents events is loaded once into
-// registers (every load in flight at once), counted, placed in shared memory
-// and written out coalesced; a larger one is counted and placed in grp
-// directly from global memory.
-__global__ void __launch_bounds__(kThreads) k_bsort(Engine e) {
-    tick_enter();
-    extern __shared__ __align__(16) unsigned long long s_sort[];  // kSortSmemEvents, then counters
-    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_sort + kSortSmemEvents);  // [2^bucket_shift]
-    const uint32_t width = 1u << e.bucket_shift;
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t b = blockIdx.x; b < e.nbuckets; b += gridDim.x) {
-        const uint32_t lo = e.bstart[b], hi = e.bstart[b + 1], m = hi - lo;
-        const uint32_t n0 = b << e.bucket_shift;
-        const uint32_t nw = e.N - n0 < width ? e.N - n0 : width;
-        const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
-        const bool small = m <= kSortSmemEvents;
-        unsigned long long v[kSortPerThread];
-        uint32_t t16[kSortPerThread];
-        if (small) {
-#pragma unroll
-            for (uint32_t k = 0; k < kSortPerThread; ++k) {
-                const uint32_t i = threadIdx.x + k * kThreads;
-                const uint4 q = i < m ? in[i] : make_uint4(0u, 0u, 0u, 0u);
-                t16[k] = q.z;
-                v[k] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
-            }
-        }
-        for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) s_cnt[j] = 0;
+// Whole block: a[0 .. len) by key (below 2^bits), with b[0 .. len) as scratch;
+// the result is in a.  Stable radix sort by 8-bit digits: every warp counts
+// and then places a contiguous share of the entries, 32 at a time in order, in
+// its own row of counters (s_cnt: kBlock / 32 rows of 256, and 256 totals), so
+// an entry's place is the digit's start, the earlier warps' entries, this
+// warp's earlier ones, and its rank among the 32.  Work linear in len.
+template <int kBlock>
+__device__ void block_radix_sort(unsigned long long* a, unsigned long long* b, uint32_t len, uint32_t bits,
+                                 uint32_t* s_cnt) {
+    constexpr uint32_t kWarps = kBlock / 32, kInFlight = 4;  // loads per lane before the first is used
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t* mine = s_cnt + 256 * warp;
+    uint32_t* s_tot = s_cnt + 256 * kWarps;
+    const uint32_t share = (len + kWarps * 32 - 1) / (kWarps * 32) * 32;
+    const uint32_t i0 = min(len, warp * share), i1 = min(len, i0 + share);
+    unsigned long long *src = a, *dst = b;
+    for (uint32_t shift = 0; shift < bits; shift += 8) {
+        for (uint32_t i = threadIdx.x; i < 256 * kWarps; i += kBlock) s_cnt[i] = 0;
         __syncthreads();
-        if (small) {
+        for (uint32_t c = i0; c < i1; c += 32 * kInFlight) {
+            unsigned long long v[kInFlight];
 #pragma unroll
-            for (uint32_t k = 0; k < kSortPerThread; ++k)
-                if (threadIdx.x + k * kThreads < m && t16[k] < nw) atomicAdd(&s_cnt[t16[k]], 1u);
-        } else {
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                const uint32_t z = in[i].z;
-                if (z < nw) atomicAdd(&s_cnt[z], 1u);
+            for (uint32_t u = 0; u < kInFlight; ++u) {
+                const uint32_t i = c + 32 * u + lane;
+                v[u] = i < i1 ? src[i] : 0ull;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kInFlight; ++u) {
+                const bool in = c + 32 * u + lane < i1;
+                const uint32_t digit = (grp_key(v[u]) >> shift) & 255u;
+                const uint32_t same = same_digit(digit, in);
+                if (in && lane == __ffs(same) - 1) mine[digit] += __popc(same);
+                __syncwarp();
             }
         }
         __syncthreads();
-        uint32_t nz = 0;  // targets with events (statistics)
-        for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) nz += s_cnt[j] != 0;
-        nz = __reduce_add_sync(0xffffffffu, nz);
-        if (lane == 0 && nz) atomicAdd(&e.ts->n_touched, nz);
-        block_scan_shared<kThreads>(s_cnt, nw);  // segment starts relative to lo
-        for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) e.seg_start[n0 + j] = lo + s_cnt[j];
-        __syncthreads();
-        if (threadIdx.x == 0) {  // the bucket's total and cursor start at zero next tick
-            e.btot[b] = 0;
-            e.bcur[b] = 0;
+        for (uint32_t d = threadIdx.x; d < 256; d += kBlock) {
+            uint32_t run = 0;
+            for (uint32_t w = 0; w < kWarps; ++w) {
+                const uint32_t c = s_cnt[256 * w + d];
+                s_cnt[256 * w + d] = run;
+                run += c;
+            }
+            s_tot[d] = run;
         }
-        if (small) {
+        __syncthreads();
+        block_scan_shared<kBlock>(s_tot, 256);
+        for (uint32_t c = i0; c < i1; c += 32 * kInFlight) {
+            unsigned long long v[kInFlight];
 #pragma unroll
-            for (uint32_t k = 0; k < kSortPerThread; ++k)
-                if (threadIdx.x + k * kThreads < m && t16[k] < nw) s_sort[atomicAdd(&s_cnt[t16[k]], 1u)] = v[k];
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) e.grp[lo + i] = s_sort[i];
-        } else {
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                const uint4 q = in[i];
-                if (q.z < nw) e.grp[lo + atomicAdd(&s_cnt[q.z], 1u)] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
+            for (uint32_t u = 0; u < kInFlight; ++u) {
+                const uint32_t i = c + 32 * u + lane;
+                v[u] = i < i1 ? src[i] : 0ull;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kInFlight; ++u) {
+                const bool in = c + 32 * u + lane < i1;
+                const uint32_t digit = (grp_key(v[u]) >> shift) & 255u;
+                const uint32_t same = same_digit(digit, in);
+                const uint32_t at = in ? mine[digit] : 0u;
+                __syncwarp();
+                if (in) dst[s_tot[digit] + at + __popc(same & ((1u << lane) - 1u))] = v[u];
+                if (in && lane == __ffs(same) - 1) mine[digit] = at + __popc(same);
+                __syncwarp();
             }
         }
+        __syncthreads();
+        unsigned long long* t = src;
+        src = dst;
+        dst = t;
+    }
+    if (src != a) {
+        for (uint32_t i = threadIdx.x; i < len; i += kBlock) a[i] = src[i];
         __syncthreads();
     }
+}
+
+// Bits of the due indices 0 .. n-1.
+__device__ __forceinline__ uint32_t due_bits(uint32_t n) { return n > 1 ? 32 - __clz(n - 1) : 1; }
+
+// Adds one to counter[j] for each lane's j (of a whole warp; j == none: no
+// count) and returns the count before the lane's own.  The lanes that agree
+// with lane 0 share one atomic: a bucket that is large because of one busy
+// target then costs a warp's entries about one atomic, not 32 on one counter.
+__device__ __forceinline__ uint32_t warp_count(uint32_t* counter, uint32_t j, uint32_t none) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t j0 = __shfl_sync(0xffffffffu, j, 0);
+    const uint32_t same = __ballot_sync(0xffffffffu, j == j0);
+    uint32_t first = 0;
+    if (j != none && (lane == 0 || j != j0)) first = atomicAdd(&counter[j], lane == 0 ? __popc(same) : 1u);
+    const uint32_t shared = __shfl_sync(0xffffffffu, first, 0);
+    return j == j0 ? shared + __popc(same & ((1u << lane) - 1u)) : first;
 }
 
 // One warp puts a target's group of `len` events in due order (up to 32
@@ -1135,13 +1167,168 @@ __device__ __forceinline__ void sort_group(unsigned long long* g, unsigned long 
     }
 }
 
-// Grouping entry point only: due order inside every target's group of grp,
-// a warp per target.
-__global__ void __launch_bounds__(kThreads) k_segsort(Engine e) {
-    const uint32_t warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t n = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); n < e.N; n += warps) {
-        const uint32_t beg = e.seg_start[n];
-        sort_group(e.grp + beg, reinterpret_cast<unsigned long long*>(e.grp_tmp) + beg, e.seg_start[n + 1] - beg);
+// The most events of one target that a block ranks in shared memory (every
+// pair of them is compared).
+constexpr uint32_t kRankEvents = 512;
+
+// Whole block: f(entry) for the entries in[0 .. m), by whole warps (a thread
+// without an entry gets one with target `none`), four loads per thread in
+// flight.
+template <typename F>
+__device__ __forceinline__ void for_entries(const uint4* in, uint32_t m, uint32_t none, F&& f) {
+    constexpr uint32_t kInFlight = 4;
+    for (uint32_t c = 0; c < m; c += blockDim.x * kInFlight) {
+        uint4 q[kInFlight];
+#pragma unroll
+        for (uint32_t u = 0; u < kInFlight; ++u) {
+            const uint32_t i = c + u * blockDim.x + threadIdx.x;
+            q[u] = i < m ? in[i] : make_uint4(0u, 0u, none, 0u);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kInFlight; ++u) f(q[u]);
+    }
+}
+
+// Events k_group holds in shared memory (each thread its share in registers
+// first), and the longest segment a warp of k_group_rest sorts.
+constexpr uint32_t kSortSmemEvents = 4096;
+constexpr uint32_t kSortPerThread = kSortSmemEvents / kThreads;
+constexpr uint32_t kWarpSortEvents = 512;
+constexpr size_t kSortSmemBytes = kSortSmemEvents * (sizeof(unsigned long long) + sizeof(uint16_t));
+
+// Grouping entry points: one block per bucket.  A bucket that fits is counted
+// by target, placed in shared memory by target, and every event goes to its
+// rank in due order among its target's events (as k_events does); a larger
+// one, or one with a long segment, is counted and placed in grp from global
+// memory, and k_group_rest sorts its segments.  Streams the events once in (16
+// bytes each) and once out (8); the due order used to be a pass of its own
+// over grp, a warp per target: 55 + 358 -> 120 us for 13 M events over 1e6
+// targets.
+__global__ void __launch_bounds__(kThreads) k_group(const __grid_constant__ Engine e) {
+    tick_enter();
+    extern __shared__ __align__(16) unsigned long long s_sort[];  // kSortSmemEvents words, their targets, counters
+    uint16_t* s_tgt = reinterpret_cast<uint16_t*>(s_sort + kSortSmemEvents);
+    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_tgt + kSortSmemEvents);  // [2^bucket_shift + 1]
+    const uint32_t width = 1u << e.bucket_shift;
+    for (uint32_t b = blockIdx.x; b < e.nbuckets; b += gridDim.x) {
+        const uint32_t lo = e.bstart[b], hi = e.bstart[b + 1], m = hi - lo;
+        const uint32_t n0 = b << e.bucket_shift;
+        const uint32_t nw = e.N - n0 < width ? e.N - n0 : width;
+        const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
+        unsigned long long* out = e.grp + lo;
+        bool small = m <= kSortSmemEvents;
+        unsigned long long v[kSortPerThread];
+        uint32_t at[kSortPerThread];  // target, and its place among the target's events << 16
+        if (small) {
+#pragma unroll
+            for (uint32_t k = 0; k < kSortPerThread; ++k) {
+                const uint32_t i = threadIdx.x + k * kThreads;
+                const uint4 q = i < m ? in[i] : make_uint4(0u, 0u, 0xFFFFu, 0u);
+                v[k] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
+                at[k] = q.z < nw ? q.z : 0xFFFFu;
+            }
+        }
+        for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) s_cnt[j] = 0;
+        __syncthreads();
+        if (small) {
+#pragma unroll
+            for (uint32_t k = 0; k < kSortPerThread; ++k)
+                if (at[k] != 0xFFFFu) at[k] |= atomicAdd(&s_cnt[at[k]], 1u) << 16;
+        } else {
+            for_entries(in, m, nw, [&](const uint4& q) { warp_count(s_cnt, q.z < nw ? q.z : nw, nw); });
+        }
+        __syncthreads();
+        uint32_t longest = 0;
+        for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) longest = max(longest, s_cnt[j]);
+        small = !__syncthreads_or(longest > kRankEvents) && small;
+        const uint32_t total = block_scan_shared<kThreads>(s_cnt, nw);  // segment starts relative to lo
+        for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) e.seg_start[n0 + j] = lo + s_cnt[j];
+        if (threadIdx.x == 0) s_cnt[nw] = total;
+        __syncthreads();
+        if (small) {
+#pragma unroll
+            for (uint32_t k = 0; k < kSortPerThread; ++k) {
+                const uint32_t j = at[k] & 0xFFFFu;
+                if (j == 0xFFFFu) continue;
+                const uint32_t p = s_cnt[j] + (at[k] >> 16);
+                s_sort[p] = v[k];
+                s_tgt[p] = static_cast<uint16_t>(j);
+            }
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
+                const unsigned long long x = s_sort[i];
+                const uint32_t j = s_tgt[i], key = grp_key(x), q1 = s_cnt[j + 1];
+                uint32_t p = s_cnt[j];
+                for (uint32_t q = p; q < q1; ++q) p += grp_key(s_sort[q]) < key;
+                out[p] = x;
+            }
+        } else {
+            // placed with cursors that start at the segment starts (s_cnt[j]
+            // ends at the segment's end, target j + 1's start)
+            for_entries(in, m, nw, [&](const uint4& q) {
+                const uint32_t p = warp_count(s_cnt, q.z < nw ? q.z : nw, nw);
+                if (q.z < nw) out[p] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
+            });
+            // the segments are sorted by k_group_rest, over the whole GPU: the
+            // totals and counts are used up, their memory takes its lists
+            if (threadIdx.x == 0) e.btot[atomicAdd(&e.ts->n_touched, 1u)] = b;
+            __syncthreads();
+            for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) {
+                const uint32_t beg = j > 0 ? s_cnt[j - 1] : 0u;
+                if (s_cnt[j] - beg > kWarpSortEvents) e.bcnt[atomicAdd(&e.ts->n_fired_targets, 1u)] = n0 + j;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+constexpr int kLongThreads = 1024;
+constexpr size_t kLongSmemBytes = 256 * (kLongThreads / 32 + 1) * sizeof(uint32_t);
+
+// Grouping entry points: due order of the segments k_group left: a warp for
+// each target of the buckets it listed, and a block for each target it listed
+// (more than kWarpSortEvents events).  One warp merged such a long segment: 200
+// ms for the 450,000 events of one target among 9 M, now 1.6 (and 0.7 in
+// k_group before it, from 1.5 with every entry's own atomic on the one counter).
+// The entries of a listed bucket are all placed: their memory is the scratch.
+__global__ void __launch_bounds__(kLongThreads) k_group_rest(const __grid_constant__ Engine e) {
+    tick_enter();
+    extern __shared__ uint32_t s_radix[];
+    const uint32_t buckets = e.ts->n_touched, targets = e.ts->n_fired_targets;
+    auto segment = [&](uint32_t n, unsigned long long*& g, unsigned long long*& tmp) {
+        const uint32_t beg = e.seg_start[n], lo = e.bstart[n >> e.bucket_shift];
+        g = e.grp + beg;
+        tmp = reinterpret_cast<unsigned long long*>(e.grp_tmp + lo) + (beg - lo);
+        return e.seg_start[n + 1] - beg;
+    };
+    unsigned long long *g, *tmp;
+    const unsigned long long items = static_cast<unsigned long long>(buckets) << e.bucket_shift;
+    const uint32_t warps = gridDim.x * (kLongThreads / 32);
+    // (item i's target: neighbouring warps take different blocks' SMs)
+    for (unsigned long long i = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; i < items; i += warps) {
+        const uint32_t n = (e.btot[i >> e.bucket_shift] << e.bucket_shift) +
+                           static_cast<uint32_t>(i & ((1u << e.bucket_shift) - 1u));
+        if (n >= e.N) continue;
+        const uint32_t len = segment(n, g, tmp);
+        if (len <= kWarpSortEvents) sort_group(g, tmp, len);
+    }
+    const uint32_t bits = due_bits(e.ts->n_due);
+    for (uint32_t k = blockIdx.x; k < targets; k += gridDim.x) {
+        const uint32_t len = segment(e.bcnt[k], g, tmp);
+        __syncthreads();
+        block_radix_sort<kLongThreads>(g, tmp, len, bits, s_radix);
+    }
+}
+
+// Grouping entry points: the scratch as the counting kernels expect it.
+__global__ void k_group_init(const __grid_constant__ Engine e, uint32_t count) {
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < e.nbuckets; b += gridDim.x * blockDim.x) {
+        e.btot[b] = 0;
+        e.bcur[b] = 0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *e.ts = TickState{};
+        *e.slot_count = count;
     }
 }
 
@@ -1255,14 +1442,12 @@ struct BucketParams {
     }
 };
 
-// Threads of a k_events block, the events it holds in shared memory, and the
-// most events of one target it ranks there (the rank compares every pair of a
-// target's events).
+// Threads of a k_events block, and the events it holds in shared memory.
 constexpr int kEventThreads = SNNGB_EVENT_THREADS;
 constexpr uint32_t kBlockPerThread = 10;
 constexpr uint32_t kBlockEvents = kBlockPerThread * kEventThreads;
-constexpr uint32_t kRankEvents = 512;
 constexpr uint32_t kSharedSynapse = 0x8000u;  // beside an event's target: its synapse has other events in the tick
+static_assert(kBlockEvents * sizeof(BucketEntry) >= 256 * (kEventThreads / 32 + 1) * sizeof(uint32_t), "s_radix");
 static_assert((1u << kMaxBucketShift) <= kSharedSynapse, "targets of a bucket");
 
 // A bucket's events grouped by target in due order, as the event and walk
@@ -1568,32 +1753,37 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
 
 // A bucket with more events than the block's shared memory, or with a long
 // group: grouped in Engine::grp (a counting sort by target, then a warp per
-// target puts its events in due order), its event inputs in Engine::evin.
+// target, or the block for a long group, puts its events in due order), its
+// event inputs in Engine::evin.  s_radix: the block's shared memory, otherwise
+// unused on this path.
 template <bool kInline>
 __device__ __noinline__ void bucket_in_global(const Engine& e, uint32_t lo, uint32_t m, uint32_t n0, uint32_t nw,
                                               uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
-                                              int temporal, float* s_wt, Refire* s_refire, uint32_t* s_refires) {
+                                              int temporal, float* s_wt, Refire* s_refire, uint32_t* s_refires,
+                                              uint32_t* s_radix) {
     const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
     unsigned long long* grp = e.grp + lo;
     // s_seg[j + 1] holds target j's count, then its cursor, then its end
     for (uint32_t j = threadIdx.x; j <= nw; j += blockDim.x) s_seg[j] = 0;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-        const uint32_t z = in[i].z;
-        if (z < nw) atomicAdd(&s_seg[z + 1], 1u);
-    }
+    for_entries(in, m, nw, [&](const uint4& q) { warp_count(s_seg + 1, q.z < nw ? q.z : nw, nw); });
     __syncthreads();
     block_scan_shared<kEventThreads>(s_seg + 1, nw);
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-        const uint4 q = in[i];
-        if (q.z < nw) grp[atomicAdd(&s_seg[q.z + 1], 1u)] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
-    }
+    for_entries(in, m, nw, [&](const uint4& q) {
+        const uint32_t p = warp_count(s_seg + 1, q.z < nw ? q.z : nw, nw);
+        if (q.z < nw) grp[p] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
+    });
     __syncthreads();
     // the bucket's own entries are placed: their memory is the merges' scratch
     unsigned long long* tmp = reinterpret_cast<unsigned long long*>(e.grp_tmp + lo);
     for (uint32_t j = threadIdx.x >> 5; j < nw; j += blockDim.x / 32) {
         const uint32_t beg = s_seg[j], len = s_seg[j + 1] - beg;
-        sort_group(grp + beg, tmp + beg, len);
+        if (len <= kWarpSortEvents) sort_group(grp + beg, tmp + beg, len);
+    }
+    for (uint32_t j = 0; j < nw; ++j) {
+        const uint32_t beg = s_seg[j], len = s_seg[j + 1] - beg;
+        if (len > kWarpSortEvents)
+            block_radix_sort<kEventThreads>(grp + beg, tmp + beg, len, due_bits(e.ts->n_due), s_radix);
     }
     __syncthreads();
     const GlobalEvents ev{grp, e.evin + lo};
@@ -1858,7 +2048,7 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
         }
         if (!small) {
             bucket_in_global<kInline>(e, lo, m, n0, nw, s_seg, par, t, stdp, temporal, &s_wt[0][0], s_refire,
-                                      &s_refires);
+                                      &s_refires, reinterpret_cast<uint32_t*>(s_raw));
             __syncthreads();
             if (m > kBlockEvents) {
                 uint32_t busy = 0;
@@ -2594,10 +2784,9 @@ static void launch_main(void (*kernel)(Engine), uint32_t grid, uint32_t block, s
 static size_t bucket_smem(const Engine& e) {
     return stream_buf_offset(e.nbuckets) + kStreamBufs * kStreamTile * sizeof(unsigned long long);
 }
-static size_t bsort_smem(const Engine& e) {
-    return kSortSmemBytes + (static_cast<size_t>(1) << e.bucket_shift) * sizeof(uint32_t);
+static size_t group_smem(uint32_t bucket_shift) {
+    return kSortSmemBytes + ((static_cast<size_t>(1) << bucket_shift) + 1) * sizeof(uint32_t);
 }
-static uint32_t bsort_grid(const Engine& e) { return e.nbuckets; }
 static size_t events_smem(uint32_t bucket_shift) {
     const size_t width = static_cast<size_t>(1) << bucket_shift;
     return kBlockEvents * (sizeof(BucketEntry) + 2 + 2) + (width <= kSharedParams ? width * sizeof(TargetParam) : 0) +
@@ -2680,23 +2869,34 @@ const char* kernel_name(int index) {
     return index >= 0 && index < kKernelCount ? names[index] : "";
 }
 
-void launch_group(const Engine& e, cudaStream_t stream) {
-    k_bcount<<<e.grid_bucket, kBucketThreads, bucket_smem(e), stream>>>(e);
-    k_bscatter<<<e.grid_bucket, kBucketThreads, bucket_smem(e), stream>>>(e);
-    k_bsort<<<bsort_grid(e), kThreads, bsort_smem(e), stream>>>(e);
-    k_segsort<<<e.grid_wide * 4, kThreads, 0, stream>>>(e);
+void launch_group(const Engine& e, uint32_t count, cudaStream_t stream) {
+    // (programmatic dependents: each kernel waits in tick_enter)
+    const uint32_t init = e.nbuckets / kThreads + 1;
+    k_group_init<<<init < 64 ? init : 64, kThreads, 0, stream>>>(e, count);
+    launch_main(k_bcount, e.grid_bucket, kBucketThreads, bucket_smem(e), stream, false, e);
+    launch_main(k_bscatter, e.grid_bucket, kBucketThreads, bucket_smem(e), stream, true, e);
+    launch_main(k_group, e.nbuckets, kThreads, group_smem(e.bucket_shift), stream, true, e);
+    // (a bucket or a segment it cannot rank needs more events than that)
+    if (count > kRankEvents) launch_main(k_group_rest, e.grid_wide / 2, kLongThreads, kLongSmemBytes, stream, true, e);
 }
 
 void configure_kernels() {
-    const int events_bytes = static_cast<int>(std::max(events_smem(kMaxBucketShift), events_smem(8)));
-    cudaFuncSetAttribute(k_events<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
-    cudaFuncSetAttribute(k_events<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
     const int bucket_bytes =
         static_cast<int>(stream_buf_offset(kMaxTickBuckets) + kStreamBufs * kStreamTile * sizeof(unsigned long long));
     cudaFuncSetAttribute(k_bcount, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_bytes);
     cudaFuncSetAttribute(k_bscatter, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_bytes);
-    cudaFuncSetAttribute(k_bsort, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kSortSmemBytes + (1u << kMaxBucketShift) * sizeof(uint32_t)));
+    const int events_bytes = static_cast<int>(std::max(events_smem(kMaxBucketShift), events_smem(8)));
+    cudaFuncSetAttribute(k_events<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
+    cudaFuncSetAttribute(k_events<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
+}
+
+void configure_group() {
+    const int bucket_bytes =
+        static_cast<int>(stream_buf_offset(kMaxTickBuckets) + kStreamBufs * kStreamTile * sizeof(unsigned long long));
+    cudaFuncSetAttribute(k_bcount, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_bytes);
+    cudaFuncSetAttribute(k_bscatter, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_bytes);
+    cudaFuncSetAttribute(k_group, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(group_smem(kMaxBucketShift)));
 }
 
 void launch_init_syn(const Engine& e, const SynA* a, cudaStream_t stream) {
