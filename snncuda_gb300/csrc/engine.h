@@ -181,6 +181,7 @@ struct TickState {
     int32_t temporal_enabled; // SynapseDendriteConfig::temporal_learning_enabled
     uint32_t done_scan;       // "last block" counters
     uint32_t done_fire_list;
+    uint32_t small_stop;      // not 0: k_small ended before its last tick (launch_small)
 };
 
 struct Tables {
@@ -332,6 +333,22 @@ struct TickStreams {
 };
 void launch_tick(const Engine& e, const TickStreams& s, cudaEvent_t* marks = nullptr);
 const char* kernel_name(int index);
+// Ticks ts->tick .. end-1 of a small network (small_network) in one kernel; it
+// stops before a tick it does not take (ts->small_stop, until which the
+// launches behind it return at once): one with more than `limit` events due
+// (small_limit).
+constexpr uint32_t kSmallBlocks = 8;
+constexpr uint32_t kSmallTargets = 4096;  // per block
+constexpr uint32_t kSmallEvents = 8192;
+constexpr uint32_t kSmallSlots = 1024;
+inline uint32_t small_limit(const Engine& e) {
+    const unsigned long long share = e.slot_cap / kSmallBlocks;  // a block's part of the per-event scratch
+    return static_cast<uint32_t>(share < kSmallEvents ? share : kSmallEvents);
+}
+inline bool small_network(const Engine& e) {
+    return e.N > 0 && e.N <= kSmallBlocks * kSmallTargets && e.W <= kSmallSlots && small_limit(e) >= 512;
+}
+void launch_small(const Engine& e, uint32_t end, uint32_t limit, cudaStream_t stream);
 void launch_inject(const Engine& e, const unsigned long long* ev, const uint32_t* slot_of_group,
                    const uint32_t* group_off, uint32_t groups, cudaStream_t stream);
 // Groups the W == 1 "wheel" of e (a caller's buffer of `count` events) by

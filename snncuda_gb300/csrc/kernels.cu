@@ -1596,12 +1596,17 @@ __device__ __forceinline__ void record_fire(const Engine& e, uint32_t n, uint32_
     atomicAdd(&e.fire_tile[(due >> 5) / kThreads], 1u);
 }
 
-// Lists a target that fired `fires` times this tick (k_post).
-__device__ __forceinline__ void record_fired_target(const Engine& e, uint32_t n, uint32_t fires) {
-    const uint32_t j = atomicAdd(&e.ts->n_fired_targets, 1u);
-    e.fired_tgt[j] = n;
-    e.fired_cnt[j] = fires;
-}
+// Where a walk's fires go: the engine's bitmap and list of fired targets.
+struct EngineFires {
+    const Engine& e;
+    __device__ __forceinline__ void fire(uint32_t n, uint32_t due) const { record_fire(e, n, due); }
+    // A target that fired `fires` times this tick (k_post).
+    __device__ __forceinline__ void target(uint32_t n, uint32_t fires) const {
+        const uint32_t j = atomicAdd(&e.ts->n_fired_targets, 1u);
+        e.fired_tgt[j] = n;
+        e.fired_cnt[j] = fires;
+    }
+};
 
 // A target whose walk goes on after its first fire.
 struct Refire {
@@ -1621,10 +1626,10 @@ struct Refire {
 // each synapse stores).  The result is the sequential order's.  `beg`: the
 // target's first event in the bucket, `lo`: the bucket's first event in the
 // tick (Engine::ev_a0 counts from there).  Returns the target's fires.
-template <typename Events>
+template <typename Events, typename Fires>
 __device__ __forceinline__ uint32_t walk_after_fire(const Engine& e, NState& s, float threshold, uint32_t n,
                                                     uint32_t beg, uint32_t len, uint32_t after, uint32_t t, int stdp,
-                                                    const Events& ev, uint32_t lo, float* s_wt) {
+                                                    const Events& ev, uint32_t lo, float* s_wt, const Fires& out) {
     const uint32_t lane = threadIdx.x & 31;
     const float* ltp = e.tab.ltp;
     uint32_t pos = after, fires = 1;
@@ -1671,7 +1676,7 @@ __device__ __forceinline__ uint32_t walk_after_fire(const Engine& e, NState& s, 
             for (uint32_t c = 0; c < m; ++c) {
                 const uint32_t bits = ev.bits_of(beg + pos + c);
                 if (process_input(s, threshold, bits & 3u, (bits >> 2) & 3u, s_wt[c], t)) {
-                    record_fire(e, n, ev.at(beg + pos + c).due);
+                    out.fire(n, ev.at(beg + pos + c).due);
                     fires += 1;
                     if (c + 1 < m) {
                         next = pos + c + 1;
@@ -1704,11 +1709,11 @@ __device__ __forceinline__ void temporal_target(const Engine& e, uint32_t n, uin
 // block's warps (one warp did its own 32 targets' one after the other: up to
 // 20 us with three or four of them, where the walk itself takes 4; sharing them
 // took the kernel from 36 to 32 us at 250,000 events, 197 to 187 at 2.5 M).
-template <typename Events>
+template <int kT, typename Events, typename Fires>
 __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, uint32_t lo, uint32_t n0, uint32_t nw,
                                             const uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
-                                            float* s_wt, Refire* s_refire, uint32_t* s_refires) {
-    for (uint32_t j0 = 0; j0 < nw; j0 += kEventThreads) {
+                                            float* s_wt, Refire* s_refire, uint32_t* s_refires, const Fires& out) {
+    for (uint32_t j0 = 0; j0 < nw; j0 += kT) {
         if (threadIdx.x == 0) *s_refires = 0;
         __syncthreads();
         const uint32_t j = j0 + threadIdx.x;
@@ -1722,11 +1727,11 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
             for (uint32_t i = 0; i < len; ++i) {
                 const uint32_t bits = ev.bits_of(beg + i);
                 if (process_input(s, threshold, bits & 3u, (bits >> 2) & 3u, ev.weight_of(beg + i), t)) {
-                    record_fire(e, n0 + j, ev.at(beg + i).due);
+                    out.fire(n0 + j, ev.at(beg + i).due);
                     if (i + 1 < len) {
                         s_refire[atomicAdd(s_refires, 1u)] = Refire{j, i + 1};
                     } else {
-                        record_fired_target(e, n0 + j, 1);
+                        out.target(n0 + j, 1);
                     }
                     break;
                 }
@@ -1735,16 +1740,16 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
         }
         __syncthreads();
         const uint32_t refires = *s_refires, warp = threadIdx.x >> 5;
-        for (uint32_t k = warp; k < refires; k += kEventThreads / 32) {
+        for (uint32_t k = warp; k < refires; k += kT / 32) {
             const Refire f = s_refire[k];
             const uint32_t n = n0 + f.j, first = s_seg[f.j];
             NState s;
             load_physics(s, e.nrec + n);
             const uint32_t fires = walk_after_fire(e, s, par[f.j].threshold, n, first, s_seg[f.j + 1] - first, f.next, t,
-                                                   stdp, ev, lo, s_wt + 32 * warp);
+                                                   stdp, ev, lo, s_wt + 32 * warp, out);
             if ((threadIdx.x & 31) == 0) {
                 store_physics(s, e.nrec + n);
-                record_fired_target(e, n, fires);
+                out.target(n, fires);
             }
         }
         __syncthreads();
@@ -1812,7 +1817,117 @@ __device__ __noinline__ void bucket_in_global(const Engine& e, uint32_t lo, uint
         if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
     }
     __syncthreads();
-    walk_bucket(e, ev, lo, n0, nw, s_seg, par, t, stdp, s_wt, s_refire, s_refires);
+    walk_bucket<kEventThreads>(e, ev, lo, n0, nw, s_seg, par, t, stdp, s_wt, s_refire, s_refires, EngineFires{e});
+}
+
+// Shared memory of a bucket's events besides SharedEvents.
+struct BucketSpace {
+    unsigned long long* word;  // the events' words grouped by target
+    uint16_t* tgt;             // their targets
+    uint16_t* list;            // first events of the synapses with several
+    uint32_t* seg;             // seg[j + 1], seg[j + 2]: first and end of target j's events
+    float* wt;                 // 32 per warp: weights of the events redone after a fire
+    Refire* refire;            // a block's threads: targets that go on after their first fire
+    uint32_t *repeats, *next, *refires;  // counters (the first two zero)
+    uint16_t* multi;                     // kAlone: targets with several reference patterns,
+    uint32_t* multis;                    // and their number (zero)
+};
+
+template <int kGroup>
+__device__ __forceinline__ void temporal_group(const Engine& e, uint32_t n, uint32_t k, uint32_t t, int enabled);
+
+// Steps 2 (from the grouped words on) to 4 of k_events for one bucket.  kAlone:
+// the block is not k_events': the temporal patterns of targets with several
+// reference patterns are done here too.
+template <bool kInline, int kT, bool kAlone, typename Fires>
+__device__ __forceinline__ void bucket_events(const Engine& e, const BucketSpace& b, const SharedEvents& ev,
+                                              uint32_t total, uint32_t lo, uint32_t n0, uint32_t nw,
+                                              const BucketParams& par, uint32_t t, int stdp, int temporal,
+                                              const Fires& out) {
+    if (kAlone && e.multi_refs)
+        for (uint32_t j = threadIdx.x; j < nw; j += kT)
+            if (b.seg[j + 2] > b.seg[j + 1] && par[j].max_refs != 1) b.multi[atomicAdd(b.multis, 1u)] = static_cast<uint16_t>(j);
+    // each event's rank in due order among its target's events
+    // (by position: the lanes of a warp read the same or the next
+    // group's words); of the synapses with several events, the
+    // first event goes on a list
+    for (uint32_t i = threadIdx.x; i < total; i += kT) {
+        const unsigned long long v = b.word[i];
+        const uint32_t j = b.tgt[i] & ~kSharedSynapse, s0 = b.seg[j + 1], s1 = b.seg[j + 2];
+        const uint32_t due = static_cast<uint32_t>(v), pay = static_cast<uint32_t>(v >> 32);
+        uint32_t p = s0, same = 0, before = 0;  // synaptic events with this payload, those due earlier
+        for (uint32_t q = s0; q < s1; ++q) {
+            const unsigned long long x = b.word[q];
+            const uint32_t d = static_cast<uint32_t>(x);
+            const bool hit = static_cast<uint32_t>(x >> 32) == pay && !(d & 1u);
+            p += d < due;
+            same += hit;
+            before += hit && d < due;
+        }
+        ev.word[p] = v;
+        if (same > 1 && !(due & 1u)) {
+            b.tgt[p] = static_cast<uint16_t>(j | kSharedSynapse);
+            if (before == 0) b.list[atomicAdd(b.repeats, 1u)] = static_cast<uint16_t>(p);
+        }
+    }
+    __syncthreads();
+    if (!kAlone && e.multi_refs)
+        for (uint32_t j = threadIdx.x; j < nw; j += kT) e.seg_start[n0 + j] = lo + b.seg[j + 1];
+    // The warps share out the rest but the walk: the temporal
+    // patterns (they need only the targets' event counts) 32
+    // targets at a time from the first warps, the synapses with
+    // several events, then all other events.
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t j = threadIdx.x; j < nw; j += kT) {
+        const uint32_t k = b.seg[j + 2] - b.seg[j + 1];
+        if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
+    }
+    __syncwarp();
+    constexpr uint32_t kGroup = 8;  // lanes per target with several reference patterns
+    const uint32_t multis = kAlone ? *b.multis : 0u, patterns = (multis + 32 / kGroup - 1) / (32 / kGroup);
+    const uint32_t repeats = *b.repeats, lists = (repeats + 31) / 32, tasks = patterns + lists + (total + 31) / 32;
+    for (;;) {
+        uint32_t task = lane == 0 ? atomicAdd(b.next, 1u) : 0u;
+        task = __shfl_sync(0xffffffffu, task, 0);
+        if (task >= tasks) break;
+        if constexpr (kAlone) {
+            if (task < patterns) {
+                const uint32_t k = (task * 32 + lane) / kGroup;
+                if (k < multis) {
+                    const uint32_t j = b.multi[k];
+                    temporal_group<kGroup>(e, n0 + j, b.seg[j + 2] - b.seg[j + 1], t, temporal);
+                }
+                __syncwarp();
+                continue;
+            }
+            task -= patterns;
+        }
+        uint32_t i = (task - lists) * 32 + lane, last = 0;
+        bool run;
+        if (task < lists) {
+            const uint32_t k = task * 32 + lane;
+            run = k < repeats;
+            if (run) {
+                i = b.list[k];
+                last = b.seg[(b.tgt[i] & ~kSharedSynapse) + 2];
+            }
+        } else {
+            run = i < total;
+            if (run && ev.external(i)) {
+                ev.put(i, __uint_as_float(ev.payload(i)), kEvExternal);
+                run = false;
+            }
+            run = run && !(b.tgt[i] & kSharedSynapse);
+            last = i + 1;
+        }
+        if (run) {
+            const uint32_t j = b.tgt[i] & ~kSharedSynapse;
+            synapse_events<kInline>(e, ev, lo, i, last, par[j], n0 + j, t, stdp, temporal);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    walk_bucket<kT>(e, ev, lo, n0, nw, b.seg + 1, par, t, stdp, b.wt, b.refire, b.refires, out);
 }
 
 // Everything a tick does at its targets, a block per bucket of consecutive
@@ -1872,6 +1987,8 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
     TargetParam* s_par = reinterpret_cast<TargetParam*>(s_list + kBlockEvents);
     const bool keep_params = width <= kSharedParams;
     uint32_t* s_seg = reinterpret_cast<uint32_t*>(s_par + (keep_params ? width : 0u));  // [width + 2]
+    const BucketSpace space{s_word, s_tgt, s_list, s_seg, &s_wt[0][0], s_refire, &s_repeats, &s_next, &s_refires,
+                            nullptr, nullptr};
     const uint32_t t = e.ts->tick;
     const int stdp = e.ts->stdp_enabled;
     const int temporal = e.ts->temporal_enabled;
@@ -1977,73 +2094,8 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
                     s_tgt[p] = static_cast<uint16_t>(j);
                 }
                 __syncthreads();
-                // each event's rank in due order among its target's events
-                // (by position: the lanes of a warp read the same or the next
-                // group's words); of the synapses with several events, the
-                // first event goes on a list
-                for (uint32_t i = threadIdx.x; i < total; i += kEventThreads) {
-                    const unsigned long long v = s_word[i];
-                    const uint32_t j = s_tgt[i] & ~kSharedSynapse, s0 = s_seg[j + 1], s1 = s_seg[j + 2];
-                    const uint32_t due = static_cast<uint32_t>(v), pay = static_cast<uint32_t>(v >> 32);
-                    uint32_t p = s0, same = 0, before = 0;  // synaptic events with this payload, those due earlier
-                    for (uint32_t q = s0; q < s1; ++q) {
-                        const unsigned long long x = s_word[q];
-                        const uint32_t d = static_cast<uint32_t>(x);
-                        const bool hit = static_cast<uint32_t>(x >> 32) == pay && !(d & 1u);
-                        p += d < due;
-                        same += hit;
-                        before += hit && d < due;
-                    }
-                    ev.word[p] = v;
-                    if (same > 1 && !(due & 1u)) {
-                        s_tgt[p] = static_cast<uint16_t>(j | kSharedSynapse);
-                        if (before == 0) s_list[atomicAdd(&s_repeats, 1u)] = static_cast<uint16_t>(p);
-                    }
-                }
-                __syncthreads();
-                if (e.multi_refs)
-                    for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) e.seg_start[n0 + j] = lo + s_seg[j + 1];
-                // The warps share out the rest but the walk: the temporal
-                // patterns (they need only the targets' event counts) 32
-                // targets at a time from the first warps, the synapses with
-                // several events, then all other events.
-                const uint32_t lane = threadIdx.x & 31;
-                for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) {
-                    const uint32_t k = s_seg[j + 2] - s_seg[j + 1];
-                    if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
-                }
-                __syncwarp();
-                const uint32_t repeats = s_repeats, lists = (repeats + 31) / 32, tasks = lists + (total + 31) / 32;
-                for (;;) {
-                    uint32_t task = lane == 0 ? atomicAdd(&s_next, 1u) : 0u;
-                    task = __shfl_sync(0xffffffffu, task, 0);
-                    if (task >= tasks) break;
-                    uint32_t i = (task - lists) * 32 + lane, last = 0;
-                    bool run;
-                    if (task < lists) {
-                        const uint32_t k = task * 32 + lane;
-                        run = k < repeats;
-                        if (run) {
-                            i = s_list[k];
-                            last = s_seg[(s_tgt[i] & ~kSharedSynapse) + 2];
-                        }
-                    } else {
-                        run = i < total;
-                        if (run && ev.external(i)) {
-                            ev.put(i, __uint_as_float(ev.payload(i)), kEvExternal);
-                            run = false;
-                        }
-                        run = run && !(s_tgt[i] & kSharedSynapse);
-                        last = i + 1;
-                    }
-                    if (run) {
-                        const uint32_t j = s_tgt[i] & ~kSharedSynapse;
-                        synapse_events<kInline>(e, ev, lo, i, last, par[j], n0 + j, t, stdp, temporal);
-                    }
-                    __syncwarp();
-                }
-                __syncthreads();
-                walk_bucket(e, ev, lo, n0, nw, s_seg + 1, par, t, stdp, &s_wt[0][0], s_refire, &s_refires);
+                bucket_events<kInline, kEventThreads, false>(e, space, ev, total, lo, n0, nw, par, t, stdp, temporal,
+                                                             EngineFires{e});
             }
         }
         if (!small) {
@@ -2117,153 +2169,157 @@ __device__ __noinline__ void temporal_target(const Engine& e, uint32_t n, uint32
 // 1,000-neuron network, and 30 us more with 43.  Runs after k_events, beside
 // the fire ordering, so it takes the tick from post_tick.
 template <int kGroup>
+__device__ __forceinline__ void temporal_group(const Engine& e, uint32_t n, uint32_t k, uint32_t t, int enabled) {
+    const uint32_t sub = threadIdx.x & (kGroup - 1);
+    const uint32_t mask = kGroup == 32 ? 0xffffffffu : ((1u << (kGroup & 31)) - 1u) << (threadIdx.x & 31 & ~(kGroup - 1));
+    const NeuronParam p = e.nparam[n];
+    NeuronRec* rec = e.nrec + n;
+    NeuronTp q = e.ntp[n];
+    if (!enabled) {
+        __syncwarp(mask);
+        if (sub == 0) e.ntp[n].last_match = 0;
+        return;
+    }
+    uint32_t match_count = rec->match_count, ws = rec->ws, len = rec->len;
+    unsigned long long* cand = e.cand + p.cand_base;
+    RefMeta* meta = e.refmeta + p.meta_base;
+    unsigned long long* ring = e.ring + p.ring_base;
+    unsigned long long last_run = q.nruns > 0 ? cand[q.nruns - 1] : 0ull;
+    __syncwarp(mask);  // the group has read its state
+    auto ref = [&](uint32_t r) -> RefMeta& { return meta[wrap_add(q.ref_head, r, p.max_refs)]; };
+    if (len == 0 || t - ws > p.window) {
+        ws = t;
+        len = 0;
+        q.nruns = 0;
+        q.cn = 0;
+        for (uint32_t r = sub; r < q.ref_count; r += kGroup) {
+            RefMeta& m = ref(r);
+            m.dot = 0;
+            m.rn = 0;
+            m.cn = 0;
+            m.cur_run = 0;
+            m.cur_pos = 0;
+            m.match = 2;
+        }
+    }
+    const uint32_t o = t - ws;
+    const uint32_t oo = o * o;
+    const bool always = 0.0f >= p.similarity;
+    for (uint32_t j = 0; j < k; ++j) {
+        // one append, and every pattern's comparison with the longer
+        // window; `frozen`: no pattern takes part in a further one
+        const bool grow = q.nruns > 0 && run_value(last_run) == o;
+        if (grow) {
+            last_run += (1ull << 16);
+        } else {
+            if (q.nruns > p.window) {  // cannot happen: at most window+1 distinct offsets
+                if (sub == 0) raise_status(e, kStatusRunOverflow);
+                break;
+            }
+            if (sub == 0 && q.nruns > 0) cand[q.nruns - 1] = last_run;
+            last_run = static_cast<unsigned long long>(o) | (1ull << 16);
+            q.nruns += 1;
+        }
+        len += 1;
+        q.cn += oo;
+        bool match = always && q.ref_count > 0 && len >= 2;
+        bool frozen = true;
+        for (uint32_t r0 = 0; r0 < q.ref_count; r0 += kGroup) {
+            bool hit = false, done = true;
+            if (r0 + sub < q.ref_count) {
+                RefMeta& m = ref(r0 + sub);
+                const uint32_t mlen = m.len;
+                uint32_t state = m.match;
+                done = len >= mlen;
+                const bool advance = len <= mlen;
+                if (advance || (state == 2 && !match && len >= 2)) {
+                    RefMeta x = m;
+                    if (advance) {
+                        const unsigned long long run = ring[wrap_add(x.start, x.cur_run, p.ring_cap)];
+                        const uint32_t v = run_value(run);
+                        if (++x.cur_pos == run_count(run)) {
+                            x.cur_run += 1;
+                            x.cur_pos = 0;
+                        }
+                        x.dot += v * o;  // 16-bit values: 32-bit products
+                        x.rn += v * v;
+                        x.cn += oo;
+                        x.match = 2;
+                    }
+                    if (!match && len >= 2) x.match = cos_ge(x.dot, x.rn, x.cn, p.similarity) ? 1 : 0;
+                    state = x.match;
+                    m = x;
+                }
+                hit = state == 1;
+            }
+            match = __any_sync(mask, hit && len >= 2) || match;
+            frozen = __all_sync(mask, done) && frozen;
+        }
+        if (match) {
+            q.last_match = 1;
+            match_count += 1;
+            if (frozen) {
+                // the remaining appends change no pattern's sums: they match too
+                const uint32_t rest = k - j - 1;
+                last_run += static_cast<unsigned long long>(rest) << 16;
+                len += rest;
+                q.cn += static_cast<unsigned long long>(oo) * rest;
+                match_count += rest;
+                break;
+            }
+            continue;
+        }
+        q.last_match = 0;
+        if (len < 2) continue;
+        // learn_pattern (:31-41): FIFO with max_reference_patterns entries
+        if (q.ref_count >= p.max_refs) {
+            q.ring_used -= ref(0).nruns;
+            __syncwarp(mask);
+            q.ref_head = wrap_add(q.ref_head, 1, p.max_refs);
+            q.ref_count -= 1;
+        }
+        if (q.ring_used + q.nruns > p.ring_cap) {
+            if (sub == 0) raise_status(e, kStatusRingOverflow);
+            break;
+        }
+        if (sub == 0) cand[q.nruns - 1] = last_run;
+        __syncwarp(mask);
+        for (uint32_t i = sub; i < q.nruns; i += kGroup) ring[wrap_add(q.ring_head, i, p.ring_cap)] = cand[i];
+        if (sub == 0) {
+            RefMeta x;
+            x.dot = x.rn = x.cn = q.cn;
+            x.start = q.ring_head;
+            x.nruns = q.nruns;
+            x.len = len;
+            x.cur_run = 0;
+            x.cur_pos = 0;
+            x.match = 2;
+            ref(q.ref_count) = x;
+        }
+        q.ring_head = wrap_add(q.ring_head, q.nruns, p.ring_cap);
+        q.ring_used += q.nruns;
+        q.ref_count += 1;
+        __syncwarp(mask);
+    }
+    if (sub == 0) {
+        if (q.nruns > 0) cand[q.nruns - 1] = last_run;
+        rec->match_count = match_count;
+        rec->ws = ws;
+        rec->len = len;
+        e.ntp[n] = q;
+    }
+    __syncwarp(mask);
+}
+
+template <int kGroup>
 __global__ void __launch_bounds__(kThreads) k_temporal(Engine e) {
     const uint32_t t = e.ts->post_tick;
     const int enabled = e.ts->temporal_enabled;
-    const uint32_t sub = threadIdx.x & (kGroup - 1);
-    const uint32_t mask = kGroup == 32 ? 0xffffffffu : ((1u << (kGroup & 31)) - 1u) << (threadIdx.x & 31 & ~(kGroup - 1));
     const uint32_t groups = gridDim.x * blockDim.x / kGroup;
     for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) / kGroup; n < e.N; n += groups) {
         const uint32_t k = e.seg_start[n + 1] - e.seg_start[n];
-        if (k == 0) continue;
-        const NeuronParam p = e.nparam[n];
-        if (p.max_refs == 1) continue;  // done by k_events
-        NeuronRec* rec = e.nrec + n;
-        NeuronTp q = e.ntp[n];
-        if (!enabled) {
-            __syncwarp(mask);
-            if (sub == 0) e.ntp[n].last_match = 0;
-            continue;
-        }
-        uint32_t match_count = rec->match_count, ws = rec->ws, len = rec->len;
-        unsigned long long* cand = e.cand + p.cand_base;
-        RefMeta* meta = e.refmeta + p.meta_base;
-        unsigned long long* ring = e.ring + p.ring_base;
-        unsigned long long last_run = q.nruns > 0 ? cand[q.nruns - 1] : 0ull;
-        __syncwarp(mask);  // the group has read its state
-        auto ref = [&](uint32_t r) -> RefMeta& { return meta[wrap_add(q.ref_head, r, p.max_refs)]; };
-        if (len == 0 || t - ws > p.window) {
-            ws = t;
-            len = 0;
-            q.nruns = 0;
-            q.cn = 0;
-            for (uint32_t r = sub; r < q.ref_count; r += kGroup) {
-                RefMeta& m = ref(r);
-                m.dot = 0;
-                m.rn = 0;
-                m.cn = 0;
-                m.cur_run = 0;
-                m.cur_pos = 0;
-                m.match = 2;
-            }
-        }
-        const uint32_t o = t - ws;
-        const uint32_t oo = o * o;
-        const bool always = 0.0f >= p.similarity;
-        for (uint32_t j = 0; j < k; ++j) {
-            // one append, and every pattern's comparison with the longer
-            // window; `frozen`: no pattern takes part in a further one
-            const bool grow = q.nruns > 0 && run_value(last_run) == o;
-            if (grow) {
-                last_run += (1ull << 16);
-            } else {
-                if (q.nruns > p.window) {  // cannot happen: at most window+1 distinct offsets
-                    if (sub == 0) raise_status(e, kStatusRunOverflow);
-                    break;
-                }
-                if (sub == 0 && q.nruns > 0) cand[q.nruns - 1] = last_run;
-                last_run = static_cast<unsigned long long>(o) | (1ull << 16);
-                q.nruns += 1;
-            }
-            len += 1;
-            q.cn += oo;
-            bool match = always && q.ref_count > 0 && len >= 2;
-            bool frozen = true;
-            for (uint32_t r0 = 0; r0 < q.ref_count; r0 += kGroup) {
-                bool hit = false, done = true;
-                if (r0 + sub < q.ref_count) {
-                    RefMeta& m = ref(r0 + sub);
-                    const uint32_t mlen = m.len;
-                    uint32_t state = m.match;
-                    done = len >= mlen;
-                    const bool advance = len <= mlen;
-                    if (advance || (state == 2 && !match && len >= 2)) {
-                        RefMeta x = m;
-                        if (advance) {
-                            const unsigned long long run = ring[wrap_add(x.start, x.cur_run, p.ring_cap)];
-                            const uint32_t v = run_value(run);
-                            if (++x.cur_pos == run_count(run)) {
-                                x.cur_run += 1;
-                                x.cur_pos = 0;
-                            }
-                            x.dot += v * o;  // 16-bit values: 32-bit products
-                            x.rn += v * v;
-                            x.cn += oo;
-                            x.match = 2;
-                        }
-                        if (!match && len >= 2) x.match = cos_ge(x.dot, x.rn, x.cn, p.similarity) ? 1 : 0;
-                        state = x.match;
-                        m = x;
-                    }
-                    hit = state == 1;
-                }
-                match = __any_sync(mask, hit && len >= 2) || match;
-                frozen = __all_sync(mask, done) && frozen;
-            }
-            if (match) {
-                q.last_match = 1;
-                match_count += 1;
-                if (frozen) {
-                    // the remaining appends change no pattern's sums: they match too
-                    const uint32_t rest = k - j - 1;
-                    last_run += static_cast<unsigned long long>(rest) << 16;
-                    len += rest;
-                    q.cn += static_cast<unsigned long long>(oo) * rest;
-                    match_count += rest;
-                    break;
-                }
-                continue;
-            }
-            q.last_match = 0;
-            if (len < 2) continue;
-            // learn_pattern (:31-41): FIFO with max_reference_patterns entries
-            if (q.ref_count >= p.max_refs) {
-                q.ring_used -= ref(0).nruns;
-                __syncwarp(mask);
-                q.ref_head = wrap_add(q.ref_head, 1, p.max_refs);
-                q.ref_count -= 1;
-            }
-            if (q.ring_used + q.nruns > p.ring_cap) {
-                if (sub == 0) raise_status(e, kStatusRingOverflow);
-                break;
-            }
-            if (sub == 0) cand[q.nruns - 1] = last_run;
-            __syncwarp(mask);
-            for (uint32_t i = sub; i < q.nruns; i += kGroup) ring[wrap_add(q.ring_head, i, p.ring_cap)] = cand[i];
-            if (sub == 0) {
-                RefMeta x;
-                x.dot = x.rn = x.cn = q.cn;
-                x.start = q.ring_head;
-                x.nruns = q.nruns;
-                x.len = len;
-                x.cur_run = 0;
-                x.cur_pos = 0;
-                x.match = 2;
-                ref(q.ref_count) = x;
-            }
-            q.ring_head = wrap_add(q.ring_head, q.nruns, p.ring_cap);
-            q.ring_used += q.nruns;
-            q.ref_count += 1;
-            __syncwarp(mask);
-        }
-        if (sub == 0) {
-            if (q.nruns > 0) cand[q.nruns - 1] = last_run;
-            rec->match_count = match_count;
-            rec->ws = ws;
-            rec->len = len;
-            e.ntp[n] = q;
-        }
-        __syncwarp(mask);
+        if (k > 0 && e.nparam[n].max_refs != 1)  // (1: done by k_events)
+            temporal_group<kGroup>(e, n, k, t, enabled);
     }
 }
 
@@ -2507,6 +2563,392 @@ __global__ void __launch_bounds__(kThreads) k_expand(Engine e) {
             }
         }
         __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// small networks: whole ticks in one cluster of blocks
+// ---------------------------------------------------------------------------
+
+constexpr int kSmallThreads = 512;
+constexpr uint32_t kSmallPlaces = 4096;  // wheel positions a block keeps (fires x classes) between finding and using them
+constexpr uint32_t kSmallGroups = 64;    // shares of a tick's fires whose events are summed side by side
+
+constexpr size_t kSmallA = (kSmallEvents + 2) * sizeof(unsigned long long);  // staged due list, words in due order; then fires
+constexpr size_t kSmallB = kSmallEvents * sizeof(unsigned long long);        // words by target; then w and bits
+constexpr size_t kSmallOffTgt = kSmallA + kSmallB;
+constexpr size_t kSmallOffList = kSmallOffTgt + kSmallEvents * sizeof(uint16_t);
+constexpr size_t kSmallOffSeg = kSmallOffList + kSmallEvents * sizeof(uint16_t);
+constexpr size_t kSmallOffSlot = kSmallOffSeg + (kSmallTargets + 2) * sizeof(uint32_t);
+constexpr size_t kSmallSmem = kSmallOffSlot + kSmallSlots * sizeof(uint32_t);
+static_assert((kSmallEvents + kSmallPlaces) * sizeof(uint32_t) <= kSmallA, "fires and places");
+static_assert(kSmallTargets <= kSmallEvents / 2, "fired targets in the lists' place, targets in their second half");
+static_assert(kSmallTargets < kSharedSynapse, "targets of a block");
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Orders this thread's generic accesses with bulk copies (the async proxy).
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// A block's fires of the tick (for every block of the cluster) and its fired
+// targets.
+struct SmallFires {
+    uint2* fires;        // (due position, neuron) in global memory
+    uint32_t* targets;   // target within the block << 16 | fires
+    uint32_t n0;
+    uint32_t *n_fires, *n_targets;
+    __device__ __forceinline__ void fire(uint32_t n, uint32_t due) const { fires[atomicAdd(n_fires, 1u)] = make_uint2(due, n); }
+    __device__ __forceinline__ void target(uint32_t n, uint32_t f) const {
+        targets[atomicAdd(n_targets, 1u)] = (n - n0) << 16 | f;
+    }
+};
+
+// Ticks ts->tick .. end-1 of a small network, kSmallBlocks blocks in one
+// cluster, each with an equal share of the targets.  Per tick a block reads
+// the whole due list into shared memory and groups the events of its own
+// targets (no pass over the other blocks' data), does what k_events does with
+// them, and the post-spike STDP of its fired targets; the blocks exchange
+// their fires through global memory and a cluster barrier; every block then
+// orders all of them (a bitmap of due positions), finds their events' places
+// in the wheel, and copies its share; a second barrier ends the tick.  Every
+// block keeps the wheel's slot counts and changes them alike.
+//
+// Bound by the latency of these steps (a global read is about 0.4 us, and the
+// barriers' acquires empty L1).  As the tick's seven kernels a tick of a
+// 1,000-neuron network with 935 events took 28.8 us, four or five of them per
+// kernel boundary; here 18.8: 3.0 due list and grouping, 8.1 synapses, patterns
+// and walk, 1.4 post-spike STDP, 4.5 fires and their events, 1.5 barriers.  A
+// burst of 27,648 relayed events over 7 ticks: 42 -> 35 us a tick.  Eight blocks (a portable cluster) of 512
+// threads; a tick with more than `limit` events due (kSmallEvents, or an
+// eighth of a wheel slot: the scratch is shared out), or a target with more
+// than kRankEvents of them, ends the run of this kernel (ts->small_stop: the
+// first tick left to the other kernels): there the whole GPU is quicker.
+template <bool kInline>
+__global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads, 1)
+    k_small(const __grid_constant__ Engine e, uint32_t end, uint32_t limit) {
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    __shared__ __align__(8) unsigned long long s_bar;
+    __shared__ float s_wt[kSmallThreads / 32][32];
+    __shared__ Refire s_refire[kSmallThreads];
+    __shared__ uint32_t s_refires, s_repeats, s_next, s_fires, s_fired, s_multis;
+    __shared__ uint32_t s_part[kSmallThreads], s_sum[kMaxClasses], s_start[kMaxClasses], s_slot_of[kMaxClasses];
+    __shared__ uint32_t s_done[kMaxClasses];
+    __shared__ uint32_t s_bits[kSmallEvents / 32], s_before[kSmallEvents / 32], s_count[kSmallBlocks];
+    unsigned long long* s_due = reinterpret_cast<unsigned long long*>(s_raw);
+    unsigned long long* s_word = reinterpret_cast<unsigned long long*>(s_raw + kSmallA);
+    uint16_t* s_tgt = reinterpret_cast<uint16_t*>(s_raw + kSmallOffTgt);
+    uint16_t* s_list = reinterpret_cast<uint16_t*>(s_raw + kSmallOffList);
+    uint32_t* s_end = reinterpret_cast<uint32_t*>(s_raw + kSmallOffSeg);  // s_end[j], s_end[j + 1]: first and end of target j
+    uint32_t* s_seg = s_end + 1;
+    uint32_t* s_slot = reinterpret_cast<uint32_t*>(s_raw + kSmallOffSlot);  // events in each wheel slot
+    uint32_t* s_fire = reinterpret_cast<uint32_t*>(s_raw);                  // firing neurons in due order
+    uint32_t* s_place = s_fire + kSmallEvents;
+    const uint32_t c = blockIdx.x;
+    uint32_t t = e.ts->tick;
+    // (every block looks before any of them can write to the tick state)
+    const bool nothing = e.ts->small_stop != 0 || t >= end;
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (nothing) return;
+    const int stdp = e.ts->stdp_enabled;
+    const int temporal = e.ts->temporal_enabled;
+    unsigned long long raster = e.ts->raster_count;
+    const uint32_t D = e.D;
+    const uint32_t per = (e.N + kSmallBlocks - 1) / kSmallBlocks;
+    const uint32_t n0 = min(e.N, c * per), nw = min(e.N, n0 + per) - n0;
+    const BucketParams par{nullptr, e.nparam + n0, false};
+    const SharedEvents ev{s_due, reinterpret_cast<float*>(s_word), reinterpret_cast<uint8_t*>(s_word) + 4 * kSmallEvents};
+    uint2* all_fires = reinterpret_cast<uint2*>(e.evin);  // [block][limit]
+    const SmallFires out{all_fires + c * limit, reinterpret_cast<uint32_t*>(s_list), n0, &s_fires, &s_fired};
+    // lanes per share of the fires: a lane per class
+    uint32_t span = 1;
+    while (span < D) span <<= 1;
+    const uint32_t groups = min(kSmallGroups, kSmallThreads / span);
+    const uint32_t cls = threadIdx.x & (span - 1), group = threadIdx.x / span;
+    const uint32_t chunk = D > 0 ? kSmallBlocks * (kSmallPlaces / D) : kSmallEvents;  // fires placed at a time
+    for (uint32_t i = threadIdx.x; i < e.W; i += kSmallThreads) s_slot[i] = e.slot_count[i];
+    if (threadIdx.x == 0) mbar_init(&s_bar, 1);
+    unsigned long long delivered = 0, external = 0, fired = 0, most = 0;
+    uint32_t parity = 0;
+    bool staging = true;
+    __syncthreads();
+    for (;;) {
+        const uint32_t slot = t & e.wmask, n = s_slot[slot];
+        if (n > limit) break;
+        // far-future injections that become reachable (as k_bcount)
+        uint32_t fb, fe, fslot;
+        if (far_range(e, t, fb, fe, fslot)) {
+            const uint32_t base = s_slot[fslot];
+            const bool fits = static_cast<unsigned long long>(base) + (fe - fb) <= e.slot_cap;
+            unsigned long long* dst = e.wheel + static_cast<size_t>(fslot) * e.slot_cap + base;
+            if (fits)
+                for (uint32_t i = c * kSmallThreads + threadIdx.x; i < fe - fb; i += kSmallBlocks * kSmallThreads)
+                    dst[i] = e.far_ev[fb + i];
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                if (fits) {
+                    s_slot[fslot] = base + (fe - fb);
+                } else if (c == 0) {
+                    raise_status(e, kStatusSlotOverflow);
+                }
+            }
+        }
+        if (threadIdx.x == 0) s_fires = s_fired = s_repeats = s_next = s_multis = 0;
+        if (n > 0) {
+            const unsigned long long* due = e.wheel + static_cast<size_t>(slot) * e.slot_cap;
+            bool ready = true;
+            if (staging && threadIdx.x == 0) {
+                proxy_fence();
+                bulk_load(s_due, due, ((n + 1) & ~1u) * 8u, &s_bar);
+            }
+            for (uint32_t j = threadIdx.x; j <= nw; j += kSmallThreads) s_end[j] = 0;
+            if (staging && threadIdx.x == 0) ready = mbar_wait(&s_bar, parity, e.stage_wait_ns);
+            ready = __syncthreads_and(ready);
+            if (staging) {
+                if (!ready) {
+                    bool drained = true;
+                    if (threadIdx.x == 0) {
+                        raise_status(e, kStatusStageTimeout);
+                        drained = mbar_wait(&s_bar, parity, kDrainWaitNs);
+                    }
+                    if (!__syncthreads_and(drained)) {
+                        // (the cluster's barriers do not wait for threads that have exited)
+                        if (threadIdx.x == 0) {
+                            e.bcnt[c] = 0;
+                            __threadfence();
+                        }
+                        return;
+                    }
+                    staging = false;
+                }
+                parity ^= 1u;
+            }
+            if (!staging) {
+                for (uint32_t i = threadIdx.x; i < n; i += kSmallThreads) s_due[i] = due[i];
+                __syncthreads();
+            }
+            // this block's events, grouped by target: counts, starts, words
+            uint32_t ext = 0;
+            for (uint32_t i = threadIdx.x; i < n; i += kSmallThreads) {
+                const uint32_t lo = static_cast<uint32_t>(s_due[i]);
+                ext += lo >> 31;
+                const uint32_t j = (lo & ~kExternalBit) - n0;
+                if (j < nw) atomicAdd(&s_seg[j], 1u);
+            }
+            if (c == 0) external += __reduce_add_sync(0xffffffffu, ext);  // (per warp; lane 0 reports)
+            __syncthreads();
+            uint32_t busy = 0, longest = 0;
+            for (uint32_t j = threadIdx.x; j < nw; j += kSmallThreads) {
+                busy += s_seg[j] != 0;
+                longest = max(longest, s_seg[j]);
+            }
+            busy = __reduce_add_sync(0xffffffffu, busy);
+            if ((threadIdx.x & 31) == 0 && busy) atomicAdd(&e.ts->touched_total, static_cast<unsigned long long>(busy));
+            if (longest > kRankEvents) atomicMax(&e.ts->small_stop, t + 1);
+            __syncthreads();
+            const uint32_t total = block_scan_shared<kSmallThreads>(s_seg, nw);
+            for (uint32_t i = threadIdx.x; i < n; i += kSmallThreads) {
+                const unsigned long long v = s_due[i];
+                const uint32_t lo = static_cast<uint32_t>(v), j = (lo & ~kExternalBit) - n0;
+                if (j >= nw) continue;
+                const uint32_t p = atomicAdd(&s_seg[j], 1u);  // ends at the target's end
+                s_word[p] = (v & 0xFFFFFFFF00000000ull) | (i << 1) | (lo >> 31);
+                s_tgt[p] = static_cast<uint16_t>(j);
+            }
+            __syncthreads();
+            if (total > 0) {
+                const BucketSpace space{s_word,      s_tgt,     s_list,     s_end - 1,  &s_wt[0][0],
+                                        s_refire,    &s_repeats, &s_next,   &s_refires, s_list + kSmallEvents / 2,
+                                        &s_multis};
+                bucket_events<kInline, kSmallThreads, true>(e, space, ev, total, c * limit, n0, nw, par, t, stdp, temporal,
+                                                            out);
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) e.bcnt[c] = s_fires;
+        __syncthreads();
+        cluster_arrive();
+        // meanwhile the post-spike STDP of this block's fired targets (k_post)
+        // (a warp per target when there are as many as warps, else the block)
+        const bool by_warp = s_fired >= kSmallThreads / 32;
+        for (uint32_t k = by_warp ? threadIdx.x >> 5 : 0u; k < s_fired; k += by_warp ? kSmallThreads / 32 : 1u) {
+            const uint32_t f = out.targets[k], tgt = n0 + (f >> 16);
+            const unsigned long long last = e.in_ptr[tgt + 1];
+            for (unsigned long long tm = e.in_ptr[tgt] + (by_warp ? threadIdx.x & 31 : threadIdx.x); tm < last;
+                 tm += by_warp ? 32 : kSmallThreads) {
+                SynA a = e.syn[tm].a;
+                if (post_catch_up(a, t, f & 0xFFFFu, e, stdp, e.tab.ltp)) e.syn[tm].a = a;
+            }
+        }
+        __syncwarp();
+        cluster_wait();
+        if (threadIdx.x < kSmallBlocks) s_count[threadIdx.x] = __ldcg(e.bcnt + threadIdx.x);
+        __syncthreads();
+        uint32_t nf = 0;
+        for (uint32_t k = 0; k < kSmallBlocks; ++k) nf += s_count[k];
+        if (nf > 0) {
+            // all fires in due order: fire i of the blocks' lists, the first
+            // one of each thread kept for the second look
+            auto load_fire = [&](uint32_t i) {
+                uint32_t k = 0;
+                while (i >= s_count[k]) i -= s_count[k++];
+                return __ldcg(all_fires + k * limit + i);
+            };
+            const uint32_t words = (n + 31) / 32;
+            const uint2 mine = threadIdx.x < nf ? load_fire(threadIdx.x) : make_uint2(0u, 0u);
+            for (uint32_t w = threadIdx.x; w < words; w += kSmallThreads) s_bits[w] = 0;
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < nf; i += kSmallThreads) {
+                const uint2 x = i < kSmallThreads ? mine : load_fire(i);
+                atomicOr(&s_bits[x.x >> 5], 1u << (x.x & 31));
+            }
+            __syncthreads();
+            static_assert(kSmallEvents / 32 <= kSmallThreads, "a thread per bitmap word");
+            const uint32_t before =
+                block_excl_scan_t<kSmallThreads>(threadIdx.x < words ? __popc(s_bits[threadIdx.x]) : 0u, nullptr);
+            if (threadIdx.x < words) s_before[threadIdx.x] = before;
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < nf; i += kSmallThreads) {
+                const uint2 x = i < kSmallThreads ? mine : load_fire(i);
+                s_fire[s_before[x.x >> 5] + __popc(s_bits[x.x >> 5] & ((1u << (x.x & 31)) - 1u))] = x.y;
+            }
+            __syncthreads();
+            if (c == 0 && e.raster_cap > 0)
+                for (uint32_t r = threadIdx.x; r < nf; r += kSmallThreads) {
+                    const unsigned long long pos = raster + r;
+                    if (pos < e.raster_cap) {
+                        e.raster[2 * pos] = t;
+                        e.raster[2 * pos + 1] = s_fire[r];
+                    }
+                }
+            // events per class of a share of the fires [f0, f0 + m)
+            auto share = [&](uint32_t m, uint32_t& q0, uint32_t& q1) {
+                const uint32_t each = (m + groups - 1) / groups;
+                q0 = min(m, group * each);
+                q1 = group < groups ? min(m, q0 + each) : q0;
+            };
+            auto events_of = [&](uint32_t r) {
+                const uint32_t* row = e.pre_off + static_cast<size_t>(s_fire[r]) * (D + 1);
+                return row[cls + 1] - row[cls];
+            };
+            auto sum_shares = [&](uint32_t f0, uint32_t m) {
+                uint32_t q0, q1, sum = 0;
+                share(m, q0, q1);
+                if (cls < D)
+                    for (uint32_t q = q0; q < q1; ++q) sum += events_of(f0 + q);
+                s_part[threadIdx.x] = sum;
+                __syncthreads();
+            };
+            // the classes' totals decide whether their slots have room
+            sum_shares(0, nf);
+            if (threadIdx.x < D) {
+                uint32_t sum = 0;
+                for (uint32_t g = 0; g < groups; ++g) sum += s_part[g * span + threadIdx.x];
+                const uint32_t sl = (t + e.cls_delta[threadIdx.x]) & e.wmask;
+                s_slot_of[threadIdx.x] = sl;
+                s_start[threadIdx.x] = s_slot[sl];
+                s_done[threadIdx.x] = 0;
+                const bool fits = static_cast<unsigned long long>(s_slot[sl]) + sum <= e.slot_cap;
+                if (!fits && c == 0) raise_status(e, kStatusSlotOverflow);
+                s_sum[threadIdx.x] = fits ? sum : 0xFFFFFFFFu;
+            }
+            __syncthreads();
+            for (uint32_t f0 = 0; f0 < nf; f0 += chunk) {
+                const uint32_t m = min(chunk, nf - f0);
+                if (nf > chunk) sum_shares(f0, m);
+                uint32_t q0, q1;
+                share(m, q0, q1);
+                uint32_t pos = 0, sum = 0;
+                if (cls < D && group < groups) {
+                    pos = s_done[cls];
+                    for (uint32_t g = 0; g < groups; ++g) {
+                        const uint32_t x = s_part[g * span + cls];
+                        pos += g < group ? x : 0u;
+                        sum += x;
+                    }
+                    for (uint32_t q = q0; q < q1; ++q) {
+                        if (q % kSmallBlocks == c) s_place[q / kSmallBlocks * D + cls] = pos;
+                        pos += events_of(f0 + q);
+                    }
+                }
+                __syncthreads();
+                if (threadIdx.x < D) s_done[threadIdx.x] += sum;  // (group 0: sum over all groups)
+                // this block's fires' events, a warp per fire (k_expand)
+                for (uint32_t i = threadIdx.x >> 5; i * kSmallBlocks + c < m; i += kSmallThreads / 32) {
+                    const uint32_t src = s_fire[f0 + i * kSmallBlocks + c];
+                    const uint32_t* row = e.pre_off + static_cast<size_t>(src) * (D + 1);
+                    const unsigned long long* from = e.pre_ev + e.pre_base[src];
+                    const uint32_t lane = threadIdx.x & 31;
+                    // the fire's class offsets: in the lanes when they fit
+                    const uint32_t own = D < 32 && lane <= D ? row[lane] : 0u;
+                    const uint32_t k0 = D < 32 ? __shfl_sync(0xffffffffu, own, 0) : row[0];
+                    const uint32_t k1 = D < 32 ? __shfl_sync(0xffffffffu, own, D & 31) : row[D];
+                    for (uint32_t kb = k0; kb < k1; kb += 32) {
+                        const uint32_t k = kb + lane;
+                        const unsigned long long v = k < k1 ? from[k] : 0ull;
+                        uint32_t d = 0, first = 0;  // row[d] = first <= k < row[d + 1]
+                        if (D < 32) {
+#pragma unroll
+                            for (uint32_t step = 16; step > 0; step >>= 1) {
+                                const uint32_t x = __shfl_sync(0xffffffffu, own, (d + step) & 31);
+                                if (d + step < D && x <= k) d += step;
+                            }
+                            first = __shfl_sync(0xffffffffu, own, d);
+                        } else {
+                            uint32_t above = D;
+                            while (above - d > 1) {
+                                const uint32_t mid = (d + above) >> 1;
+                                if (row[mid] <= k) {
+                                    d = mid;
+                                } else {
+                                    above = mid;
+                                }
+                            }
+                            first = row[d];
+                        }
+                        if (k < k1 && s_sum[d] != 0xFFFFFFFFu)
+                            e.wheel[static_cast<size_t>(s_slot_of[d]) * e.slot_cap + s_start[d] + s_place[i * D + d] +
+                                    (k - first)] = v;
+                    }
+                }
+                __syncthreads();
+            }
+            if (threadIdx.x < D && s_sum[threadIdx.x] != 0xFFFFFFFFu)
+                s_slot[s_slot_of[threadIdx.x]] += s_sum[threadIdx.x];
+            if (e.raster_cap > 0) {
+                if (c == 0 && threadIdx.x == 0 && raster + nf > e.raster_cap) raise_status(e, kStatusRasterOverflow);
+                raster += nf;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_slot[slot] = 0;
+        delivered += n;
+        fired += nf;
+        most = n > most ? n : most;
+        proxy_fence();  // (the next due list, written here, comes in by a bulk copy)
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        ++t;
+        if (t >= end) break;
+        const uint32_t stop = __ldcg(&e.ts->small_stop);
+        if (stop != 0 && stop <= t) break;
+        __syncthreads();
+    }
+    __syncthreads();
+    if (c != 0) return;
+    for (uint32_t i = threadIdx.x; i < e.W; i += kSmallThreads) e.slot_count[i] = s_slot[i];
+    if ((threadIdx.x & 31) == 0 && external) atomicAdd(&e.ts->external, external);
+    if (threadIdx.x == 0) {
+        TickState* ts = e.ts;
+        if (t < end) atomicMax(&ts->small_stop, t == 0 ? 1u : t);
+        ts->tick = t;
+        ts->delivered += delivered;
+        ts->fired += fired;
+        if (most > ts->max_slot_events) ts->max_slot_events = most;
+        ts->raster_count = raster;
     }
 }
 
@@ -2888,6 +3330,8 @@ void configure_kernels() {
     const int events_bytes = static_cast<int>(std::max(events_smem(kMaxBucketShift), events_smem(8)));
     cudaFuncSetAttribute(k_events<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
     cudaFuncSetAttribute(k_events<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, events_bytes);
+    cudaFuncSetAttribute(k_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmallSmem));
+    cudaFuncSetAttribute(k_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmallSmem));
 }
 
 void configure_group() {
@@ -2897,6 +3341,14 @@ void configure_group() {
     cudaFuncSetAttribute(k_bscatter, cudaFuncAttributeMaxDynamicSharedMemorySize, bucket_bytes);
     cudaFuncSetAttribute(k_group, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          static_cast<int>(group_smem(kMaxBucketShift)));
+}
+
+void launch_small(const Engine& e, uint32_t end, uint32_t limit, cudaStream_t stream) {
+    if (e.inline_codes) {
+        k_small<true><<<kSmallBlocks, kSmallThreads, kSmallSmem, stream>>>(e, end, limit);
+    } else {
+        k_small<false><<<kSmallBlocks, kSmallThreads, kSmallSmem, stream>>>(e, end, limit);
+    }
 }
 
 void launch_init_syn(const Engine& e, const SynA* a, cudaStream_t stream) {

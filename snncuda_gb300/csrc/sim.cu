@@ -191,6 +191,10 @@ struct snncuda_sim {
     unsigned char* inj{nullptr};
     size_t inj_cap{0};
     uint32_t far_ticks_set{0};  // TickState::far_ticks on the device between runs
+    uint32_t run_far[2]{};      // the run's TickState::far_first_tick, far_ticks
+    // Runs go to k_small until it has met a tick that it does not take.
+    bool small{false};
+    bool small_run{false};      // the run in flight does
     // graphs
     cudaGraphExec_t graph_many{nullptr};
     cudaGraphExec_t graph_one{nullptr};
@@ -560,6 +564,7 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     // large networks: post-spike STDP in tick order (two random-access
     // kernels side by side slowed each other by more than the overlap gave)
     e.side_serial = e.S >= (1ull << 26) ? 1u : 0u;
+    sim->small = small_network(e);
     sim->ensure_far(1, 2);
     check(cudaStreamSynchronize(st), "create synchronize");
 }
@@ -954,6 +959,55 @@ void sort_pending(snncuda_sim* sim) {
     }
 }
 
+// Run parameters live in device memory so the captured graphs stay valid.
+void set_far(snncuda_sim* sim, uint32_t ticks) {
+    if (ticks == 0 && sim->far_ticks_set == 0) return;
+    const uint32_t params[2] = {sim->run_far[0], ticks};
+    static_assert(offsetof(TickState, far_ticks) == offsetof(TickState, far_first_tick) + 4, "copied together");
+    check(cudaMemcpyAsync(reinterpret_cast<char*>(sim->e.ts) + offsetof(TickState, far_first_tick), params, sizeof(params),
+                          cudaMemcpyHostToDevice, sim->stream), "run params");
+    sim->far_ticks_set = ticks;
+}
+
+// Enqueues ticks p .. T (none if T < p) and the copies that end a run.
+void enqueue_ticks(snncuda_sim* sim, uint64_t p, uint64_t T) {
+    Engine& e = sim->e;
+    cudaStream_t st = sim->stream;
+    uint64_t ticks = T + 1 - p;
+    if (sim->small_run) {
+        // in launches of a few milliseconds, so that other streams' kernels
+        // get the SMs in between
+        constexpr uint64_t kLaunch = 512;
+        for (uint64_t first = p; first <= T; first += kLaunch)
+            launch_small(e, static_cast<uint32_t>(std::min(T, first + kLaunch - 1) + 1), small_limit(e), st);
+        check(cudaGetLastError(), "tick launch");
+        ticks = 0;
+    }
+    if (ticks >= sim->ticks_per_graph && sim->graph_many == nullptr)
+        sim->graph_many = sim->capture(static_cast<int>(sim->ticks_per_graph));
+    if (ticks > 0 && sim->graph_one == nullptr) sim->graph_one = sim->capture(1);
+    while (ticks >= sim->ticks_per_graph) {
+        check(cudaGraphLaunch(sim->graph_many, st), "graph launch");
+        ticks -= sim->ticks_per_graph;
+    }
+    while (ticks > 0) {
+        check(cudaGraphLaunch(sim->graph_one, st), "graph launch");
+        ticks -= 1;
+    }
+    set_far(sim, 0);
+    if (sim->ts_pinned == nullptr)
+        check(cudaMallocHost(reinterpret_cast<void**>(&sim->ts_pinned), sizeof(TickState)), "pinned tick state");
+    if (sim->counts_pinned == nullptr)
+        check(cudaMallocHost(reinterpret_cast<void**>(&sim->counts_pinned), e.W * sizeof(uint32_t)),
+              "pinned slot counts");
+    if (sim->run_done == nullptr) check(cudaEventCreateWithFlags(&sim->run_done, cudaEventDisableTiming), "event");
+    check(cudaMemcpyAsync(sim->ts_pinned, e.ts, sizeof(TickState), cudaMemcpyDeviceToHost, st), "read tick state");
+    check(cudaMemcpyAsync(sim->counts_pinned, e.slot_count, e.W * sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
+          "read slot counts");
+    check(cudaEventRecord(sim->run_done, st), "event record");
+}
+
+
 // Enqueues ticks next_tick .. T on the simulation's stream and returns
 // without waiting; run_complete() waits and checks the device status.
 void run_enqueue(snncuda_sim* sim, uint64_t T, snncuda_profile* prof) {
@@ -1046,16 +1100,9 @@ void run_enqueue(snncuda_sim* sim, uint64_t T, snncuda_profile* prof) {
         sim->pend_sorted -= head;
         sim->pend_head = 0;
     }
-    // run parameters live in device memory so the captured graphs stay valid
-    auto set_far = [&](uint32_t n) {
-        if (n == 0 && sim->far_ticks_set == 0) return;
-        const uint32_t params[2] = {far_first, n};
-        static_assert(offsetof(TickState, far_ticks) == offsetof(TickState, far_first_tick) + 4, "copied together");
-        check(cudaMemcpyAsync(reinterpret_cast<char*>(e.ts) + offsetof(TickState, far_first_tick), params,
-                              sizeof(params), cudaMemcpyHostToDevice, st), "run params");
-        sim->far_ticks_set = n;
-    };
-    set_far(far_ticks);
+    sim->run_far[0] = far_first;
+    sim->run_far[1] = far_ticks;
+    set_far(sim, far_ticks);
     uint64_t ticks = T - p + 1;
     if (prof != nullptr) {
         const TickState before = sim->read_ts();
@@ -1077,29 +1124,9 @@ void run_enqueue(snncuda_sim* sim, uint64_t T, snncuda_profile* prof) {
         prof->touched_targets += after.touched_total - before.touched_total;
         ticks = 0;
     }
-    if (ticks >= sim->ticks_per_graph && sim->graph_many == nullptr)
-        sim->graph_many = sim->capture(static_cast<int>(sim->ticks_per_graph));
-    if (ticks > 0 && sim->graph_one == nullptr) sim->graph_one = sim->capture(1);
-    while (ticks >= sim->ticks_per_graph) {
-        check(cudaGraphLaunch(sim->graph_many, st), "graph launch");
-        ticks -= sim->ticks_per_graph;
-    }
-    while (ticks > 0) {
-        check(cudaGraphLaunch(sim->graph_one, st), "graph launch");
-        ticks -= 1;
-    }
-    set_far(0);
-    if (sim->ts_pinned == nullptr)
-        check(cudaMallocHost(reinterpret_cast<void**>(&sim->ts_pinned), sizeof(TickState)), "pinned tick state");
-    if (sim->counts_pinned == nullptr)
-        check(cudaMallocHost(reinterpret_cast<void**>(&sim->counts_pinned), e.W * sizeof(uint32_t)),
-              "pinned slot counts");
-    if (sim->run_done == nullptr) check(cudaEventCreateWithFlags(&sim->run_done, cudaEventDisableTiming), "event");
-    check(cudaMemcpyAsync(sim->ts_pinned, e.ts, sizeof(TickState), cudaMemcpyDeviceToHost, st), "read tick state");
-    check(cudaMemcpyAsync(sim->counts_pinned, e.slot_count, e.W * sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
-          "read slot counts");
-    check(cudaEventRecord(sim->run_done, st), "event record");
     sim->run_target = T;
+    sim->small_run = sim->small && ticks > 0;
+    enqueue_ticks(sim, p, prof == nullptr ? T : p - 1);
     sim->run_in_flight = true;
 }
 
@@ -1114,11 +1141,24 @@ bool run_complete(snncuda_sim* sim, bool wait) {
         if (q == cudaErrorNotReady) return false;
         check(q, "run query");
     }
+    const uint64_t T = sim->run_target;
+    if (sim->small_run && sim->ts_pinned->small_stop != 0) {
+        // k_small left the run's last ticks: the other kernels take them, and
+        // this simulation's later runs
+        sim->small = sim->small_run = false;
+        const TickState at = *sim->ts_pinned;
+        const uint32_t none = 0;
+        check(cudaMemcpyAsync(&sim->e.ts->small_stop, &none, sizeof(none), cudaMemcpyHostToDevice, sim->stream), "run params");
+        if (at.tick <= T) {
+            set_far(sim, sim->run_far[1]);
+            enqueue_ticks(sim, at.tick, T);
+            return wait ? run_complete(sim, true) : false;
+        }
+    }
     sim->run_in_flight = false;
     sim->stage_in_use = false;
     sim->pinned_current = true;
     const TickState ts = *sim->ts_pinned;
-    const uint64_t T = sim->run_target;
     sim->next_tick = T + 1;
     if (ts.tick != static_cast<uint32_t>(T + 1)) throw_fail(SNNCUDA_ERR_DEVICE, "device tick counter out of step");
     if (ts.status != 0) {
