@@ -249,8 +249,8 @@ struct Engine {
     // complete instead of going to DRAM half-written.
     uint32_t scatter_pass_events;
     // 1: k_post and k_temporal run on the main stream in tick order instead
-    // of on the side stream beside the fire ordering (two random-access
-    // kernels side by side can take longer than one after the other).
+    // of on the side stream beside the fire ordering (on very large networks
+    // the two slow each other by more than the overlap gives).
     uint32_t side_serial;
     uint32_t inline_codes;                 // 1: inline_code_pattern holds for every target
     uint32_t multi_refs;                   // 1: some target keeps several reference patterns (k_temporal runs)

@@ -561,9 +561,10 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     e.grid_process = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((N + 255) / 256, sms * 8ull)));
     e.grid_walk = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((N + 63) / 64, sms * 8ull)));
     e.grid_fire = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(fire_tiles, sms * 8ull)));
-    // large networks: post-spike STDP in tick order (two random-access
-    // kernels side by side slowed each other by more than the overlap gave)
-    e.side_serial = e.S >= (1ull << 26) ? 1u : 0u;
+    // Post-spike STDP beside the fire ordering or in tick order: a tick of
+    // 7e7 synapses takes 124 us beside and 130 in order, of 2e8 334 and 348,
+    // of 6e8 1,015 and 1,001 (there both move enough bytes to slow each other)
+    e.side_serial = e.S >= (1ull << 28) ? 1u : 0u;
     sim->small = small_network(e);
     sim->ensure_far(1, 2);
     check(cudaStreamSynchronize(st), "create synchronize");

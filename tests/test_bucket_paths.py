@@ -52,8 +52,10 @@ def _run(lib, n, net, advance):
     return out
 
 
-# about 1.5 delays x codes per tick: each case reaches its limit in some tick
-@pytest.mark.parametrize("hub,other", [(0, 40), (33, 5), (511, 0), (700, 100), (1023, 300), (1400, 1300), (4000, 0)])
+# about 1.5 delays x codes per tick: each case reaches its limit in some tick;
+# 257, 1024 and 1025 are edges of the rows that post-spike STDP reads at once
+@pytest.mark.parametrize("hub,other", [(0, 40), (33, 5), (257, 0), (511, 0), (700, 100), (1023, 300), (1024, 0),
+                                       (1025, 0), (1400, 1300), (4000, 0)])
 @pytest.mark.parametrize("threshold,patterns,codes", [(1e6, 1, 1), (0.8, 1, 4), (0.8, 3, 6)])
 def test_busy_targets(gpu_lib, port_lib, hub, other, threshold, patterns, codes):
     n, net = _fan_in(hub, other, threshold, patterns, codes, hub + other)
