@@ -701,14 +701,22 @@ int snncuda_readout_create(const snncuda_network* net, snncuda_readout** out) {
         // incoming synapses of each neuron in Connectome order (stable
         // counting sort by target)
         std::vector<unsigned long long> ptr(static_cast<size_t>(N) + 1, 0);
+        uint64_t run = 0;  // first synapse of the current run of one source
         for (uint64_t k = 0; k < S; ++k) {
             if (net->source[k] >= N || net->target[k] >= N)
                 throw Fail{SNNCUDA_ERR_INVALID_ARGUMENT, "synapse endpoint out of range"};
             ++ptr[net->target[k] + 1];
-            ++r->degree[net->target[k]];
-            ++r->degree[net->source[k]];
+            // synapses usually come source by source: one update a run
+            if (k > 0 && net->source[k] != net->source[run]) {
+                r->degree[net->source[run]] += k - run;
+                run = k;
+            }
         }
-        for (uint32_t n = 0; n < N; ++n) ptr[n + 1] += ptr[n];
+        if (S > 0) r->degree[net->source[run]] += S - run;
+        for (uint32_t n = 0; n < N; ++n) {
+            r->degree[n] += ptr[n + 1];  // still the count of n's incoming synapses
+            ptr[n + 1] += ptr[n];
+        }
         std::vector<unsigned long long> fill(ptr.begin(), ptr.end() - 1);
         std::vector<uint32_t> src(S), dly(S);
         std::vector<float> w(S);
