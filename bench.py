@@ -69,11 +69,19 @@ if "--serve" in sys.argv:
 METRIC = "synaptic_events_per_s"
 UNIT = "events/s"
 ORACLE = ROOT / "oracle" / "_build" / "liboracle_port.so"
-# kernels per tick (launch_tick in snncuda_gb300/csrc/kernels.cu): the
-# profile API's kernel count; plus one injection kernel per timed step
-def kernels_per_tick():
-    from snncuda_gb300 import _abi
-    return _abi.KERNEL_COUNT
+# Kernels per tick (launch_tick in snncuda_gb300/csrc/kernels.cu): k_bcount,
+# k_bscatter, k_events, k_fire_list, k_fire_count, k_expand, k_post
+# (k_temporal, only launched when a target keeps several patterns, is not
+# counted).
+KERNELS_PER_TICK = 7
+SMALL_NEURONS = 8 * 4096  # networks up to this size run many ticks per launch (k_small)
+
+
+def gpu_launches(neurons, ticks, steps):
+    """Kernels launched in the timed steps, counted low: one injection kernel
+    per step, plus the tick kernels (one k_small per step on small networks)."""
+    return steps + (steps if neurons <= SMALL_NEURONS else ticks * KERNELS_PER_TICK)
+
 
 # Minimal algorithmic bytes of a compact structure-of-arrays design of the
 # tick, per fire F, synaptic event E, external event X, touched target U:
@@ -86,33 +94,28 @@ def kernels_per_tick():
 #                          bound) and code-state write
 #   U * 48 + X * 8         touched neurons' state read-modify-write, externals
 #   F * fanin * 16         post-spike STDP over the fired neurons' in-rows
-# Per kernel: the synapse-side kernel k_events carries the delivery read and
-# the synapse terms (8 + 29 + 20 = 57 B per synaptic event, 8 B per
-# external); k_process the touched-neuron term.  (per synaptic event, per
-# external event, per touched target)
+# Per kernel: k_events carries the delivery read and the synapse terms
+# (8 + 29 + 20 = 57 B per synaptic event, 8 B per external) and the
+# touched-neuron term.  (per synaptic event, per external event, per touched
+# target)
 MINIMAL_BYTES = {
-    "k_events": (57, 8, 0),
-    "k_process": (0, 0, 48),
+    "k_events": (57, 8, 48),
 }
 # Bytes of this engine's own layout (snncuda_gb300/csrc/engine.h) per
 # synaptic event, external event and touched target:
-#   k_events   grouped entry (8), synapse record read + write (2 x 64), event
-#              input (16), the record's changing fields before the event (16);
-#              externals: entry + input; per target its parameters (64) and
-#              segment bounds (8)
-#   k_process  event input (16); per target its threshold (4) and the
-#              physics fields of its record, read + write (2 x 52)
+#   k_events   bucketed entry (16), synapse record read + write (2 x 64);
+#              externals: entry; per target its parameters (64), neuron
+#              record and temporal bookkeeping, read + write (2 x 64 + 2 x 32)
 LAYOUT_BYTES = {
-    "k_events": (8 + 64 + 64 + 16 + 16, 8 + 16, 64 + 8),
-    "k_process": (16, 16, 4 + 2 * 52),
+    "k_events": (16 + 64 + 64, 16, 64 + 2 * 64 + 2 * 32),
 }
 # DRAM bytes (read + write) per synaptic event of a kernel, from one ncu
-# capture (dram__bytes_read.sum + dram__bytes_write.sum) of all 240 k_events
-# launches of the timed steps of a 20,000-neuron case of recog_1m (7.863 GB
-# over 59.87 M synaptic events: 127.2 B read, 4.2 B written; the records'
+# capture (dram__bytes_read.sum + dram__bytes_write.sum) of the 80 k_events
+# launches of a timed step of a 40,000-neuron case of recog_1m (7.590 GB over
+# 39.75 M synaptic events: 159.8 B read, 31.2 B written; most of the records'
 # write-back happens after the kernel); roofline.traffic scales it to the
 # events of one full-size launch.
-MEASURED_TRAFFIC_PER_EVENT = {"k_events": 131.3}
+MEASURED_TRAFFIC_PER_EVENT = {"k_events": 190.9}
 
 
 def load_peaks():
@@ -854,7 +857,7 @@ def main():
     ap.add_argument("--batch-networks", type=int, default=64,
                     help="networks of the batched leg of the default run (0 skips it)")
     ap.add_argument("--rmw-floor", action="store_true",
-                    help="time random 64-byte record read-modify-writes (the per-event access floor)")
+                    help="time random 64-byte record read-modify-writes")
     ap.add_argument("--rmw-args", default="",
                     help="records events [bands band_len picks rows row_len] for --rmw-floor")
     ap.add_argument("--group-bench", default="",
@@ -974,7 +977,7 @@ def main():
             "ticks_per_s": steps_ticks / (ms_max / 1e3),
             "fires_per_tick": r["fires"] / steps_ticks,
             "events_per_tick": r["events"] / steps_ticks,
-            "gpu_launches": steps_ticks * kernels_per_tick() + args.steps,
+            "gpu_launches": gpu_launches(w.neurons, steps_ticks, args.steps),
             "tick_roofline": tick_roofline(w, r["events"], r["fires"], r["ext"], prof, steps_ticks, ms_max),
             "clocks": r["clocks"], "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
             **({"recognition": r["recognition"]} if r["recognition"] is not None else {}),
