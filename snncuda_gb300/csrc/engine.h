@@ -14,6 +14,7 @@
 //     scheduling order (the reference bucket FIFO order).
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 
 namespace snngb {
@@ -297,7 +298,7 @@ constexpr uint32_t kMaxBucketShift = 14;  // at most 2^14 targets per bucket: N 
 
 // Targets per bucket (log2) for N targets: the smallest 2^s >= 256 with at
 // most kMaxBuckets buckets.  Returns 0 when N needs more than 2^28 targets.
-__host__ __device__ inline uint32_t bucket_shift_for(uint32_t N) {
+__host__ __device__ constexpr uint32_t bucket_shift_for(uint32_t N) {
     uint32_t s = 8;
     while (((static_cast<unsigned long long>(N) + (1ull << s) - 1) >> s) > kMaxBuckets) ++s;
     return s <= kMaxBucketShift ? s : 0;
@@ -317,6 +318,47 @@ inline uint32_t tick_bucket_shift(uint32_t N, uint32_t sms) {
     while (((static_cast<unsigned long long>(N) + (1ull << s) - 1) >> s) > kMaxTickBuckets) ++s;
     return s;
 }
+
+// Grouping entry points: blocks of the counting and placing kernels, at most
+// (fixed, so that the static scratch has a fixed size), and the longest segment
+// that a warp of k_group_rest sorts.
+constexpr uint32_t kGroupGrid = 256;
+constexpr uint32_t kWarpSortEvents = 512;
+
+constexpr uint32_t group_buckets(uint32_t neuron_count) {
+    const uint32_t shift = bucket_shift_for(neuron_count);
+    const uint64_t n = (static_cast<uint64_t>(neuron_count) + (1u << shift) - 1) >> shift;
+    return n > 0 ? static_cast<uint32_t>(n) : 1u;
+}
+
+// Entries of a grouping call's Engine::bcnt: the counting blocks' rows of
+// counters, in whose memory k_group then lists the targets that have more than
+// kWarpSortEvents events each.  `count` events hold at most count /
+// (kWarpSortEvents + 1) of them: more than the rows hold where a bucket is
+// wider than kGroupGrid targets (above 2^22 neurons) and most targets are busy.
+constexpr size_t group_counters(uint32_t count, uint32_t neuron_count) {
+    const size_t rows = static_cast<size_t>(kGroupGrid) * group_buckets(neuron_count);
+    const size_t listed = count / (kWarpSortEvents + 1);
+    return rows > listed ? rows : listed;
+}
+
+// Byte offsets (256-byte aligned) of a grouping call's arrays in its scratch.
+struct GroupLayout {
+    size_t bcnt, btot, bstart, bcur, grp_tmp, slot_count, ts, bytes;
+};
+constexpr GroupLayout group_layout(uint32_t count, uint32_t neuron_count) {
+    const size_t buckets = group_buckets(neuron_count);
+    GroupLayout l{};
+    l.btot = l.bcnt + (group_counters(count, neuron_count) * 4 + 255) / 256 * 256;
+    l.bstart = l.btot + (buckets * 4 + 255) / 256 * 256;
+    l.bcur = l.bstart + ((buckets + 1) * 4 + 255) / 256 * 256;
+    l.grp_tmp = l.bcur + (buckets * 4 + 255) / 256 * 256;
+    l.slot_count = l.grp_tmp + ((count > 0 ? count : 1u) * sizeof(BucketEntry) + 255) / 256 * 256;
+    l.ts = l.slot_count + 256;
+    l.bytes = l.ts + (sizeof(TickState) + 255) / 256 * 256;
+    return l;
+}
+
 constexpr int kExpandFires = 8;          // fires per expansion block (one warp each)
 constexpr uint32_t kMaxClasses = 256;    // distinct delivery delays
 

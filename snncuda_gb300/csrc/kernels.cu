@@ -1190,10 +1190,9 @@ __device__ __forceinline__ void for_entries(const uint4* in, uint32_t m, uint32_
 }
 
 // Events k_group holds in shared memory (each thread its share in registers
-// first), and the longest segment a warp of k_group_rest sorts.
+// first).
 constexpr uint32_t kSortSmemEvents = 4096;
 constexpr uint32_t kSortPerThread = kSortSmemEvents / kThreads;
-constexpr uint32_t kWarpSortEvents = 512;
 constexpr size_t kSortSmemBytes = kSortSmemEvents * (sizeof(unsigned long long) + sizeof(uint16_t));
 
 // Grouping entry points: one block per bucket.  A bucket that fits is counted
@@ -1271,6 +1270,7 @@ __global__ void __launch_bounds__(kThreads) k_group(const __grid_constant__ Engi
             });
             // the segments are sorted by k_group_rest, over the whole GPU: the
             // totals and counts are used up, their memory takes its lists
+            // (group_counters)
             if (threadIdx.x == 0) e.btot[atomicAdd(&e.ts->n_touched, 1u)] = b;
             __syncthreads();
             for (uint32_t j = threadIdx.x; j < nw; j += blockDim.x) {

@@ -1843,32 +1843,10 @@ int snncuda_sim_residency(snncuda_sim* sim, int32_t* resident_out, uint64_t* evi
 
 namespace {
 
-// Scratch of one grouping call (device pointers).
-struct GroupScratch {
-    uint32_t* bcnt;       // kGroupGrid x buckets
-    uint32_t* btot;       // buckets
-    uint32_t* bstart;     // buckets + 1
-    uint32_t* bcur;       // buckets
-    BucketEntry* grp_tmp;  // count
-    uint32_t* slot_count;
-    TickState* ts;
-};
-
-// Blocks of the grouping entry points' counting and placing kernels (fixed,
-// so the static scratch has a fixed size).
-constexpr uint32_t kGroupGrid = 256;
-
-uint32_t group_buckets(uint32_t neuron_count) {
-    const uint32_t shift = bucket_shift_for(neuron_count);
-    return static_cast<uint32_t>(std::max<uint64_t>(1, (static_cast<uint64_t>(neuron_count) + (1u << shift) - 1) >> shift));
-}
-
 // The tick's counting and placing kernels, then k_group, on a caller's event
-// buffer seen as a one-slot wheel.  Scratch sizes: kGroupGrid x
-// group_buckets() counts, group_buckets() (+1) bucket totals, starts and
-// cursors, `count` bucket-ordered events (BucketEntry).
+// buffer seen as a one-slot wheel; `scratch` is laid out as `l`.
 void group_run(const uint64_t* events, uint32_t count, uint32_t neuron_count, uint64_t* grouped,
-               uint32_t* segment_start, cudaStream_t st, const GroupScratch& sc) {
+               uint32_t* segment_start, cudaStream_t st, unsigned char* scratch, const GroupLayout& l) {
     int dev = 0, sms = 0;
     check(cudaGetDevice(&dev), "cudaGetDevice");
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
@@ -1878,27 +1856,27 @@ void group_run(const uint64_t* events, uint32_t count, uint32_t neuron_count, ui
     e.wmask = 0;
     e.slot_cap = count;
     e.wheel = const_cast<unsigned long long*>(reinterpret_cast<const unsigned long long*>(events));
-    e.slot_count = sc.slot_count;
+    e.slot_count = reinterpret_cast<uint32_t*>(scratch + l.slot_count);
     e.bucket_shift = bucket_shift_for(neuron_count);
     e.nbuckets = group_buckets(neuron_count);
     // a chunk of at least 2,048 events per block (fewer blocks: fewer counter rows)
     e.grid_bucket = std::max(1u, std::min(kGroupGrid, (count + 2047) / 2048));
     e.scatter_pass_events = kScatterPassEvents;
     e.stage_wait_ns = 100000000ull;  // the bulk copies' wait limit (as snncuda_config's default)
-    e.bcnt = sc.bcnt;
-    e.btot = sc.btot;
-    e.bstart = sc.bstart;
-    e.bcur = sc.bcur;
+    e.bcnt = reinterpret_cast<uint32_t*>(scratch + l.bcnt);
+    e.btot = reinterpret_cast<uint32_t*>(scratch + l.btot);
+    e.bstart = reinterpret_cast<uint32_t*>(scratch + l.bstart);
+    e.bcur = reinterpret_cast<uint32_t*>(scratch + l.bcur);
     e.seg_start = segment_start;
     e.grp = reinterpret_cast<unsigned long long*>(grouped);
-    e.grp_tmp = sc.grp_tmp;
-    e.ts = sc.ts;
+    e.grp_tmp = reinterpret_cast<BucketEntry*>(scratch + l.grp_tmp);
+    e.ts = reinterpret_cast<TickState*>(scratch + l.ts);
     e.grid_wide = static_cast<uint32_t>(std::max(1, sms * 2));
     configure_group();
     launch_group(e, count, st);
     check(cudaGetLastError(), "group launch");
     uint32_t status = 0;
-    check(cudaMemcpyAsync(&status, &sc.ts->status, sizeof(status), cudaMemcpyDeviceToHost, st), "status");
+    check(cudaMemcpyAsync(&status, &e.ts->status, sizeof(status), cudaMemcpyDeviceToHost, st), "status");
     check(cudaStreamSynchronize(st), "group synchronize");
     if (status & kStatusBadEvent) throw_fail(SNNCUDA_ERR_INVALID_ARGUMENT, "event target >= neuron_count");
 }
@@ -1916,26 +1894,9 @@ int snncuda_group_events(const uint64_t* events, uint32_t count, uint32_t neuron
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     unsigned char* scratch = nullptr;  // (a stream-ordered one of 215 MB took 2.9 ms: the default pool keeps nothing)
     const int rc = guarded([&] {
-        const size_t buckets = group_buckets(neuron_count);
-        size_t bytes = 0;
-        auto place = [&](size_t n) {
-            const size_t at = bytes;
-            bytes = (bytes + n + 255) / 256 * 256;
-            return at;
-        };
-        const size_t tmp = place(std::max<size_t>(count, 1) * sizeof(BucketEntry)), bcnt = place(kGroupGrid * buckets * 4),
-                     btot = place(buckets * 4), bstart = place((buckets + 1) * 4), bcur = place(buckets * 4),
-                     slot = place(sizeof(uint32_t)), state = place(sizeof(TickState));
-        check(cudaMalloc(reinterpret_cast<void**>(&scratch), bytes), "cudaMalloc");
-        GroupScratch sc;
-        sc.bcnt = reinterpret_cast<uint32_t*>(scratch + bcnt);
-        sc.btot = reinterpret_cast<uint32_t*>(scratch + btot);
-        sc.bstart = reinterpret_cast<uint32_t*>(scratch + bstart);
-        sc.bcur = reinterpret_cast<uint32_t*>(scratch + bcur);
-        sc.grp_tmp = reinterpret_cast<BucketEntry*>(scratch + tmp);
-        sc.slot_count = reinterpret_cast<uint32_t*>(scratch + slot);
-        sc.ts = reinterpret_cast<TickState*>(scratch + state);
-        group_run(events, count, neuron_count, grouped, segment_start, st, sc);
+        const GroupLayout l = group_layout(count, neuron_count);
+        check(cudaMalloc(reinterpret_cast<void**>(&scratch), l.bytes), "cudaMalloc");
+        group_run(events, count, neuron_count, grouped, segment_start, st, scratch, l);
     });
     if (rc != SNNCUDA_OK) cudaStreamSynchronize(st);
     if (scratch) cudaFree(scratch);
@@ -1947,21 +1908,11 @@ namespace {
 // Static scratch of snncuda_group_events_static: bucket counters and the
 // bucket-ordered events for at most kStaticEvents events over kStaticNeurons
 // neurons (about 17 MB).
-constexpr size_t kStaticEvents = SNNCUDA_GROUP_STATIC_MAX_EVENTS;
-constexpr size_t kStaticNeurons = SNNCUDA_GROUP_STATIC_MAX_NEURONS;
-constexpr size_t kStaticBuckets = (kStaticNeurons + 255) / 256;  // bucket_shift_for(2^18) == 8
-static_assert(kStaticBuckets <= kMaxBuckets, "static grouping buckets");
-constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
-constexpr size_t kOffBcnt = 0;
-constexpr size_t kOffBtot = kOffBcnt + align256(kGroupGrid * kStaticBuckets * 4);
-constexpr size_t kOffBstart = kOffBtot + align256(kStaticBuckets * 4);
-constexpr size_t kOffBcur = kOffBstart + align256((kStaticBuckets + 1) * 4);
-constexpr size_t kOffGrpTmp = kOffBcur + align256(kStaticBuckets * 4);
-constexpr size_t kOffSlot = kOffGrpTmp + align256(kStaticEvents * sizeof(BucketEntry));
-constexpr size_t kOffTs = kOffSlot + 256;
-constexpr size_t kStaticBytes = kOffTs + align256(sizeof(TickState));
+constexpr uint32_t kStaticEvents = SNNCUDA_GROUP_STATIC_MAX_EVENTS;
+constexpr uint32_t kStaticNeurons = SNNCUDA_GROUP_STATIC_MAX_NEURONS;
+constexpr GroupLayout kStaticLayout = group_layout(kStaticEvents, kStaticNeurons);
 
-static __device__ __align__(256) unsigned char g_group_scratch[kStaticBytes];
+static __device__ __align__(256) unsigned char g_group_scratch[kStaticLayout.bytes];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mutex;
@@ -2002,16 +1953,7 @@ int snncuda_group_events_static(const uint64_t* events, uint32_t count, uint32_t
                          "use snncuda_group_events");
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     const int rc = guarded([&] {
-        unsigned char* base = static_scratch(st);
-        GroupScratch sc;
-        sc.bcnt = reinterpret_cast<uint32_t*>(base + kOffBcnt);
-        sc.btot = reinterpret_cast<uint32_t*>(base + kOffBtot);
-        sc.bstart = reinterpret_cast<uint32_t*>(base + kOffBstart);
-        sc.bcur = reinterpret_cast<uint32_t*>(base + kOffBcur);
-        sc.grp_tmp = reinterpret_cast<BucketEntry*>(base + kOffGrpTmp);
-        sc.slot_count = reinterpret_cast<uint32_t*>(base + kOffSlot);
-        sc.ts = reinterpret_cast<TickState*>(base + kOffTs);
-        group_run(events, count, neuron_count, grouped, segment_start, st, sc);
+        group_run(events, count, neuron_count, grouped, segment_start, st, static_scratch(st), kStaticLayout);
     });
     // a failed call may have left kernels writing the shared scratch and the
     // caller's buffers: they finish before the caller's next call can start
