@@ -241,7 +241,9 @@ int snncuda_sim_read_raster(snncuda_sim* sim, uint64_t first, uint64_t count, ui
  * candidates: blocks of the synapse-event kernel, of the grouping and of the
  * temporal update, and the ticks per captured graph; then it shrinks the wheel-slot capacity to twice the
  * largest per-tick due list seen plus 2^16 events when that saves a quarter
- * or more of it.  The probed ticks are ordinary ticks of the simulation and
+ * or more of it.  Networks small enough to run whole ticks in one kernel,
+ * which has no such shapes, are probed in the kernels that have: the shapes
+ * serve their busy ticks.  The probed ticks are ordinary ticks of the simulation and
  * launch shapes never change results.  Threads per block stay 256: the
  * kernels' shared-memory layouts are built for it, and blocks per SM (the
  * knobs above) are the occupancy lever. */

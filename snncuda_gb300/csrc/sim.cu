@@ -788,7 +788,8 @@ void run_enqueue(snncuda_sim* sim, uint64_t T, snncuda_profile* prof);
 void resident(snncuda_sim* sim);
 
 // Device time per tick of the next `ticks` ticks (they are the simulation's
-// own ticks: launch shapes do not change results).
+// own ticks: launch shapes do not change results) in the kernels of
+// launch_tick: a run handed over by k_small would go on after event b.
 double probe_ms_per_tick(snncuda_sim* sim, uint64_t ticks) {
     cudaEvent_t a = nullptr, b = nullptr;
     check(cudaEventCreate(&a), "event");
@@ -827,6 +828,14 @@ void autotune_impl(snncuda_sim* sim, uint64_t probe_ticks, snncuda_tuning* out) 
     run_complete(sim, true);
     Engine& e = sim->e;
     const uint32_t sms = sim->sms;
+    // k_small reads none of the knobs: the probes of a small network take the
+    // kernels that do (which its busy ticks, or a larger one, run)
+    struct Launched {
+        bool& small;
+        const bool was{small};
+        ~Launched() { small = was; }
+    } launched{sim->small};
+    sim->small = false;
     uint32_t probes = 0;
     double best = probe_ms_per_tick(sim, probe_ticks);
     ++probes;
