@@ -318,6 +318,13 @@ inline uint32_t tick_bucket_shift(uint32_t N, uint32_t sms) {
     while (((static_cast<unsigned long long>(N) + (1ull << s) - 1) >> s) > kMaxTickBuckets) ++s;
     return s;
 }
+inline uint32_t tick_buckets(uint32_t N, uint32_t sms) {
+    const uint32_t s = tick_bucket_shift(N, sms);
+    const uint64_t n = (static_cast<uint64_t>(N) + (1u << s) - 1) >> s;
+    return n > 0 ? static_cast<uint32_t>(n) : 1u;
+}
+// Counting and placing blocks per SM, at most (the rows of Engine::bcnt).
+constexpr uint32_t kBucketBlocksPerSm = 4;
 
 // Grouping entry points: blocks of the counting and placing kernels, at most
 // (fixed, so that the static scratch has a fixed size), and the longest segment

@@ -463,14 +463,14 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sim->device), "device attribute");
     e.bucket_shift = tick_bucket_shift(N, static_cast<uint32_t>(std::max(1, sms)));
     if (e.bucket_shift == 0) throw_fail(SNNCUDA_ERR_UNSUPPORTED, "at most 2^28 neurons");
-    e.nbuckets = static_cast<uint32_t>(std::max<uint64_t>(1, (static_cast<uint64_t>(N) + (1u << e.bucket_shift) - 1) >> e.bucket_shift));
+    e.nbuckets = tick_buckets(N, static_cast<uint32_t>(std::max(1, sms)));
     // counting and placing blocks: two per SM, fewer for small networks (one
     // per 2^18 synapses), whose grids then leave room for other streams'
     // kernels (side-by-side jobs of a server)
     e.grid_bucket = static_cast<uint32_t>(
         std::max<uint64_t>(1, std::min<uint64_t>(sms * 2ull, (static_cast<uint64_t>(sim->S) + (1u << 18) - 1) >> 18)));
     e.scatter_pass_events = kScatterPassEvents;
-    const uint32_t grid_bucket_max = static_cast<uint32_t>(std::max(1, sms * 4));  // the autotuner's largest
+    const uint32_t grid_bucket_max = kBucketBlocksPerSm * static_cast<uint32_t>(std::max(1, sms));  // the autotuner's largest
 
     // ---- tables ----
     uint32_t decay_len = 0;
@@ -846,7 +846,7 @@ void autotune_impl(snncuda_sim* sim, uint64_t probe_ticks, snncuda_tuning* out) 
     };
     std::vector<Knob> knobs = {
         {&e.grid_events, {sms * 4, sms * 8, sms * 16}},
-        {&e.grid_bucket, {sms, sms * 2, sms * 4}},
+        {&e.grid_bucket, {sms, sms * 2, sms * kBucketBlocksPerSm}},
         {&e.scatter_pass_events, {kScatterPassEvents / 2, kScatterPassEvents * 2, 0u}},
         {&e.side_serial, {0u, 1u}},
         {&e.grid_process, {sms * 2, sms * 4, sms * 8}},
@@ -903,7 +903,7 @@ void apply_tuning_impl(snncuda_sim* sim, const snncuda_tuning& t) {
     const uint32_t walk_max = static_cast<uint32_t>(std::max<uint64_t>(1, (static_cast<uint64_t>(sim->N) + 63) / 64));
     auto in = [](uint32_t v, uint32_t lo, uint32_t hi) { return v >= lo && v <= hi; };
     if (!in(t.grid_events, 1, sms * 16) || !in(t.grid_walk, 1, std::max(walk_max, sms * 8)) ||
-        !in(t.grid_bucket, 1, sms * 4) || !in(t.grid_temporal, 1, sms * 8) || !in(t.ticks_per_graph, 1, 64) ||
+        !in(t.grid_bucket, 1, sms * kBucketBlocksPerSm) || !in(t.grid_temporal, 1, sms * 8) || !in(t.ticks_per_graph, 1, 64) ||
         t.side_serial > 1 || (t.block_threads != 0 && t.block_threads != 256))
         throw_fail(SNNCUDA_ERR_INVALID_ARGUMENT, "tuning field outside the autotuner's ranges");
     e.grid_events = t.grid_events;
@@ -2302,10 +2302,19 @@ static uint64_t estimate_bytes_impl(const snncuda_network* net, const snncuda_co
     if (slot_cap == 0) slot_cap = std::min<uint64_t>(1ull << 27, std::max<uint64_t>(1ull << 16, pre_total / 8));
     const uint64_t fire_cap = std::min<uint64_t>(slot_cap, std::max<uint64_t>(65536, 4ull * N));
     const uint64_t lcode = refs_max > 1 ? 2ull * S * refs_max * kMaxExpected : 0;
-    // grouping: bucket counters of up to 512 chunks
-    const uint64_t buckets = (N + 255) / 256 < kMaxBuckets ? (N + 255) / 256 + 1 : kMaxBuckets;
+    // grouping: the counters as create_impl makes them for the current device
+    // (without one, for 152 SMs); 0 buckets: a network it refuses
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        sms = 152;
+    }
+    const uint32_t sm_count = static_cast<uint32_t>(std::max(1, sms));
+    const uint64_t buckets = bucket_shift_for(net->neuron_count) ? tick_buckets(net->neuron_count, sm_count) : 0;
+    const uint64_t counters = buckets * (kBucketBlocksPerSm * sm_count + 3) * 4;
     const uint64_t persistent = 64 * S + 8 * S + 8 * pre_total + neuron_bytes + lcode +
-                                W * slot_cap * 8 + slot_cap * (8 + 16 + 16 + 16 + 4 + 1) + 512 * 4 * buckets +
+                                W * slot_cap * 8 + slot_cap * (8 + 16 + 16 + 16 + 4 + 1) + counters +
                                 fire_cap * 4 + (fire_cap / 8 + 1) * 12 * std::max<uint64_t>(D, 1) +
                                 16 * cfg.raster_capacity + (16u << 20);
     const uint64_t transient = S * (23 + 8 + 12 + 8) + 4 * (has_codes ? net->code_offset_ptr[S] : 0) +
