@@ -183,6 +183,8 @@ struct TickState {
     uint32_t done_scan;       // "last block" counters
     uint32_t done_fire_list;
     uint32_t small_stop;      // not 0: k_small ended before its last tick (launch_small)
+    uint32_t n_parts;         // entries of Engine::parts this tick (reset by k_bcount),
+    uint32_t part_events;     // and events of a part (part_shift)
 };
 
 struct Tables {
@@ -259,6 +261,8 @@ struct Engine {
     uint32_t* btot;                        // [nbuckets] events per bucket (zero between ticks)
     uint32_t* bstart;                      // [nbuckets + 1] first grouped position of each bucket
     uint32_t* bcur;                        // [nbuckets] placement cursor of each bucket
+    uint32_t* parts;                       // [parts_cap] parts of the buckets that k_events shares out to
+                                           // several blocks: bucket | part << 15 (null: grouping calls)
     uint32_t* seg_start;                   // [N + 1] first grouped position of each target
     unsigned long long* grp;               // [slot_cap] due events grouped by target, due order inside
                                            // a target: (payload << 32) | (due index | ext << 31)
@@ -365,6 +369,26 @@ constexpr GroupLayout group_layout(uint32_t count, uint32_t neuron_count) {
     l.bytes = l.ts + (sizeof(TickState) + 255) / 256 * 256;
     return l;
 }
+
+// A bucket with more events than a block's shared memory holds is taken in
+// 2^part_shift parts of equal target ranges (fewer where it has fewer targets),
+// a block for each.  One block took such a bucket from global memory, target
+// after target: a layer of 100 output neurons behind 200,000 others (100 events
+// each in a tick, two buckets) kept one or two SMs busy for 1.8 ms, now 0.096;
+// with every bucket too large (50,000 neurons, 25 events per target) 340 us a
+// tick, now 250.  A part has part_events of the events if they are spread
+// evenly: as few as make kPartBlocks parts (the blocks the GPU holds at once) of
+// all such buckets, but not fewer than a block's threads, nor more than leave
+// room for uneven targets in a block's 1,280 (a part that does not fit goes
+// through global memory).
+constexpr uint32_t kPartEvents = 800, kPartEventsMin = 160, kPartBlocks = 760;
+__host__ __device__ inline uint32_t part_shift(uint32_t events, uint32_t part_events, uint32_t bucket_shift) {
+    uint32_t p = 0;
+    while (p < bucket_shift && (events >> p) > part_events) ++p;
+    return p;
+}
+// Parts of a tick, at most: a bucket has fewer than 2 events / part_events.
+constexpr size_t parts_cap(unsigned long long slot_cap) { return slot_cap / (kPartEvents / 2) + 2 * kPartBlocks; }
 
 constexpr int kExpandFires = 8;          // fires per expansion block (one warp each)
 constexpr uint32_t kMaxClasses = 256;    // distinct delivery delays

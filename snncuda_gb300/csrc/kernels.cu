@@ -673,6 +673,13 @@ __device__ __forceinline__ void code_update(SynB& b, const TargetParam& p, uint3
 // per bucket: no per-target global atomics.
 // ---------------------------------------------------------------------------
 
+// Threads of a k_events block, and the events it holds in shared memory.
+constexpr int kEventThreads = SNNGB_EVENT_THREADS;
+constexpr uint32_t kBlockPerThread = 10;
+constexpr uint32_t kBlockEvents = kBlockPerThread * kEventThreads;
+constexpr uint32_t kPartShift = 15;  // Engine::parts: bucket | part << kPartShift
+static_assert(kMaxTickBuckets <= 1u << kPartShift && kMaxBucketShift + kPartShift <= 32, "Engine::parts");
+
 // Block-wide exclusive scan of a[0 .. n) in shared memory, in place; returns
 // the total.  Every thread takes a run of consecutive entries.
 template <int kBlock>
@@ -887,6 +894,24 @@ __global__ void __launch_bounds__(kBucketThreads) k_bcount(Engine e) {
         e.ts->n_due = n;
         e.ts->post_tick = t;        // the previous tick's k_post has finished
         e.ts->n_fired_targets = 0;
+        e.ts->n_parts = 0;
+    }
+}
+
+// Lists the parts of the buckets that are too large for a block of k_events
+// (`large`: events in those of this thread's buckets [b0, b1)); one block.
+__device__ __noinline__ void list_parts(const Engine& e, uint32_t b0, uint32_t b1, uint32_t large) {
+    uint32_t total;
+    block_excl_scan_t<kBucketThreads>(large, &total);
+    const uint32_t part_events = min(max(total / kPartBlocks, kPartEventsMin), kPartEvents);
+    if (threadIdx.x == 0) e.ts->part_events = part_events;
+    if (large == 0) return;
+    for (uint32_t b = b0; b < b1; ++b) {
+        const uint32_t c = __ldcg(e.btot + b);
+        if (c <= kBlockEvents) continue;
+        const uint32_t parts = 1u << part_shift(c, part_events, e.bucket_shift);
+        const uint32_t at = atomicAdd(&e.ts->n_parts, parts);
+        for (uint32_t k = 0; k < parts; ++k) e.parts[at + k] = b | (k << kPartShift);
     }
 }
 
@@ -901,11 +926,12 @@ __global__ void __launch_bounds__(kBucketThreads) k_bscatter(Engine e) {
         const uint32_t per = (B + blockDim.x - 1) / blockDim.x;
         const uint32_t b0 = threadIdx.x * per < B ? threadIdx.x * per : B;
         const uint32_t b1 = b0 + per < B ? b0 + per : B;
-        uint32_t sum = 0;
+        uint32_t sum = 0, large = 0;
         for (uint32_t b = b0; b < b1; ++b) {
             const uint32_t c = __ldcg(e.btot + b);
             s_pos[b] = c;
             sum += c;
+            if (c > kBlockEvents) large += c;
         }
         uint32_t total;
         uint32_t run = block_excl_scan_t<kBucketThreads>(sum, &total);
@@ -920,7 +946,8 @@ __global__ void __launch_bounds__(kBucketThreads) k_bscatter(Engine e) {
             e.seg_start[e.N] = total;
             count_far_injections(e, e.ts->tick);
         }
-        __syncthreads();
+        const bool list = blockIdx.x == gridDim.x - 1 && e.parts != nullptr;
+        if (__syncthreads_or(list && large > 0)) list_parts(e, b0, b1, large);
     }
     // this chunk's place in each bucket: behind the chunks that reserved
     // before it (the cursors start at zero every tick; k_events clears them)
@@ -1170,6 +1197,8 @@ __device__ __forceinline__ void sort_group(unsigned long long* g, unsigned long 
 // The most events of one target that a block ranks in shared memory (every
 // pair of them is compared).
 constexpr uint32_t kRankEvents = 512;
+
+constexpr uint32_t kNoTarget = 0xFFFFFFFFu;
 
 // Whole block: f(entry) for the entries in[0 .. m), by whole warps (a thread
 // without an entry gets one with target `none`), four loads per thread in
@@ -1455,10 +1484,6 @@ struct BucketParams {
     }
 };
 
-// Threads of a k_events block, and the events it holds in shared memory.
-constexpr int kEventThreads = SNNGB_EVENT_THREADS;
-constexpr uint32_t kBlockPerThread = 10;
-constexpr uint32_t kBlockEvents = kBlockPerThread * kEventThreads;
 constexpr uint32_t kSharedSynapse = 0x8000u;  // beside an event's target: its synapse has other events in the tick
 static_assert(kBlockEvents * sizeof(BucketEntry) >= 256 * (kEventThreads / 32 + 1) * sizeof(uint32_t), "s_radix");
 static_assert((1u << kMaxBucketShift) <= kSharedSynapse, "targets of a bucket");
@@ -1769,31 +1794,34 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
     }
 }
 
-// A bucket with more events than the block's shared memory, or with a long
-// group: grouped in Engine::grp (a counting sort by target, then a warp per
-// target, or the block for a long group, puts its events in due order), its
-// event inputs in Engine::evin.  s_radix: the block's shared memory, otherwise
-// unused on this path.
+// A part with more events than the block's shared memory, or a bucket or part
+// with a long group: grouped in Engine::grp (a counting sort by target, then a
+// warp per target, or the block for a long group, puts its events in due
+// order), its event inputs in Engine::evin.  `in`: the whole bucket's `all`
+// entries, of which those of the targets j0 .. j0 + nw - 1 are meant (`lo`: the
+// first one's position in the tick).  s_radix: the block's shared memory,
+// otherwise unused on this path.
 template <bool kInline>
-__device__ __noinline__ void bucket_in_global(const Engine& e, uint32_t lo, uint32_t m, uint32_t n0, uint32_t nw,
-                                              uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
-                                              int temporal, float* s_wt, Refire* s_refire, uint32_t* s_refires,
+__device__ __noinline__ void bucket_in_global(const Engine& e, const uint4* in, uint32_t all, uint32_t j0,
+                                              uint32_t lo, uint32_t n0, uint32_t nw, uint32_t* s_seg,
+                                              const BucketParams& par, uint32_t t, int stdp, int temporal,
+                                              float* s_wt, Refire* s_refire, uint32_t* s_refires,
                                               uint32_t* s_radix) {
-    const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
     unsigned long long* grp = e.grp + lo;
     // s_seg[j + 1] holds target j's count, then its cursor, then its end
     for (uint32_t j = threadIdx.x; j <= nw; j += blockDim.x) s_seg[j] = 0;
     __syncthreads();
-    for_entries(in, m, nw, [&](const uint4& q) { warp_count(s_seg + 1, q.z < nw ? q.z : nw, nw); });
+    for_entries(in, all, kNoTarget, [&](const uint4& q) { warp_count(s_seg + 1, min(q.z - j0, nw), nw); });
     __syncthreads();
     block_scan_shared<kEventThreads>(s_seg + 1, nw);
-    for_entries(in, m, nw, [&](const uint4& q) {
-        const uint32_t p = warp_count(s_seg + 1, q.z < nw ? q.z : nw, nw);
-        if (q.z < nw) grp[p] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
+    for_entries(in, all, kNoTarget, [&](const uint4& q) {
+        const uint32_t j = min(q.z - j0, nw), p = warp_count(s_seg + 1, j, nw);
+        if (j < nw) grp[p] = (static_cast<unsigned long long>(q.y) << 32) | q.x;
     });
     __syncthreads();
-    // the bucket's own entries are placed: their memory is the merges' scratch
-    unsigned long long* tmp = reinterpret_cast<unsigned long long*>(e.grp_tmp + lo);
+    // the events' inputs are written after the sorts: until then their memory
+    // is the merges' scratch (the entries may still be read for other parts)
+    unsigned long long* tmp = reinterpret_cast<unsigned long long*>(e.evin + lo);
     for (uint32_t j = threadIdx.x >> 5; j < nw; j += blockDim.x / 32) {
         const uint32_t beg = s_seg[j], len = s_seg[j + 1] - beg;
         if (len <= kWarpSortEvents) sort_group(grp + beg, tmp + beg, len);
@@ -1944,7 +1972,9 @@ __device__ __forceinline__ void bucket_events(const Engine& e, const BucketSpace
 }
 
 // Everything a tick does at its targets, a block per bucket of consecutive
-// targets (a bucket's events are one contiguous run of grp_tmp):
+// targets (a bucket's events are one contiguous run of grp_tmp), or per part of
+// a bucket that is too large for a block (part_shift), whose entries the block
+// picks out of the bucket's:
 //
 //   1. the bucket's entries come in with one bulk copy (bounded mbarrier
 //      wait) while the targets' parameters are loaded; every thread holds its
@@ -1988,6 +2018,7 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
     __shared__ Refire s_refire[kEventThreads];      // targets that go on after their first fire
     __shared__ uint32_t s_refires;
     __shared__ uint32_t s_longest;                  // events of the busiest target
+    __shared__ uint32_t s_mine, s_before;           // a part's entries, and the bucket's before them
     const uint32_t width = 1u << e.bucket_shift;
     // the staged entries (16 bytes per event); once they are in registers, the
     // words grouped by target (8) and the words in due order (8); once those
@@ -2009,18 +2040,56 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
     __syncthreads();
     uint32_t parity = 0;
     bool staging = true;  // false after a copy outlived its wait: no more copies
-    for (uint32_t b = blockIdx.x; b < e.nbuckets; b += gridDim.x) {
-        const uint32_t lo = e.bstart[b], m = e.bstart[b + 1] - lo;
-        const uint32_t n0 = b << e.bucket_shift;
-        const uint32_t nw = e.N - n0 < width ? e.N - n0 : width;
+    // the parts of the large buckets, then the buckets
+    const uint32_t parts = e.ts->n_parts, part_events = e.ts->part_events;
+    for (uint32_t w = blockIdx.x; w < parts + e.nbuckets; w += gridDim.x) {
+        const bool part = w < parts;
+        const uint32_t item = part ? e.parts[w] : w - parts, b = item & ((1u << kPartShift) - 1u);
+        uint32_t lo = e.bstart[b], m = e.bstart[b + 1] - lo;
+        uint32_t n0 = b << e.bucket_shift;
+        uint32_t nw = e.N - n0 < width ? e.N - n0 : width;
+        const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
+        const uint32_t all = m;
+        uint32_t j0 = 0;  // the part's first target
+        if (part) {
+            const uint32_t range = ((nw - 1) >> part_shift(all, part_events, e.bucket_shift)) + 1;
+            j0 = (item >> kPartShift) * range;
+            if (j0 >= nw) continue;  // past the last target
+            nw = min(nw - j0, range);
+            n0 += j0;
+            __syncthreads();
+            if (threadIdx.x == 0) s_mine = s_before = 0;
+            __syncthreads();
+            // its entries, as far as they fit, and the number before them
+            uint32_t before = 0;
+            for_entries(in, all, kNoTarget, [&](const uint4& q) {
+                const uint32_t j = q.z - j0, mine = __ballot_sync(0xffffffffu, j < nw);
+                before += q.z < j0;
+                if (mine == 0) return;
+                uint32_t p = 0;
+                if ((threadIdx.x & 31) == 0) p = atomicAdd(&s_mine, __popc(mine));
+                p = __shfl_sync(0xffffffffu, p, 0) + __popc(mine & ((1u << (threadIdx.x & 31)) - 1u));
+                if (j < nw && p < kBlockEvents) s_in[p] = make_uint4(q.x, q.y, j, 0u);
+            });
+            before = __reduce_add_sync(0xffffffffu, before);
+            if ((threadIdx.x & 31) == 0 && before) atomicAdd(&s_before, before);
+            __syncthreads();
+            m = s_mine;
+            lo += s_before;
+        } else {
+            if (threadIdx.x == 0) {  // the bucket's total and cursor start at zero next tick
+                e.btot[b] = 0;
+                e.bcur[b] = 0;
+            }
+            if (m > kBlockEvents) continue;  // its parts do it
+        }
         if (m == 0) {
             if (e.multi_refs)
                 for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) e.seg_start[n0 + j] = lo;
             continue;
         }
-        const uint4* in = reinterpret_cast<const uint4*>(e.grp_tmp) + lo;
         bool small = m <= kBlockEvents;
-        const bool staged = small && staging;
+        const bool staged = !part && staging;
         if (staged && threadIdx.x == 0) bulk_load(s_raw, in, m * static_cast<uint32_t>(sizeof(BucketEntry)), &s_bar);
         const BucketParams par{s_par, e.nparam + n0, keep_params};
         if (keep_params)
@@ -2030,10 +2099,6 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
             prefetch_l2(e.ntp + n0 + j);
         }
         for (uint32_t j = threadIdx.x; j <= nw; j += kEventThreads) s_seg[j] = 0;
-        if (threadIdx.x == 0) {  // the bucket's total and cursor start at zero next tick
-            e.btot[b] = 0;
-            e.bcur[b] = 0;
-        }
         bool ready = true;
         if (staged && threadIdx.x == 0) ready = mbar_wait(&s_bar, parity, e.stage_wait_ns);
         ready = __syncthreads_and(ready);
@@ -2051,7 +2116,7 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
             }
             parity ^= 1u;
         }
-        if (small && !(staged && ready)) {  // no copy: the entries come in directly
+        if (!part && !(staged && ready)) {  // no copy: the entries come in directly
             for (uint32_t i = threadIdx.x; i < m; i += kEventThreads) s_in[i] = in[i];
             __syncthreads();
         }
@@ -2112,7 +2177,7 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
             }
         }
         if (!small) {
-            bucket_in_global<kInline>(e, lo, m, n0, nw, s_seg, par, t, stdp, temporal, &s_wt[0][0], s_refire,
+            bucket_in_global<kInline>(e, in, all, j0, lo, n0, nw, s_seg, par, t, stdp, temporal, &s_wt[0][0], s_refire,
                                       &s_refires, reinterpret_cast<uint32_t*>(s_raw));
             __syncthreads();
             if (m > kBlockEvents) {
@@ -3293,7 +3358,7 @@ void launch_tick(const Engine& e, const TickStreams& s, cudaEvent_t* marks) {
     mark(false); launch_main(k_bscatter, e.grid_bucket, kBucketThreads, bucket_smem(e), stream, dep, e); mark(true);
     mark(false);
     launch_main(e.inline_codes ? k_events<true> : k_events<false>,
-                e.grid_events < e.nbuckets ? e.grid_events : e.nbuckets, kEventThreads,
+                std::min(e.grid_events, std::max(e.nbuckets, wide)), kEventThreads,
                 events_smem(e.bucket_shift), stream, dep, e);
     mark(true);
     if (e.side_serial) {

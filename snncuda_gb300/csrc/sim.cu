@@ -494,6 +494,7 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     e.btot = salloc<uint32_t>(sim, e.nbuckets, BufKind::kZero);
     e.bstart = salloc<uint32_t>(sim, static_cast<size_t>(e.nbuckets) + 1, BufKind::kScratch);
     e.bcur = salloc<uint32_t>(sim, e.nbuckets, BufKind::kZero);
+    e.parts = salloc<uint32_t>(sim, parts_cap(slot_cap), BufKind::kScratch);
     e.grp = salloc<unsigned long long>(sim, slot_cap, BufKind::kScratch);
     e.grp_tmp = salloc<BucketEntry>(sim, slot_cap, BufKind::kScratch);
     e.evin = salloc<EvIn>(sim, slot_cap, BufKind::kScratch);
@@ -596,7 +597,7 @@ void remap_engine(Engine& e, const DeviceBuffers& from, const DeviceBuffers& to)
     };
     fix(e.in_ptr); fix(e.nparam); fix(e.nrec); fix(e.ntp); fix(e.cand); fix(e.refmeta); fix(e.ring); fix(e.syn);
     fix(e.lcode); fix(e.pre_base); fix(e.pre_off); fix(e.pre_ev); fix(e.cls_delta); fix(e.wheel);
-    fix(e.slot_count); fix(e.bcnt); fix(e.btot); fix(e.bstart); fix(e.bcur); fix(e.seg_start); fix(e.grp);
+    fix(e.slot_count); fix(e.bcnt); fix(e.btot); fix(e.bstart); fix(e.bcur); fix(e.parts); fix(e.seg_start); fix(e.grp);
     fix(e.grp_tmp); fix(e.evin); fix(e.ev_a0); fix(e.fire_bits); fix(e.fire_at);
     fix(e.fire_tile); fix(e.fire_list); fix(e.fired_tgt); fix(e.fired_cnt); fix(e.xsum); fix(e.xdst);
     fix(e.xdst_ok); fix(e.raster); fix(e.ts); fix(e.tab.decay); fix(e.tab.ltp); fix(e.tab.ltd);
@@ -766,6 +767,7 @@ void resize_slots(snncuda_sim* sim, uint64_t cap) {
     };
     sim->drop_graphs();
     realloc_buf(e.wheel, static_cast<size_t>(e.W) * cap * 8);
+    realloc_buf(e.parts, parts_cap(cap) * 4);
     realloc_buf(e.grp, cap * 8);
     realloc_buf(e.grp_tmp, cap * sizeof(BucketEntry));
     realloc_buf(e.evin, cap * sizeof(EvIn));
@@ -2314,7 +2316,7 @@ static uint64_t estimate_bytes_impl(const snncuda_network* net, const snncuda_co
     const uint64_t buckets = bucket_shift_for(net->neuron_count) ? tick_buckets(net->neuron_count, sm_count) : 0;
     const uint64_t counters = buckets * (kBucketBlocksPerSm * sm_count + 3) * 4;
     const uint64_t persistent = 64 * S + 8 * S + 8 * pre_total + neuron_bytes + lcode +
-                                W * slot_cap * 8 + slot_cap * (8 + 16 + 16 + 16 + 4 + 1) + counters +
+                                W * slot_cap * 8 + slot_cap * (8 + 16 + 16 + 16 + 4 + 1) + 4 * parts_cap(slot_cap) + counters +
                                 fire_cap * 4 + (fire_cap / 8 + 1) * 12 * std::max<uint64_t>(D, 1) +
                                 16 * cfg.raster_capacity + (16u << 20);
     const uint64_t transient = S * (23 + 8 + 12 + 8) + 4 * (has_codes ? net->code_offset_ptr[S] : 0) +
