@@ -1475,12 +1475,42 @@ __device__ __forceinline__ TargetParam load_param(const NeuronParam* p) {
     return TargetParam{__uint_as_float(q.x), q.y, __uint_as_float(q.z), q.w};
 }
 
+// The blocks of k_small share out the neurons by runs of kSmallChunk: every block
+// has one of eight neighbouring runs, at a place that changes with the digits of
+// the run's number.  Neighbours, which are often busy together (an output layer),
+// so go to different blocks, whatever the distance of such groups; one by one,
+// the records' reads would take twice the lines (38 us a tick of 5,000 events
+// with runs of 8 or 32, 45 with 1).
+constexpr uint32_t kSmallChunk = 8;
+static_assert(kSmallBlocks == 8 && kSmallBlocks * kSmallTargets <= 1u << 15, "the digits summed up");
+
+__device__ __forceinline__ uint32_t small_block(uint32_t n) {
+    const uint32_t run = n / kSmallChunk;
+    return (run + (run >> 3) + (run >> 6) + (run >> 9)) % kSmallBlocks;
+}
+// A neuron's place among its block's, and the neuron at place j of block c.
+__device__ __forceinline__ uint32_t small_place(uint32_t n) {
+    return n / (kSmallChunk * kSmallBlocks) * kSmallChunk + n % kSmallChunk;
+}
+__device__ __forceinline__ uint32_t small_neuron(uint32_t c, uint32_t j) {
+    const uint32_t high = j / kSmallChunk, run = high * kSmallBlocks + (c - high - (high >> 3) - (high >> 6)) % kSmallBlocks;
+    return run * kSmallChunk + j % kSmallChunk;
+}
+
+// Target j of a block: neuron first + j, or (kSmall) k_small's.
+template <bool kSmall>
+__device__ __forceinline__ uint32_t neuron_of(uint32_t first, uint32_t j) {
+    return kSmall ? small_neuron(first, j) : first + j;
+}
+
+template <bool kSmall>
 struct BucketParams {
     const TargetParam* shared;
-    const NeuronParam* global;  // the bucket's first target
+    const NeuronParam* global;
+    uint32_t first;  // (neuron_of)
     bool in_shared;
     __device__ __forceinline__ TargetParam operator[](uint32_t j) const {
-        return in_shared ? shared[j] : load_param(global + j);
+        return in_shared ? shared[j] : load_param(global + neuron_of<kSmall>(first, j));
     }
 };
 
@@ -1747,17 +1777,20 @@ __device__ __forceinline__ void temporal_target(const Engine& e, uint32_t n, uin
 // block's warps (one warp did its own 32 targets' one after the other: up to
 // 20 us with three or four of them, where the walk itself takes 4; sharing them
 // took the kernel from 36 to 32 us at 250,000 events, 197 to 187 at 2.5 M).
-template <int kT, typename Events, typename Fires>
+// The targets: the block's nw, or of them the nw in `list` (if not null).
+template <int kT, bool kSmall, typename Events, typename Fires>
 __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, uint32_t lo, uint32_t n0, uint32_t nw,
-                                            const uint32_t* s_seg, const BucketParams& par, uint32_t t, int stdp,
-                                            float* s_wt, Refire* s_refire, uint32_t* s_refires, const Fires& out) {
+                                            const uint16_t* list, const uint32_t* s_seg,
+                                            const BucketParams<kSmall>& par, uint32_t t, int stdp, float* s_wt,
+                                            Refire* s_refire, uint32_t* s_refires, const Fires& out) {
     for (uint32_t j0 = 0; j0 < nw; j0 += kT) {
         if (threadIdx.x == 0) *s_refires = 0;
         __syncthreads();
-        const uint32_t j = j0 + threadIdx.x;
-        const uint32_t beg = j < nw ? s_seg[j] : 0u, len = j < nw ? s_seg[j + 1] - beg : 0u;
+        const uint32_t at = j0 + threadIdx.x, j = at < nw && list ? list[at] : at;
+        const uint32_t n = neuron_of<kSmall>(n0, j);
+        const uint32_t beg = at < nw ? s_seg[j] : 0u, len = at < nw ? s_seg[j + 1] - beg : 0u;
         if (len > 0) {
-            NeuronRec* rec = e.nrec + n0 + j;
+            NeuronRec* rec = e.nrec + n;
             const float threshold = par[j].threshold;
             NState s;
             load_physics(s, rec);
@@ -1765,11 +1798,11 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
             for (uint32_t i = 0; i < len; ++i) {
                 const uint32_t bits = ev.bits_of(beg + i);
                 if (process_input(s, threshold, bits & 3u, (bits >> 2) & 3u, ev.weight_of(beg + i), t)) {
-                    out.fire(n0 + j, ev.at(beg + i).due);
+                    out.fire(n, ev.at(beg + i).due);
                     if (i + 1 < len) {
                         s_refire[atomicAdd(s_refires, 1u)] = Refire{j, i + 1};
                     } else {
-                        out.target(n0 + j, 1);
+                        out.target(n, 1);
                     }
                     break;
                 }
@@ -1780,7 +1813,7 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
         const uint32_t refires = *s_refires, warp = threadIdx.x >> 5;
         for (uint32_t k = warp; k < refires; k += kT / 32) {
             const Refire f = s_refire[k];
-            const uint32_t n = n0 + f.j, first = s_seg[f.j];
+            const uint32_t n = neuron_of<kSmall>(n0, f.j), first = s_seg[f.j];
             NState s;
             load_physics(s, e.nrec + n);
             const uint32_t fires = walk_after_fire(e, s, par[f.j].threshold, n, first, s_seg[f.j + 1] - first, f.next, t,
@@ -1804,7 +1837,7 @@ __device__ __forceinline__ void walk_bucket(const Engine& e, const Events& ev, u
 template <bool kInline>
 __device__ __noinline__ void bucket_in_global(const Engine& e, const uint4* in, uint32_t all, uint32_t j0,
                                               uint32_t lo, uint32_t n0, uint32_t nw, uint32_t* s_seg,
-                                              const BucketParams& par, uint32_t t, int stdp, int temporal,
+                                              const BucketParams<false>& par, uint32_t t, int stdp, int temporal,
                                               float* s_wt, Refire* s_refire, uint32_t* s_refires,
                                               uint32_t* s_radix) {
     unsigned long long* grp = e.grp + lo;
@@ -1858,7 +1891,8 @@ __device__ __noinline__ void bucket_in_global(const Engine& e, const uint4* in, 
         if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
     }
     __syncthreads();
-    walk_bucket<kEventThreads>(e, ev, lo, n0, nw, s_seg, par, t, stdp, s_wt, s_refire, s_refires, EngineFires{e});
+    walk_bucket<kEventThreads>(e, ev, lo, n0, nw, nullptr, s_seg, par, t, stdp, s_wt, s_refire, s_refires,
+                               EngineFires{e});
 }
 
 // Shared memory of a bucket's events besides SharedEvents.
@@ -1872,6 +1906,7 @@ struct BucketSpace {
     uint32_t *repeats, *next, *refires;  // counters (the first two zero)
     uint16_t* multi;                     // kAlone: targets with several reference patterns,
     uint32_t* multis;                    // and their number (zero)
+    const uint16_t* touched;             // targets with events (null: all are looked at)
 };
 
 template <int kGroup>
@@ -1879,15 +1914,19 @@ __device__ __forceinline__ void temporal_group(const Engine& e, uint32_t n, uint
 
 // Steps 2 (from the grouped words on) to 4 of k_events for one bucket.  kAlone:
 // the block is not k_events': the temporal patterns of targets with several
-// reference patterns are done here too.
+// reference patterns are done here too.  The targets: the nw in b.touched, or all
+// nw.
 template <bool kInline, int kT, bool kAlone, typename Fires>
 __device__ __forceinline__ void bucket_events(const Engine& e, const BucketSpace& b, const SharedEvents& ev,
                                               uint32_t total, uint32_t lo, uint32_t n0, uint32_t nw,
-                                              const BucketParams& par, uint32_t t, int stdp, int temporal,
+                                              const BucketParams<kAlone>& par, uint32_t t, int stdp, int temporal,
                                               const Fires& out) {
+    auto target = [&](uint32_t i) { return kAlone && b.touched ? b.touched[i] : i; };
     if (kAlone && e.multi_refs)
-        for (uint32_t j = threadIdx.x; j < nw; j += kT)
+        for (uint32_t i = threadIdx.x; i < nw; i += kT) {
+            const uint32_t j = target(i);
             if (b.seg[j + 2] > b.seg[j + 1] && par[j].max_refs != 1) b.multi[atomicAdd(b.multis, 1u)] = static_cast<uint16_t>(j);
+        }
     // each event's rank in due order among its target's events
     // (by position: the lanes of a warp read the same or the next
     // group's words); of the synapses with several events, the
@@ -1919,9 +1958,9 @@ __device__ __forceinline__ void bucket_events(const Engine& e, const BucketSpace
     // targets at a time from the first warps, the synapses with
     // several events, then all other events.
     const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t j = threadIdx.x; j < nw; j += kT) {
-        const uint32_t k = b.seg[j + 2] - b.seg[j + 1];
-        if (k > 0 && par[j].max_refs == 1) temporal_target(e, n0 + j, k, t, temporal);
+    for (uint32_t i = threadIdx.x; i < nw; i += kT) {
+        const uint32_t j = target(i), k = b.seg[j + 2] - b.seg[j + 1];
+        if (k > 0 && par[j].max_refs == 1) temporal_target(e, neuron_of<kAlone>(n0, j), k, t, temporal);
     }
     __syncwarp();
     constexpr uint32_t kGroup = 8;  // lanes per target with several reference patterns
@@ -1936,7 +1975,7 @@ __device__ __forceinline__ void bucket_events(const Engine& e, const BucketSpace
                 const uint32_t k = (task * 32 + lane) / kGroup;
                 if (k < multis) {
                     const uint32_t j = b.multi[k];
-                    temporal_group<kGroup>(e, n0 + j, b.seg[j + 2] - b.seg[j + 1], t, temporal);
+                    temporal_group<kGroup>(e, neuron_of<kAlone>(n0, j), b.seg[j + 2] - b.seg[j + 1], t, temporal);
                 }
                 __syncwarp();
                 continue;
@@ -1963,12 +2002,13 @@ __device__ __forceinline__ void bucket_events(const Engine& e, const BucketSpace
         }
         if (run) {
             const uint32_t j = b.tgt[i] & ~kSharedSynapse;
-            synapse_events<kInline>(e, ev, lo, i, last, par[j], n0 + j, t, stdp, temporal);
+            synapse_events<kInline>(e, ev, lo, i, last, par[j], neuron_of<kAlone>(n0, j), t, stdp, temporal);
         }
         __syncwarp();
     }
     __syncthreads();
-    walk_bucket<kT>(e, ev, lo, n0, nw, b.seg + 1, par, t, stdp, b.wt, b.refire, b.refires, out);
+    walk_bucket<kT>(e, ev, lo, n0, nw, kAlone ? b.touched : nullptr, b.seg + 1, par, t, stdp, b.wt, b.refire, b.refires,
+                    out);
 }
 
 // Everything a tick does at its targets, a block per bucket of consecutive
@@ -2032,7 +2072,7 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
     const bool keep_params = width <= kSharedParams;
     uint32_t* s_seg = reinterpret_cast<uint32_t*>(s_par + (keep_params ? width : 0u));  // [width + 2]
     const BucketSpace space{s_word, s_tgt, s_list, s_seg, &s_wt[0][0], s_refire, &s_repeats, &s_next, &s_refires,
-                            nullptr, nullptr};
+                            nullptr, nullptr, nullptr};
     const uint32_t t = e.ts->tick;
     const int stdp = e.ts->stdp_enabled;
     const int temporal = e.ts->temporal_enabled;
@@ -2091,7 +2131,7 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
         bool small = m <= kBlockEvents;
         const bool staged = !part && staging;
         if (staged && threadIdx.x == 0) bulk_load(s_raw, in, m * static_cast<uint32_t>(sizeof(BucketEntry)), &s_bar);
-        const BucketParams par{s_par, e.nparam + n0, keep_params};
+        const BucketParams<false> par{s_par, e.nparam, n0, keep_params};
         if (keep_params)
             for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) s_par[j] = load_param(e.nparam + n0 + j);
         for (uint32_t j = threadIdx.x; j < nw; j += kEventThreads) {
@@ -2671,6 +2711,12 @@ constexpr size_t kSmallOffList = kSmallOffTgt + kSmallEvents * sizeof(uint16_t);
 constexpr size_t kSmallOffSeg = kSmallOffList + kSmallEvents * sizeof(uint16_t);
 constexpr size_t kSmallOffSlot = kSmallOffSeg + (kSmallTargets + 2) * sizeof(uint32_t);
 constexpr size_t kSmallSmem = kSmallOffSlot + kSmallSlots * sizeof(uint32_t);
+// The list of the targets with events takes the end of the words' memory, where
+// a block has no more than this many events (8 KB more shared memory, which L1
+// then lacks, took a tick of 7,000 events from 41 to 44 us).
+constexpr size_t kSmallOffTouched = kSmallOffTgt - kSmallTargets * sizeof(uint16_t);
+constexpr uint32_t kSmallListed = (kSmallOffTouched - kSmallA) / sizeof(unsigned long long);
+static_assert(kSmallEvents * (sizeof(float) + 1) <= kSmallOffTouched - kSmallA, "w and bits before the list");
 static_assert((kSmallEvents + kSmallPlaces) * sizeof(uint32_t) <= kSmallA, "fires and places");
 static_assert(kSmallTargets <= kSmallEvents / 2, "fired targets in the lists' place, targets in their second half");
 static_assert(kSmallTargets < kSharedSynapse, "targets of a block");
@@ -2686,16 +2732,15 @@ __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async;
 struct SmallFires {
     uint2* fires;        // (due position, neuron) in global memory
     uint32_t* targets;   // target within the block << 16 | fires
-    uint32_t n0;
     uint32_t *n_fires, *n_targets;
     __device__ __forceinline__ void fire(uint32_t n, uint32_t due) const { fires[atomicAdd(n_fires, 1u)] = make_uint2(due, n); }
     __device__ __forceinline__ void target(uint32_t n, uint32_t f) const {
-        targets[atomicAdd(n_targets, 1u)] = (n - n0) << 16 | f;
+        targets[atomicAdd(n_targets, 1u)] = small_place(n) << 16 | f;
     }
 };
 
 // Ticks ts->tick .. end-1 of a small network, kSmallBlocks blocks in one
-// cluster, each with an equal share of the targets.  Per tick a block reads
+// cluster, each with an eighth of the targets (small_block).  Per tick a block reads
 // the whole due list into shared memory and groups the events of its own
 // targets (no pass over the other blocks' data), does what k_events does with
 // them, and the post-spike STDP of its fired targets; the blocks exchange
@@ -2721,7 +2766,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     __shared__ __align__(8) unsigned long long s_bar;
     __shared__ float s_wt[kSmallThreads / 32][32];
     __shared__ Refire s_refire[kSmallThreads];
-    __shared__ uint32_t s_refires, s_repeats, s_next, s_fires, s_fired, s_multis;
+    __shared__ uint32_t s_refires, s_repeats, s_next, s_fires, s_fired, s_multis, s_touches;
     __shared__ uint32_t s_part[kSmallThreads], s_sum[kMaxClasses], s_start[kMaxClasses], s_slot_of[kMaxClasses];
     __shared__ uint32_t s_done[kMaxClasses];
     __shared__ uint32_t s_bits[kSmallEvents / 32], s_before[kSmallEvents / 32], s_count[kSmallBlocks];
@@ -2732,6 +2777,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     uint32_t* s_end = reinterpret_cast<uint32_t*>(s_raw + kSmallOffSeg);  // s_end[j], s_end[j + 1]: first and end of target j
     uint32_t* s_seg = s_end + 1;
     uint32_t* s_slot = reinterpret_cast<uint32_t*>(s_raw + kSmallOffSlot);  // events in each wheel slot
+    uint16_t* s_touched = reinterpret_cast<uint16_t*>(s_raw + kSmallOffTouched);  // targets with events
     uint32_t* s_fire = reinterpret_cast<uint32_t*>(s_raw);                  // firing neurons in due order
     uint32_t* s_place = s_fire + kSmallEvents;
     const uint32_t c = blockIdx.x;
@@ -2746,12 +2792,13 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     const int temporal = e.ts->temporal_enabled;
     unsigned long long raster = e.ts->raster_count;
     const uint32_t D = e.D;
-    const uint32_t per = (e.N + kSmallBlocks - 1) / kSmallBlocks;
-    const uint32_t n0 = min(e.N, c * per), nw = min(e.N, n0 + per) - n0;
-    const BucketParams par{nullptr, e.nparam + n0, false};
+    // its targets: whole runs, then what there is of the last one
+    const uint32_t whole = e.N / (kSmallChunk * kSmallBlocks) * kSmallChunk, last = small_neuron(c, whole);
+    const uint32_t nw = whole + (e.N > last ? min(e.N - last, kSmallChunk) : 0u);
+    const BucketParams<true> par{nullptr, e.nparam, c, false};
     const SharedEvents ev{s_due, reinterpret_cast<float*>(s_word), reinterpret_cast<uint8_t*>(s_word) + 4 * kSmallEvents};
     uint2* all_fires = reinterpret_cast<uint2*>(e.evin);  // [block][limit]
-    const SmallFires out{all_fires + c * limit, reinterpret_cast<uint32_t*>(s_list), n0, &s_fires, &s_fired};
+    const SmallFires out{all_fires + c * limit, reinterpret_cast<uint32_t*>(s_list), &s_fires, &s_fired};
     // lanes per share of the fires: a lane per class
     uint32_t span = 1;
     while (span < D) span <<= 1;
@@ -2785,7 +2832,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
                 }
             }
         }
-        if (threadIdx.x == 0) s_fires = s_fired = s_repeats = s_next = s_multis = 0;
+        if (threadIdx.x == 0) s_fires = s_fired = s_repeats = s_next = s_multis = s_touches = 0;
         if (n > 0) {
             const unsigned long long* due = e.wheel + static_cast<size_t>(slot) * e.slot_cap;
             bool ready = true;
@@ -2823,26 +2870,41 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
             uint32_t ext = 0;
             for (uint32_t i = threadIdx.x; i < n; i += kSmallThreads) {
                 const uint32_t lo = static_cast<uint32_t>(s_due[i]);
+                const uint32_t tgt = lo & ~kExternalBit;
                 ext += lo >> 31;
-                const uint32_t j = (lo & ~kExternalBit) - n0;
-                if (j < nw) atomicAdd(&s_seg[j], 1u);
+                if (small_block(tgt) == c) atomicAdd(&s_seg[small_place(tgt)], 1u);
             }
             if (c == 0) external += __reduce_add_sync(0xffffffffu, ext);  // (per warp; lane 0 reports)
             __syncthreads();
             uint32_t busy = 0, longest = 0;
-            for (uint32_t j = threadIdx.x; j < nw; j += kSmallThreads) {
-                busy += s_seg[j] != 0;
-                longest = max(longest, s_seg[j]);
+            if (nw <= kSmallThreads) {
+                longest = threadIdx.x < nw ? s_seg[threadIdx.x] : 0u;
+                busy = longest != 0;
+            } else {
+                // a thread has several targets: those with events are listed
+                // (of 4,096 mostly a few hundred)
+                const uint32_t lane = threadIdx.x & 31;
+                for (uint32_t j0 = threadIdx.x - lane; j0 < nw; j0 += kSmallThreads) {
+                    const uint32_t j = j0 + lane, k = j < nw ? s_seg[j] : 0u;
+                    const uint32_t some = __ballot_sync(0xffffffffu, k > 0);
+                    longest = max(longest, k);
+                    busy += k > 0;
+                    uint32_t p = 0;
+                    if (lane == 0 && some) p = atomicAdd(&s_touches, __popc(some));
+                    p = __shfl_sync(0xffffffffu, p, 0) + __popc(some & ((1u << lane) - 1u));
+                    if (k > 0) s_touched[p] = static_cast<uint16_t>(j);
+                }
             }
             busy = __reduce_add_sync(0xffffffffu, busy);
             if ((threadIdx.x & 31) == 0 && busy) atomicAdd(&e.ts->touched_total, static_cast<unsigned long long>(busy));
             if (longest > kRankEvents) atomicMax(&e.ts->small_stop, t + 1);
             __syncthreads();
             const uint32_t total = block_scan_shared<kSmallThreads>(s_seg, nw);
+            const bool listed = nw > kSmallThreads && total <= kSmallListed;
             for (uint32_t i = threadIdx.x; i < n; i += kSmallThreads) {
                 const unsigned long long v = s_due[i];
-                const uint32_t lo = static_cast<uint32_t>(v), j = (lo & ~kExternalBit) - n0;
-                if (j >= nw) continue;
+                const uint32_t lo = static_cast<uint32_t>(v), tgt = lo & ~kExternalBit, j = small_place(tgt);
+                if (small_block(tgt) != c) continue;
                 const uint32_t p = atomicAdd(&s_seg[j], 1u);  // ends at the target's end
                 s_word[p] = (v & 0xFFFFFFFF00000000ull) | (i << 1) | (lo >> 31);
                 s_tgt[p] = static_cast<uint16_t>(j);
@@ -2851,9 +2913,9 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
             if (total > 0) {
                 const BucketSpace space{s_word,      s_tgt,     s_list,     s_end - 1,  &s_wt[0][0],
                                         s_refire,    &s_repeats, &s_next,   &s_refires, s_list + kSmallEvents / 2,
-                                        &s_multis};
-                bucket_events<kInline, kSmallThreads, true>(e, space, ev, total, c * limit, n0, nw, par, t, stdp, temporal,
-                                                            out);
+                                        &s_multis, listed ? s_touched : nullptr};
+                bucket_events<kInline, kSmallThreads, true>(e, space, ev, total, c * limit, c, listed ? s_touches : nw, par,
+                                                            t, stdp, temporal, out);
             }
         }
         __syncthreads();
@@ -2864,7 +2926,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
         // (a warp per target when there are as many as warps, else the block)
         const bool by_warp = s_fired >= kSmallThreads / 32;
         for (uint32_t k = by_warp ? threadIdx.x >> 5 : 0u; k < s_fired; k += by_warp ? kSmallThreads / 32 : 1u) {
-            const uint32_t f = out.targets[k], tgt = n0 + (f >> 16);
+            const uint32_t f = out.targets[k], tgt = small_neuron(c, f >> 16);
             const unsigned long long last = e.in_ptr[tgt + 1];
             for (unsigned long long tm = e.in_ptr[tgt] + (by_warp ? threadIdx.x & 31 : threadIdx.x); tm < last;
                  tm += by_warp ? 32 : kSmallThreads) {
