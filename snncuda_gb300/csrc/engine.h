@@ -185,6 +185,7 @@ struct TickState {
     uint32_t small_stop;      // not 0: k_small ended before its last tick (launch_small)
     uint32_t n_parts;         // entries of Engine::parts this tick (reset by k_bcount),
     uint32_t part_events;     // and events of a part (part_shift)
+    uint32_t small_debt[8];   // per block of k_small: ns that its ticks have lost (kSmallDebt)
 };
 
 struct Tables {
@@ -409,11 +410,28 @@ const char* kernel_name(int index);
 // Ticks ts->tick .. end-1 of a small network (small_network) in one kernel; it
 // stops before a tick it does not take (ts->small_stop, until which the
 // launches behind it return at once): one with more than `limit` events due
-// (small_limit).
+// (small_limit), or any after its ticks have lost more than kSmallDebt.
 constexpr uint32_t kSmallBlocks = 8;
 constexpr uint32_t kSmallTargets = 4096;  // per block
 constexpr uint32_t kSmallEvents = 8192;
 constexpr uint32_t kSmallSlots = 1024;
+// What eight SMs take longer for than the launched kernels, which have them all,
+// in ns: a row of post-spike STDP of one block (512 at a time, about 1 us), an
+// event of the fire with the most (one warp copies them: 32 in 0.5 us), a fire
+// and delay class (190 fires x 250 classes: 54 us, launched 46), an event above
+// kSmallEven where the blocks have more targets than threads (4,000 events on
+// 8,000 and 16,000 neurons 31 and 32 us, launched 33 and 32; 7,000 43 and 44,
+// launched 38 and 35).  A quiet tick gains kSmallGain (1,000 neurons, 1,000
+// events: 22 us, launched 30) less N / 8 and, as the launched kernels count the
+// fires by class, kSmallClassGain per class more.  Once a block's ticks have lost
+// kSmallDebt more than they gained, the launched kernels take over: rare heavy
+// ticks do not do that, a layer of 100 output neurons with 30,000 inputs each that
+// fires all the time (4,700 us a tick here, 126 launched) does in a few.
+constexpr uint32_t kSmallRow = 2, kSmallCopy = 16, kSmallClass10 = 4, kSmallEvent = 3, kSmallEven = 4096;
+constexpr uint32_t kSmallGain = 8000, kSmallClassGain = 32;
+constexpr uint32_t kSmallDebt = 1u << 20;
+static_assert(sizeof(TickState::small_debt) == kSmallBlocks * sizeof(uint32_t), "a block's debt");
+static_assert(kSmallGain >= kSmallBlocks * kSmallTargets / 8, "a gain for every size");
 inline uint32_t small_limit(const Engine& e) {
     const unsigned long long share = e.slot_cap / kSmallBlocks;  // a block's part of the per-event scratch
     return static_cast<uint32_t>(share < kSmallEvents ? share : kSmallEvents);

@@ -2756,9 +2756,11 @@ struct SmallFires {
 // and walk, 1.4 post-spike STDP, 4.5 fires and their events, 1.5 barriers.  A
 // burst of 27,648 relayed events over 7 ticks: 42 -> 35 us a tick.  Eight blocks (a portable cluster) of 512
 // threads; a tick with more than `limit` events due (kSmallEvents, or an
-// eighth of a wheel slot: the scratch is shared out), or a target with more
-// than kRankEvents of them, ends the run of this kernel (ts->small_stop: the
-// first tick left to the other kernels): there the whole GPU is quicker.
+// eighth of a wheel slot: the scratch is shared out), a target with more than
+// kRankEvents of them, or ticks that lost too much (kSmallDebt) end the run of
+// this kernel (ts->small_stop: the first tick left to the other kernels): there
+// the whole GPU is quicker.  The first block to set small_stop decides for all (a
+// later and larger value would be seen by some blocks only).
 template <bool kInline>
 __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads, 1)
     k_small(const __grid_constant__ Engine e, uint32_t end, uint32_t limit) {
@@ -2766,7 +2768,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     __shared__ __align__(8) unsigned long long s_bar;
     __shared__ float s_wt[kSmallThreads / 32][32];
     __shared__ Refire s_refire[kSmallThreads];
-    __shared__ uint32_t s_refires, s_repeats, s_next, s_fires, s_fired, s_multis, s_touches;
+    __shared__ uint32_t s_refires, s_repeats, s_next, s_fires, s_fired, s_multis, s_touches, s_rows, s_widest;
     __shared__ uint32_t s_part[kSmallThreads], s_sum[kMaxClasses], s_start[kMaxClasses], s_slot_of[kMaxClasses];
     __shared__ uint32_t s_done[kMaxClasses];
     __shared__ uint32_t s_bits[kSmallEvents / 32], s_before[kSmallEvents / 32], s_count[kSmallBlocks];
@@ -2810,6 +2812,8 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     unsigned long long delivered = 0, external = 0, fired = 0, most = 0;
     uint32_t parity = 0;
     bool staging = true;
+    uint32_t debt = threadIdx.x == 0 ? e.ts->small_debt[c] : 0u;  // (thread 0 keeps it)
+    const uint32_t gain = kSmallGain - e.N / 8 + kSmallClassGain * D;
     __syncthreads();
     for (;;) {
         const uint32_t slot = t & e.wmask, n = s_slot[slot];
@@ -2832,7 +2836,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
                 }
             }
         }
-        if (threadIdx.x == 0) s_fires = s_fired = s_repeats = s_next = s_multis = s_touches = 0;
+        if (threadIdx.x == 0) s_fires = s_fired = s_repeats = s_next = s_multis = s_touches = s_rows = s_widest = 0;
         if (n > 0) {
             const unsigned long long* due = e.wheel + static_cast<size_t>(slot) * e.slot_cap;
             bool ready = true;
@@ -2897,7 +2901,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
             }
             busy = __reduce_add_sync(0xffffffffu, busy);
             if ((threadIdx.x & 31) == 0 && busy) atomicAdd(&e.ts->touched_total, static_cast<unsigned long long>(busy));
-            if (longest > kRankEvents) atomicMax(&e.ts->small_stop, t + 1);
+            if (longest > kRankEvents) atomicCAS(&e.ts->small_stop, 0u, t + 1);
             __syncthreads();
             const uint32_t total = block_scan_shared<kSmallThreads>(s_seg, nw);
             const bool listed = nw > kSmallThreads && total <= kSmallListed;
@@ -2927,9 +2931,10 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
         const bool by_warp = s_fired >= kSmallThreads / 32;
         for (uint32_t k = by_warp ? threadIdx.x >> 5 : 0u; k < s_fired; k += by_warp ? kSmallThreads / 32 : 1u) {
             const uint32_t f = out.targets[k], tgt = small_neuron(c, f >> 16);
-            const unsigned long long last = e.in_ptr[tgt + 1];
-            for (unsigned long long tm = e.in_ptr[tgt] + (by_warp ? threadIdx.x & 31 : threadIdx.x); tm < last;
-                 tm += by_warp ? 32 : kSmallThreads) {
+            const unsigned long long first = e.in_ptr[tgt], last = e.in_ptr[tgt + 1];
+            const uint32_t me = by_warp ? threadIdx.x & 31 : threadIdx.x;
+            if (me == 0) atomicAdd(&s_rows, static_cast<uint32_t>(min(last - first, 1ull << 17)));
+            for (unsigned long long tm = first + me; tm < last; tm += by_warp ? 32 : kSmallThreads) {
                 SynA a = e.syn[tm].a;
                 if (post_catch_up(a, t, f & 0xFFFFu, e, stdp, e.tab.ltp)) e.syn[tm].a = a;
             }
@@ -3037,6 +3042,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
                     const uint32_t own = D < 32 && lane <= D ? row[lane] : 0u;
                     const uint32_t k0 = D < 32 ? __shfl_sync(0xffffffffu, own, 0) : row[0];
                     const uint32_t k1 = D < 32 ? __shfl_sync(0xffffffffu, own, D & 31) : row[D];
+                    if (lane == 0 && k1 - k0 > 256) atomicMax(&s_widest, min(k1 - k0, 1u << 24));
                     for (uint32_t kb = k0; kb < k1; kb += 32) {
                         const uint32_t k = kb + lane;
                         const unsigned long long v = k < k1 ? from[k] : 0ull;
@@ -3082,6 +3088,15 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
         proxy_fence();  // (the next due list, written here, comes in by a bulk copy)
         __syncwarp();
         cluster_arrive();
+        if (threadIdx.x == 0) {
+            debt += kSmallRow * s_rows + kSmallCopy * s_widest + nf * span / 10 * kSmallClass10 +
+                    (nw > kSmallThreads && n > kSmallEven ? (n - kSmallEven) * kSmallEvent : 0u);
+            debt = debt > gain ? debt - gain : 0u;
+            // (the other blocks may not see this before their next tick's
+            // barrier: the run ends after that tick)
+            if (debt > kSmallDebt) atomicCAS(&e.ts->small_stop, 0u, t + 2);
+        }
+        __syncwarp();
         cluster_wait();
         ++t;
         if (t >= end) break;
@@ -3090,12 +3105,13 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
         __syncthreads();
     }
     __syncthreads();
+    if (threadIdx.x == 0) e.ts->small_debt[c] = debt;
     if (c != 0) return;
     for (uint32_t i = threadIdx.x; i < e.W; i += kSmallThreads) e.slot_count[i] = s_slot[i];
     if ((threadIdx.x & 31) == 0 && external) atomicAdd(&e.ts->external, external);
     if (threadIdx.x == 0) {
         TickState* ts = e.ts;
-        if (t < end) atomicMax(&ts->small_stop, t == 0 ? 1u : t);
+        if (t < end) atomicCAS(&ts->small_stop, 0u, t == 0 ? 1u : t);
         ts->tick = t;
         ts->delivered += delivered;
         ts->fired += fired;

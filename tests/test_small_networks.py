@@ -89,3 +89,45 @@ def test_long_run_in_pieces(gpu_lib, port_lib):
         out.append((sim.digest(), [x.tolist() for x in sim.raster()]))
         sim.close()
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("kind", ["rows", "classes", "fan-out"])
+def test_costly_ticks(gpu_lib, port_lib, kind):
+    """Networks whose ticks lose time in the one-kernel form (many rows of
+    post-spike STDP, fires times delivery classes, one fire's events), so that
+    the other kernels take over in the middle of a run."""
+    rng = np.random.default_rng(4)
+    if kind == "rows":  # 4,000 inputs to each of 40 outputs that fire in every tick
+        n, delays = 4040, [1]
+        source, target = np.repeat(np.arange(4000), 40), np.tile(np.arange(4000, 4040), 4000)
+    elif kind == "classes":
+        n, delays = 2500, np.arange(1, 250)
+        source, target = np.repeat(np.arange(n), 2), rng.integers(0, n, 2 * n)
+    else:
+        n, delays = 9000, np.arange(1, 250)
+        source, target = np.repeat(np.arange(3), 60_000), rng.integers(3, n, 180_000)
+    s = source.size
+    threshold = np.ones(n, np.float32)
+    if kind == "rows":
+        threshold[4000:] = 0.01
+    net = Connectome(
+        threshold=threshold, pattern_window_ticks=np.full(n, 9, np.uint64), similarity_threshold=np.full(n, 0.9, np.float32),
+        max_reference_patterns=np.full(n, 1, np.uint64), source=source.astype(np.uint32), target=target.astype(np.uint32),
+        weight=np.full(s, 0.004, np.float32), max_weight=np.full(s, 0.005, np.float32),
+        delay_ticks=rng.choice(delays, s).astype(np.uint32), compartment=np.ones(s, np.uint8), receptor=np.zeros(s, np.uint8),
+        plasticity_enabled=np.ones(s, np.uint8))
+    out = []
+    for lib in (gpu_lib, port_lib):
+        sim = Simulation(net, default_config(lib, raster_capacity=1 << 20), lib)
+        drive = np.random.default_rng(6)
+        for tick in range(60):
+            some = [tick % 3] if kind == "fan-out" and tick % 4 == 0 else [3] if kind == "fan-out" else \
+                drive.choice(2500 if kind == "classes" else 4000, 60 if kind == "rows" else 900, replace=False)
+            sim.inject(some, np.full(len(some), tick), np.full(len(some), 1.5, np.float32))
+        for stop in (0, 1, 30, 59):
+            sim.run_until(stop)
+            c, r = sim.counters(), sim.raster()
+            out.append(([c[k] for k in ("delivered_spikes", "fired_spikes", "external_events", "pending_events")],
+                        r[0].tolist(), r[1].tolist(), sim.digest()))
+        sim.close()
+    assert out[:4] == out[4:]
