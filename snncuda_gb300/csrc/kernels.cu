@@ -1095,13 +1095,14 @@ __device__ void block_radix_sort(unsigned long long* a, unsigned long long* b, u
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* mine = s_cnt + 256 * warp;
     uint32_t* s_tot = s_cnt + 256 * kWarps;
-    const uint32_t share = (len + kWarps * 32 - 1) / (kWarps * 32) * 32;
+    constexpr uint32_t kStep = 32 * kInFlight;  // a warp's shares are whole steps: none of them mostly empty
+    const uint32_t share = (len + kWarps * kStep - 1) / (kWarps * kStep) * kStep;
     const uint32_t i0 = min(len, warp * share), i1 = min(len, i0 + share);
     unsigned long long *src = a, *dst = b;
     for (uint32_t shift = 0; shift < bits; shift += 8) {
         for (uint32_t i = threadIdx.x; i < 256 * kWarps; i += kBlock) s_cnt[i] = 0;
         __syncthreads();
-        for (uint32_t c = i0; c < i1; c += 32 * kInFlight) {
+        for (uint32_t c = i0; c < i1; c += kStep) {
             unsigned long long v[kInFlight];
 #pragma unroll
             for (uint32_t u = 0; u < kInFlight; ++u) {
@@ -1129,7 +1130,7 @@ __device__ void block_radix_sort(unsigned long long* a, unsigned long long* b, u
         }
         __syncthreads();
         block_scan_shared<kBlock>(s_tot, 256);
-        for (uint32_t c = i0; c < i1; c += 32 * kInFlight) {
+        for (uint32_t c = i0; c < i1; c += kStep) {
             unsigned long long v[kInFlight];
 #pragma unroll
             for (uint32_t u = 0; u < kInFlight; ++u) {
@@ -1312,11 +1313,15 @@ __global__ void __launch_bounds__(kThreads) k_group(const __grid_constant__ Engi
 }
 
 constexpr int kLongThreads = 1024;
+// The longest listed segment that a warp sorts when there is one for every warp:
+// a block takes about 10 us for it whatever its length (20,000 segments of 650
+// events 1.5 ms by warps, 2.0 by blocks; of 1,000 events 2.4 and 2.7).
+constexpr uint32_t kWarpSortMany = 1024;
 constexpr size_t kLongSmemBytes = 256 * (kLongThreads / 32 + 1) * sizeof(uint32_t);
 
 // Grouping entry points: due order of the segments k_group left: a warp for
 // each target of the buckets it listed, and a block for each target it listed
-// (more than kWarpSortEvents events).  One warp merged such a long segment: 200
+// (more than kWarpSortEvents events; of many, a warp for the shorter ones).  One warp merged such a long segment: 200
 // ms for the 450,000 events of one target among 9 M, now 1.6 (and 0.7 in
 // k_group before it, from 1.5 with every entry's own atomic on the one counter).
 // The entries of a listed bucket are all placed: their memory is the scratch.
@@ -1342,8 +1347,15 @@ __global__ void __launch_bounds__(kLongThreads) k_group_rest(const __grid_consta
         if (len <= kWarpSortEvents) sort_group(g, tmp, len);
     }
     const uint32_t bits = due_bits(e.ts->n_due);
+    const bool many = targets >= warps;
+    if (many)
+        for (uint32_t k = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; k < targets; k += warps) {
+            const uint32_t len = segment(e.bcnt[k], g, tmp);
+            if (len <= kWarpSortMany) sort_group(g, tmp, len);
+        }
     for (uint32_t k = blockIdx.x; k < targets; k += gridDim.x) {
         const uint32_t len = segment(e.bcnt[k], g, tmp);
+        if (many && len <= kWarpSortMany) continue;
         __syncthreads();
         block_radix_sort<kLongThreads>(g, tmp, len, bits, s_radix);
     }

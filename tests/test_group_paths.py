@@ -46,3 +46,13 @@ def test_full_bucket(gpu_lib, count):
     ev = make_events(rng, count, 200)  # one bucket
     _check(gpu_lib, ev, 200, "snncuda_group_events")
     assert (ev & EXT).any()
+
+
+def test_a_long_segment_for_every_warp(gpu_lib):
+    """More segments above 512 events than the kernel has warps: up to 1,024
+    events each is a warp's work then, more a block's."""
+    neurons, rng = 6000, np.random.default_rng(9)
+    sizes = rng.choice([512, 513, 600, 1024, 1025, 1300], neurons)
+    ev = make_events(rng, int(sizes.sum()), neurons)
+    target = rng.permutation(np.repeat(np.arange(neurons, dtype=np.uint64), sizes))
+    _check(gpu_lib, (ev & ~np.uint64(0x7FFFFFFF)) | target, neurons, "snncuda_group_events")
