@@ -1257,10 +1257,17 @@ HostState fetch_all(snncuda_sim* sim, bool temporal) {
     return h;
 }
 
-// Neurons or synapses from which a read unpacks the records on the device:
-// below, copying the records and filling the caller's arrays here is as quick
-// as a copy per array (64 bytes a record, under 1 MB).
-constexpr uint64_t kUnpackFrom = 8192;
+// Whether a read of n neurons or synapses unpacks the records on the device, `cap`
+// at a time: a round is about 14 kernels and copies, 100 us, which its records
+// have to make good against copying them whole and filling the caller's arrays
+// here.  That takes 12 to 18 ns a neuron (16,384: 246 us both ways, 32,768: 291
+// and 409) and, as the order's cache misses grow, 17 to 50 ns a synapse (12,000:
+// 200 and 207 us, 65,536: 303 and 2,045; 1e6 by 2,048, 489 rounds: 53 and 50 ms).
+bool unpack_pays(uint64_t n, uint64_t cap, uint64_t per_round) {
+    return n > 0 && (n + cap - 1) / cap * per_round <= n;
+}
+constexpr uint64_t kUnpackNeurons = 16384;
+constexpr uint64_t unpack_synapses_from(uint64_t n) { return n >= 65536 ? 3072 : 12288; }
 
 // The caller's arrays of one read and their places in the device buffer that
 // the unpacking kernel fills for up to `cap` records at a time.  The buffers
@@ -1523,7 +1530,7 @@ static void unpack_neurons(snncuda_sim* sim, uint32_t n0, uint32_t n1, const snn
 
 // Neurons [n0, n1) into o[0 .. n1-n0).
 static void read_neurons_range(snncuda_sim* sim, uint32_t n0, uint32_t n1, const snncuda_neuron_state* o) {
-    if (n1 - n0 >= kUnpackFrom) {
+    if (unpack_pays(n1 - n0, UnpackBuffers(sim->e).cap, kUnpackNeurons)) {
         unpack_neurons(sim, n0, n1, o);
         return;
     }
@@ -1604,7 +1611,7 @@ static void unpack_synapses(snncuda_sim* sim, uint64_t c0, uint64_t c1, const sn
 // [t0, t1), into o[0 .. c1-c0).
 static void read_synapses_range(snncuda_sim* sim, uint64_t c0, uint64_t c1, uint64_t t0, uint64_t t1,
                          const snncuda_synapse_state* o) {
-    if (c1 - c0 >= kUnpackFrom) {
+    if (unpack_pays(c1 - c0, UnpackBuffers(sim->e).cap, unpack_synapses_from(c1 - c0))) {
         unpack_synapses(sim, c0, c1, o);
         return;
     }
