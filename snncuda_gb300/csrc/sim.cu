@@ -1263,6 +1263,8 @@ HostState fetch_all(snncuda_sim* sim, bool temporal) {
 // here.  That takes 12 to 18 ns a neuron (16,384: 246 us both ways, 32,768: 291
 // and 409) and, as the order's cache misses grow, 17 to 50 ns a synapse (12,000:
 // 200 and 207 us, 65,536: 303 and 2,045; 1e6 by 2,048, 489 rounds: 53 and 50 ms).
+// With wheel slots of 1,024 events 100,000 neurons took 23 ms in rounds, 1.1
+// whole; 9,000 neurons 229 us in one round, 164 whole.
 bool unpack_pays(uint64_t n, uint64_t cap, uint64_t per_round) {
     return n > 0 && (n + cap - 1) / cap * per_round <= n;
 }
