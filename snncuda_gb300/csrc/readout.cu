@@ -99,6 +99,9 @@ __device__ __forceinline__ float input_weight(const uint32_t* nb, const float* w
 // would.  A call with 64 samples x 100 inputs and 100 readouts of 500 synapses
 // went from 1.55 to 0.67 ms, together with the call's one copy each way; what
 // is left is the conversion of the samples in Python.
+//
+// kThread: a thread per readout all the same (forward_by_thread).
+template <bool kThread>
 __global__ void __launch_bounds__(kThreads) k_feedforward(ForwardArgs a) {
     extern __shared__ uint32_t s_key[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -119,28 +122,40 @@ __global__ void __launch_bounds__(kThreads) k_feedforward(ForwardArgs a) {
             }
             __syncthreads();
         }
-        for (uint32_t r = blockIdx.x * (kThreads / 32) + warp; r < a.R; r += gridDim.x * (kThreads / 32)) {
-            const uint32_t n = a.readouts[r];
-            const unsigned long long e0 = a.g.ptr[n], e1 = a.g.ptr[n + 1];
-            float score = 0.0F;
-            for (unsigned long long c = e0; c < e1; c += 32) {
-                const bool in = c + lane < e1;
-                const uint32_t src = in ? a.g.src[c + lane] : kNoNeuron;
-                float x = 0.0F;
-                if (in && a.hashed) {
-                    uint32_t at = hash_of(src, mask), key;
-                    while ((key = s_key[at]) != kNoNeuron && key != src) at = (at + 1) & mask;
-                    if (key == src) x = s_val[at];
-                } else if (in) {
-                    x = input_weight(a.in_n + b, a.in_w + b, m, src);
+        auto weight_of = [&](uint32_t src) {
+            if (!a.hashed) return input_weight(a.in_n + b, a.in_w + b, m, src);
+            uint32_t at = hash_of(src, mask), key;
+            while ((key = s_key[at]) != kNoNeuron && key != src) at = (at + 1) & mask;
+            return key == src ? s_val[at] : 0.0F;
+        };
+        auto put = [&](uint32_t r, float score) {
+            a.scores[static_cast<size_t>(s) * a.R + r] = score;
+            a.spikes[static_cast<size_t>(s) * a.R + r] = score >= a.thresholds[r] ? 1ull : 0ull;
+        };
+        if constexpr (kThread) {
+            for (uint32_t r = blockIdx.x * kThreads + threadIdx.x; r < a.R; r += gridDim.x * kThreads) {
+                const uint32_t n = a.readouts[r];
+                const unsigned long long e1 = a.g.ptr[n + 1];
+                float score = 0.0F;
+                for (unsigned long long e = a.g.ptr[n]; e < e1; ++e) {
+                    const float x = weight_of(a.g.src[e]);
+                    if (x != 0.0F) score = __fadd_rn(score, __fmul_rn(x, a.g.w[e]));
                 }
-                const float v = x != 0.0F ? __fmul_rn(x, a.g.w[c + lane]) : 0.0F;
-                for (uint32_t hit = __ballot_sync(0xffffffffu, x != 0.0F); hit; hit &= hit - 1)
-                    score = __fadd_rn(score, __shfl_sync(0xffffffffu, v, __ffs(hit) - 1));
+                put(r, score);
             }
-            if (lane == 0) {
-                a.scores[static_cast<size_t>(s) * a.R + r] = score;
-                a.spikes[static_cast<size_t>(s) * a.R + r] = score >= a.thresholds[r] ? 1ull : 0ull;
+        } else {
+            for (uint32_t r = blockIdx.x * (kThreads / 32) + warp; r < a.R; r += gridDim.x * (kThreads / 32)) {
+                const uint32_t n = a.readouts[r];
+                const unsigned long long e0 = a.g.ptr[n], e1 = a.g.ptr[n + 1];
+                float score = 0.0F;
+                for (unsigned long long c = e0; c < e1; c += 32) {
+                    const bool in = c + lane < e1;
+                    const float x = in ? weight_of(a.g.src[c + lane]) : 0.0F;
+                    const float v = x != 0.0F ? __fmul_rn(x, a.g.w[c + lane]) : 0.0F;
+                    for (uint32_t hit = __ballot_sync(0xffffffffu, x != 0.0F); hit; hit &= hit - 1)
+                        score = __fadd_rn(score, __shfl_sync(0xffffffffu, v, __ffs(hit) - 1));
+                }
+                if (lane == 0) put(r, score);
             }
         }
     }
@@ -591,6 +606,7 @@ struct snncuda_readout {
     uint32_t* delay{nullptr};
     float* w{nullptr};
     std::vector<uint64_t> degree;  // [N] incoming plus outgoing synapses
+    std::vector<unsigned long long> in_ptr;  // [N+1] ptr's contents
     // A call's device buffers are carved out of one that the handle keeps
     // (grown when a call needs more, freed with the handle), and its inputs
     // and results pass through one pinned host buffer: a call is one copy to
@@ -679,6 +695,12 @@ void fetch_results(snncuda_readout* r, size_t res, size_t spikes_at, size_t end,
     std::memcpy(spikes, r->host + spikes_at, count * sizeof(uint64_t));
 }
 
+// Whether a call's `results` (samples x readouts) take a thread each rather than
+// a warp: with enough of them to fill the GPU, and readouts of few synapses, whose
+// rows leave most of a warp's lanes idle.  1e6 results of 10 synapses 30 us by
+// threads, 239 by warps, 8.4e6 of 300 4.1 and 4.2 ms; 6,400 of 40 22 and 6 us.
+bool forward_by_thread(size_t results, uint64_t synapses) { return results >= (1u << 18) && synapses <= 256; }
+
 // Pinned bytes of a call whose inputs are [0, res) and results [res, end).
 size_t pinned_bytes(size_t res, size_t end) { return end - res > kStagedResults ? res : end; }
 
@@ -751,6 +773,7 @@ int snncuda_readout_create(const snncuda_network* net, snncuda_readout** out) {
         upload(r->src, src);
         upload(r->delay, dly);
         upload(r->w, w);
+        r->in_ptr = std::move(ptr);
     } catch (const Fail& f) {
         code = fail_code(f);
     } catch (const std::bad_alloc&) {
@@ -810,11 +833,16 @@ int snncuda_readout_feedforward(snncuda_readout* r, uint32_t samples, const uint
         a.scores = placed<float>(r, o_scores);
         a.spikes = placed<unsigned long long>(r, o_spikes);
         const size_t smem = a.hashed ? hash_slots(m.most) * 8ull : 0;
-        check(cudaFuncSetAttribute(k_feedforward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        uint64_t synapses = 0;
+        for (uint32_t n : list) synapses += r->in_ptr[n + 1] - r->in_ptr[n];
+        const bool by_thread = forward_by_thread(count, synapses / readout_count);
+        auto* kernel = by_thread ? k_feedforward<true> : k_feedforward<false>;
+        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(hash_slots(kHashInputs) * 8)),
               "feedforward attribute");
-        const uint32_t share = std::min(65535u, (readout_count + kThreads / 32 - 1) / (kThreads / 32));
-        k_feedforward<<<dim3(share, std::min(65535u, samples)), kThreads, smem>>>(a);
+        const uint32_t each = by_thread ? kThreads : kThreads / 32;  // readouts of a block at a time
+        const uint32_t share = std::min(65535u, (readout_count + each - 1) / each);
+        kernel<<<dim3(share, std::min(65535u, samples)), kThreads, smem>>>(a);
         check(cudaGetLastError(), "feedforward launch");
         fetch_results(r, res, o_spikes, l.at, count, scores, spikes);
     } catch (const Fail& f) {
