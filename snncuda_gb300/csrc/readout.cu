@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <type_traits>
 #include <utility>
@@ -610,7 +611,8 @@ struct snncuda_readout {
     // A call's device buffers are carved out of one that the handle keeps
     // (grown when a call needs more, freed with the handle), and its inputs
     // and results pass through one pinned host buffer: a call is one copy to
-    // the device, its kernels and one copy back.
+    // the device, its kernels and one copy back.  One call at a time has them.
+    std::mutex in_use;
     unsigned char* work{nullptr};
     size_t work_bytes{0};
     unsigned char* host{nullptr};
@@ -799,6 +801,7 @@ int snncuda_readout_feedforward(snncuda_readout* r, uint32_t samples, const uint
                                 uint64_t* delivered) {
     if (r == nullptr || (samples > 0 && input_ptr == nullptr)) return SNNCUDA_ERR_INVALID_ARGUMENT;
     int code = SNNCUDA_OK;
+    std::lock_guard<std::mutex> lock(r->in_use);
     try {
         if (delivered) std::fill(delivered, delivered + samples, 0);
         if (samples == 0 || readout_count == 0) return SNNCUDA_OK;
@@ -872,6 +875,7 @@ int snncuda_readout_recurrent(snncuda_readout* r, uint32_t samples, const uint64
     if (r == nullptr || options == nullptr || (samples > 0 && input_ptr == nullptr))
         return SNNCUDA_ERR_INVALID_ARGUMENT;
     int code = SNNCUDA_OK;
+    std::lock_guard<std::mutex> lock(r->in_use);
     try {
         if (delivered) std::fill(delivered, delivered + samples, 0);
         const uint64_t T = static_cast<uint64_t>(r->max_delay) * (1 + 2ull * options->iterations) + 1;
