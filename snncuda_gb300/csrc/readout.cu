@@ -609,7 +609,8 @@ struct snncuda_readout {
     std::vector<uint64_t> degree;  // [N] incoming plus outgoing synapses
     std::vector<unsigned long long> in_ptr;  // [N+1] ptr's contents
     // A call's device buffers are carved out of one that the handle keeps
-    // (grown when a call needs more, freed with the handle), and its inputs
+    // (grown when a call needs more, freed with the handle, or after the call if
+    // it is larger than the handle may keep: 256 MB, 64 MB pinned), and its inputs
     // and results pass through one pinned host buffer: a call is one copy to
     // the device, its kernels and one copy back.  One call at a time has them.
     std::mutex in_use;
@@ -626,6 +627,18 @@ struct snncuda_readout {
         if (host) cudaFreeHost(host);
     }
     InEdges edges() const { return InEdges{ptr, src, delay, w}; }
+    void trim() {
+        if (work_bytes > (256u << 20)) {
+            cudaFree(work);
+            work = nullptr;
+            work_bytes = 0;
+        }
+        if (host_bytes > (64u << 20)) {
+            cudaFreeHost(host);
+            host = nullptr;
+            host_bytes = 0;
+        }
+    }
     void need(size_t device_bytes, size_t pinned_bytes) {
         if (device_bytes > work_bytes) {
             cudaFree(work);
@@ -650,6 +663,13 @@ int fail_code(const Fail& f) {
     snngb::set_last_error_message(f.msg);
     return f.code;
 }
+
+// A call on a handle: no other at the same time, large buffers given back.
+struct Call {
+    snncuda_readout* r;
+    std::lock_guard<std::mutex> lock{r->in_use};
+    ~Call() { r->trim(); }
+};
 
 // Places of a call's arrays in the handle's buffers, each 256-byte aligned:
 // the inputs (copied from the pinned buffer, where they have the same
@@ -801,7 +821,7 @@ int snncuda_readout_feedforward(snncuda_readout* r, uint32_t samples, const uint
                                 uint64_t* delivered) {
     if (r == nullptr || (samples > 0 && input_ptr == nullptr)) return SNNCUDA_ERR_INVALID_ARGUMENT;
     int code = SNNCUDA_OK;
-    std::lock_guard<std::mutex> lock(r->in_use);
+    const Call call{r};
     try {
         if (delivered) std::fill(delivered, delivered + samples, 0);
         if (samples == 0 || readout_count == 0) return SNNCUDA_OK;
@@ -875,7 +895,7 @@ int snncuda_readout_recurrent(snncuda_readout* r, uint32_t samples, const uint64
     if (r == nullptr || options == nullptr || (samples > 0 && input_ptr == nullptr))
         return SNNCUDA_ERR_INVALID_ARGUMENT;
     int code = SNNCUDA_OK;
-    std::lock_guard<std::mutex> lock(r->in_use);
+    const Call call{r};
     try {
         if (delivered) std::fill(delivered, delivered + samples, 0);
         const uint64_t T = static_cast<uint64_t>(r->max_delay) * (1 + 2ull * options->iterations) + 1;

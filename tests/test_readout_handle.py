@@ -36,3 +36,16 @@ def test_two_threads(gpu_lib):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_large_call_gives_its_memory_back(gpu_lib):
+    """After a call with 400 MB of results, the handle keeps no buffer of that size."""
+    import torch
+    _, net = _network(9000, 9000, 2)
+    readout, chosen = Readout(net, gpu_lib), np.arange(8192)
+    samples = [[(i, 1.0)] for i in range(4096)]
+    readout.feedforward(samples[:2], chosen[:2])
+    before = torch.cuda.mem_get_info()[0]
+    scores = readout.feedforward(samples, chosen)[0]
+    assert before - torch.cuda.mem_get_info()[0] < 300 << 20
+    assert np.array_equal(readout.feedforward(samples[:64], chosen)[0], scores[:64])
