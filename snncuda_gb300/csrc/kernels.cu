@@ -3169,17 +3169,26 @@ __global__ void k_range_counts(Engine e, uint32_t nb, uint32_t ne, unsigned long
         pre += e.syn[i].b.pre_count;
         code_matches += e.syn[i].b.code_matches;
     }
-    // the wheel: blocks share out its slots (the loop over all of them in
-    // every block waited for W slot counts one after the other)
-    const uint32_t parts = gridDim.x > e.W ? gridDim.x / e.W : 1u;
-    for (uint32_t task = blockIdx.x; task < e.W * parts; task += gridDim.x) {
-        const uint32_t slot = task % e.W, part = task / e.W;
-        const uint32_t cnt = e.slot_count[slot];
+    // the wheel: every block has all slots' counts at once (one after the other
+    // they were W waits; a slot shared out to some blocks only took 91 us where this
+    // takes 71, 40,000 events in 32 slots); wheels of more slots than a block has
+    // threads are shared out by slots
+    auto count_events = [&](uint32_t slot, uint32_t cnt, unsigned long long from, unsigned long long step) {
         const unsigned long long* ev = e.wheel + static_cast<size_t>(slot) * e.slot_cap;
-        for (unsigned long long i = part * blockDim.x + threadIdx.x; i < cnt; i += parts * blockDim.x) {
+        for (unsigned long long i = from; i < cnt; i += step) {
             const uint32_t tgt = static_cast<uint32_t>(ev[i]) & ~kExternalBit;
             wheel += tgt >= nb && tgt < ne;
         }
+    };
+    __shared__ uint32_t s_count[kThreads];
+    if (e.W <= kThreads) {
+        if (threadIdx.x < e.W) s_count[threadIdx.x] = e.slot_count[threadIdx.x];
+        __syncthreads();
+        for (uint32_t slot = 0; slot < e.W; ++slot) count_events(slot, s_count[slot], first, stride);
+    } else {
+        const uint32_t parts = gridDim.x > e.W ? gridDim.x / e.W : 1u;
+        for (uint32_t task = blockIdx.x; task < e.W * parts; task += gridDim.x)
+            count_events(task % e.W, e.slot_count[task % e.W], task / e.W * blockDim.x + threadIdx.x, parts * blockDim.x);
     }
     if (spikes) atomicAdd(out, spikes);
     if (pre) atomicAdd(out + 1, pre);
