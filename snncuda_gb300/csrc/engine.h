@@ -257,7 +257,7 @@ struct Engine {
     // the two slow each other by more than the overlap gives).
     uint32_t side_serial;
     uint32_t inline_codes;                 // 1: inline_code_pattern holds for every target
-    uint32_t multi_refs;                   // 1: some target keeps several reference patterns (k_temporal runs)
+    uint32_t multi_refs;                   // most reference patterns of a target if several (k_temporal runs), else 0
     uint32_t* bcnt;                        // [grid_bucket][nbuckets] events of each (chunk, bucket)
     uint32_t* btot;                        // [nbuckets] events per bucket (zero between ticks)
     uint32_t* bstart;                      // [nbuckets + 1] first grouped position of each bucket

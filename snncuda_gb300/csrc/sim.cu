@@ -416,7 +416,7 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
         p.window = static_cast<uint32_t>(window);
         p.similarity = net->similarity_threshold[n];
         p.max_refs = static_cast<uint32_t>(refs);
-        if (refs > 1) e.multi_refs = 1;
+        if (refs > 1) e.multi_refs = std::max(e.multi_refs, static_cast<uint32_t>(refs));
         if (!inline_code_pattern(p.max_refs, max_expected)) e.inline_codes = 0;
         const uint64_t full = refs * (window + 1);
         p.ring_cap = static_cast<uint32_t>(std::min<uint64_t>(full, std::max<uint64_t>(window + 1, run_budget)));
