@@ -313,18 +313,25 @@ __host__ __device__ constexpr uint32_t bucket_shift_for(uint32_t N) {
 // target and tick on the dense workloads, 800 of the 1,280 a block's shared
 // memory holds) were the best fit there: 128 targets with twice the threads
 // took 273 us where 64 took 219 (recog_1m distributions at 200,000 neurons).
-// 32 targets where 64 would leave fewer than three blocks per SM.  Wider only
-// when there would be more than kMaxTickBuckets buckets (their counters fill
-// the placing blocks' shared memory).
+// 32 targets where 64 would leave fewer than three blocks per SM.  Wider, up to
+// 256 targets, where they have fewer than kBucketSynapses synapses, so that a
+// bucket's events would not keep a block busy, and at least kWideBuckets buckets
+// per SM are left (1e6 neurons of 50 synapses, 100,000 events: 266 us a tick with
+// 64 targets, 124 with 256; 2e6 of 5, 200,000 events: 736 and 492; at 5 buckets
+// per SM ticks of 1e6 and more events took 2 to 6 % longer), or when there would be
+// more than kMaxTickBuckets (their counters fill the placing blocks' shared
+// memory).
 constexpr uint32_t kMaxTickBuckets = 32768;
-inline uint32_t tick_bucket_shift(uint32_t N, uint32_t sms) {
+constexpr uint32_t kWideBuckets = 20, kBucketSynapses = 16384;
+inline uint32_t tick_bucket_shift(uint32_t N, uint64_t synapses, uint32_t sms) {
     if (bucket_shift_for(N) == 0) return 0;
     uint32_t s = (N >> 6) < 3 * sms ? 5 : 6;
+    while (s < 8 && (N >> (s + 1)) >= kWideBuckets * sms && (synapses << s) / N < kBucketSynapses) ++s;
     while (((static_cast<unsigned long long>(N) + (1ull << s) - 1) >> s) > kMaxTickBuckets) ++s;
     return s;
 }
-inline uint32_t tick_buckets(uint32_t N, uint32_t sms) {
-    const uint32_t s = tick_bucket_shift(N, sms);
+inline uint32_t tick_buckets(uint32_t N, uint64_t synapses, uint32_t sms) {
+    const uint32_t s = tick_bucket_shift(N, synapses, sms);
     const uint64_t n = (static_cast<uint64_t>(N) + (1u << s) - 1) >> s;
     return n > 0 ? static_cast<uint32_t>(n) : 1u;
 }

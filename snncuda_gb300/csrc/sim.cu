@@ -461,9 +461,9 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     // ---- grouping buckets and launch shapes ----
     int sms = 0;
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sim->device), "device attribute");
-    e.bucket_shift = tick_bucket_shift(N, static_cast<uint32_t>(std::max(1, sms)));
+    e.bucket_shift = tick_bucket_shift(N, S, static_cast<uint32_t>(std::max(1, sms)));
     if (e.bucket_shift == 0) throw_fail(SNNCUDA_ERR_UNSUPPORTED, "at most 2^28 neurons");
-    e.nbuckets = tick_buckets(N, static_cast<uint32_t>(std::max(1, sms)));
+    e.nbuckets = tick_buckets(N, S, static_cast<uint32_t>(std::max(1, sms)));
     // counting and placing blocks: two per SM, fewer for small networks (one
     // per 2^18 synapses), whose grids then leave room for other streams'
     // kernels (side-by-side jobs of a server)
@@ -2322,7 +2322,7 @@ static uint64_t estimate_bytes_impl(const snncuda_network* net, const snncuda_co
         sms = 152;
     }
     const uint32_t sm_count = static_cast<uint32_t>(std::max(1, sms));
-    const uint64_t buckets = bucket_shift_for(net->neuron_count) ? tick_buckets(net->neuron_count, sm_count) : 0;
+    const uint64_t buckets = bucket_shift_for(net->neuron_count) ? tick_buckets(net->neuron_count, S, sm_count) : 0;
     const uint64_t counters = buckets * (kBucketBlocksPerSm * sm_count + 3) * 4;
     const uint64_t persistent = 64 * S + 8 * S + 8 * pre_total + neuron_bytes + lcode +
                                 W * slot_cap * 8 + slot_cap * (8 + 16 + 16 + 16 + 4 + 1) + 4 * parts_cap(slot_cap) + counters +

@@ -36,6 +36,8 @@ def test_covers_the_buffers(n):
     _ensure_built()
     lib, slots, window = _abi.bind(str(GPU_PATH)), 4096, 1
     shift = 5 if n >> 6 < 3 * SMS else 6
+    while shift < 8 and n >> (shift + 1) >= 20 * SMS:  # (hardly any synapses: wide buckets)
+        shift += 1
     while -(-n >> shift) > 32768:
         shift += 1
     buckets = -(-n >> shift)
