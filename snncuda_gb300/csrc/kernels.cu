@@ -1338,21 +1338,19 @@ __global__ void __launch_bounds__(kLongThreads) k_group_rest(const __grid_consta
     unsigned long long *g, *tmp;
     const unsigned long long items = static_cast<unsigned long long>(buckets) << e.bucket_shift;
     const uint32_t warps = gridDim.x * (kLongThreads / 32);
-    // (item i's target: neighbouring warps take different blocks' SMs)
-    for (unsigned long long i = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; i < items; i += warps) {
-        const uint32_t n = (e.btot[i >> e.bucket_shift] << e.bucket_shift) +
-                           static_cast<uint32_t>(i & ((1u << e.bucket_shift) - 1u));
+    const bool many = targets >= warps;
+    // (item i's target: neighbouring warps take different blocks' SMs; the
+    // listed targets come behind the buckets')
+    for (unsigned long long i = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; i < items + (many ? targets : 0u); i += warps) {
+        const bool listed = i >= items;
+        const uint32_t n = listed ? e.bcnt[i - items]
+                                  : (e.btot[i >> e.bucket_shift] << e.bucket_shift) +
+                                        static_cast<uint32_t>(i & ((1u << e.bucket_shift) - 1u));
         if (n >= e.N) continue;
         const uint32_t len = segment(n, g, tmp);
-        if (len <= kWarpSortEvents) sort_group(g, tmp, len);
+        if (listed ? len <= kWarpSortMany : len <= kWarpSortEvents) sort_group(g, tmp, len);
     }
     const uint32_t bits = due_bits(e.ts->n_due);
-    const bool many = targets >= warps;
-    if (many)
-        for (uint32_t k = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; k < targets; k += warps) {
-            const uint32_t len = segment(e.bcnt[k], g, tmp);
-            if (len <= kWarpSortMany) sort_group(g, tmp, len);
-        }
     for (uint32_t k = blockIdx.x; k < targets; k += gridDim.x) {
         const uint32_t len = segment(e.bcnt[k], g, tmp);
         if (many && len <= kWarpSortMany) continue;
