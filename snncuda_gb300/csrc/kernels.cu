@@ -1486,24 +1486,26 @@ __device__ __forceinline__ TargetParam load_param(const NeuronParam* p) {
 }
 
 // The blocks of k_small share out the neurons by runs of kSmallChunk: every block
-// has one of eight neighbouring runs, at a place that changes with the digits of
-// the run's number.  Neighbours, which are often busy together (an output layer),
-// so go to different blocks, whatever the distance of such groups; one by one,
-// the records' reads would take twice the lines (38 us a tick of 5,000 events
-// with runs of 8 or 32, 45 with 1).
+// has one of eight neighbouring runs, at a place that the number of their group
+// turns by a little less than three.  Neighbours, which are often busy together
+// (an output layer), so go to different blocks, and so do groups of them at any
+// regular distance (a layer of every column: the busiest block has 1.04 times
+// its share on average, 1.2 at worst, over widths of 5 to 32 and 3 to 32 layers).
+// One by one, the records' reads would take twice the lines (38 us a tick of
+// 5,000 events with runs of 8 or 32, 45 with 1).
 constexpr uint32_t kSmallChunk = 8;
-static_assert(kSmallBlocks == 8 && kSmallBlocks * kSmallTargets <= 1u << 15, "the digits summed up");
+static_assert(kSmallBlocks == 8, "a group is eight runs");
 
+__device__ __forceinline__ uint32_t small_turn(uint32_t group) { return group * 93 >> 5; }
 __device__ __forceinline__ uint32_t small_block(uint32_t n) {
-    const uint32_t run = n / kSmallChunk;
-    return (run + (run >> 3) + (run >> 6) + (run >> 9)) % kSmallBlocks;
+    return (n / kSmallChunk + small_turn(n / (kSmallChunk * kSmallBlocks))) % kSmallBlocks;
 }
 // A neuron's place among its block's, and the neuron at place j of block c.
 __device__ __forceinline__ uint32_t small_place(uint32_t n) {
     return n / (kSmallChunk * kSmallBlocks) * kSmallChunk + n % kSmallChunk;
 }
 __device__ __forceinline__ uint32_t small_neuron(uint32_t c, uint32_t j) {
-    const uint32_t high = j / kSmallChunk, run = high * kSmallBlocks + (c - high - (high >> 3) - (high >> 6)) % kSmallBlocks;
+    const uint32_t group = j / kSmallChunk, run = group * kSmallBlocks + (c - small_turn(group)) % kSmallBlocks;
     return run * kSmallChunk + j % kSmallChunk;
 }
 
@@ -2823,7 +2825,7 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     uint32_t parity = 0;
     bool staging = true;
     uint32_t debt = threadIdx.x == 0 ? e.ts->small_debt[c] : 0u;  // (thread 0 keeps it)
-    const uint32_t gain = kSmallGain - e.N / 8 + kSmallClassGain * D;
+    const uint32_t gain = kSmallGain - e.N / 4 + kSmallClassGain * D;
     __syncthreads();
     for (;;) {
         const uint32_t slot = t & e.wmask, n = s_slot[slot];
@@ -2939,16 +2941,18 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
         // meanwhile the post-spike STDP of this block's fired targets (k_post)
         // (a warp per target when there are as many as warps, else the block)
         const bool by_warp = s_fired >= kSmallThreads / 32;
+        uint32_t rows = 0;
         for (uint32_t k = by_warp ? threadIdx.x >> 5 : 0u; k < s_fired; k += by_warp ? kSmallThreads / 32 : 1u) {
             const uint32_t f = out.targets[k], tgt = small_neuron(c, f >> 16);
             const unsigned long long first = e.in_ptr[tgt], last = e.in_ptr[tgt + 1];
             const uint32_t me = by_warp ? threadIdx.x & 31 : threadIdx.x;
-            if (me == 0) atomicAdd(&s_rows, static_cast<uint32_t>(min(last - first, 1ull << 17)));
+            if (me == 0) rows += static_cast<uint32_t>(min(last - first, 1ull << 17));
             for (unsigned long long tm = first + me; tm < last; tm += by_warp ? 32 : kSmallThreads) {
                 SynA a = e.syn[tm].a;
                 if (post_catch_up(a, t, f & 0xFFFFu, e, stdp, e.tab.ltp)) e.syn[tm].a = a;
             }
         }
+        if (rows > kSmallThreads / 4) atomicAdd(&s_rows, rows);  // (a few are no loss)
         __syncwarp();
         cluster_wait();
         if (threadIdx.x < kSmallBlocks) s_count[threadIdx.x] = __ldcg(e.bcnt + threadIdx.x);
