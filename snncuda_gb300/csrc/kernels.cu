@@ -2023,6 +2023,30 @@ __device__ __forceinline__ void bucket_events(const Engine& e, const BucketSpace
                     out);
 }
 
+// The entries of the targets j0 .. j0 + nw - 1 among a bucket's `all`, as far as
+// they fit, into s_in (targets from j0); whole block.  Returns their number and
+// that of the entries before j0.
+__device__ __noinline__ uint2 pick_part(const uint4* in, uint32_t all, uint32_t j0, uint32_t nw, uint4* s_in) {
+    __shared__ uint32_t s_mine, s_before;
+    __syncthreads();
+    if (threadIdx.x == 0) s_mine = s_before = 0;
+    __syncthreads();
+    uint32_t before = 0;
+    for_entries(in, all, kNoTarget, [&](const uint4& q) {
+        const uint32_t j = q.z - j0, mine = __ballot_sync(0xffffffffu, j < nw);
+        before += q.z < j0;
+        if (mine == 0) return;
+        uint32_t p = 0;
+        if ((threadIdx.x & 31) == 0) p = atomicAdd(&s_mine, __popc(mine));
+        p = __shfl_sync(0xffffffffu, p, 0) + __popc(mine & ((1u << (threadIdx.x & 31)) - 1u));
+        if (j < nw && p < kBlockEvents) s_in[p] = make_uint4(q.x, q.y, j, 0u);
+    });
+    before = __reduce_add_sync(0xffffffffu, before);
+    if ((threadIdx.x & 31) == 0 && before) atomicAdd(&s_before, before);
+    __syncthreads();
+    return make_uint2(s_mine, s_before);
+}
+
 // Everything a tick does at its targets, a block per bucket of consecutive
 // targets (a bucket's events are one contiguous run of grp_tmp), or per part of
 // a bucket that is too large for a block (part_shift), whose entries the block
@@ -2070,7 +2094,6 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
     __shared__ Refire s_refire[kEventThreads];      // targets that go on after their first fire
     __shared__ uint32_t s_refires;
     __shared__ uint32_t s_longest;                  // events of the busiest target
-    __shared__ uint32_t s_mine, s_before;           // a part's entries, and the bucket's before them
     const uint32_t width = 1u << e.bucket_shift;
     // the staged entries (16 bytes per event); once they are in registers, the
     // words grouped by target (8) and the words in due order (8); once those
@@ -2109,25 +2132,9 @@ __global__ void __launch_bounds__(kEventThreads, SNNGB_EVENTS_MIN_BLOCKS) k_even
             if (j0 >= nw) continue;  // past the last target
             nw = min(nw - j0, range);
             n0 += j0;
-            __syncthreads();
-            if (threadIdx.x == 0) s_mine = s_before = 0;
-            __syncthreads();
-            // its entries, as far as they fit, and the number before them
-            uint32_t before = 0;
-            for_entries(in, all, kNoTarget, [&](const uint4& q) {
-                const uint32_t j = q.z - j0, mine = __ballot_sync(0xffffffffu, j < nw);
-                before += q.z < j0;
-                if (mine == 0) return;
-                uint32_t p = 0;
-                if ((threadIdx.x & 31) == 0) p = atomicAdd(&s_mine, __popc(mine));
-                p = __shfl_sync(0xffffffffu, p, 0) + __popc(mine & ((1u << (threadIdx.x & 31)) - 1u));
-                if (j < nw && p < kBlockEvents) s_in[p] = make_uint4(q.x, q.y, j, 0u);
-            });
-            before = __reduce_add_sync(0xffffffffu, before);
-            if ((threadIdx.x & 31) == 0 && before) atomicAdd(&s_before, before);
-            __syncthreads();
-            m = s_mine;
-            lo += s_before;
+            const uint2 got = pick_part(in, all, j0, nw, s_in);
+            m = got.x;
+            lo += got.y;
         } else {
             if (threadIdx.x == 0) {  // the bucket's total and cursor start at zero next tick
                 e.btot[b] = 0;

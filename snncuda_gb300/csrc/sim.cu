@@ -494,7 +494,6 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     e.btot = salloc<uint32_t>(sim, e.nbuckets, BufKind::kZero);
     e.bstart = salloc<uint32_t>(sim, static_cast<size_t>(e.nbuckets) + 1, BufKind::kScratch);
     e.bcur = salloc<uint32_t>(sim, e.nbuckets, BufKind::kZero);
-    e.parts = salloc<uint32_t>(sim, parts_cap(slot_cap), BufKind::kScratch);
     e.grp = salloc<unsigned long long>(sim, slot_cap, BufKind::kScratch);
     e.grp_tmp = salloc<BucketEntry>(sim, slot_cap, BufKind::kScratch);
     e.evin = salloc<EvIn>(sim, slot_cap, BufKind::kScratch);
@@ -513,6 +512,9 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     auto* d_decay = salloc<float>(sim, decay.size());
     auto* d_ltp = salloc<float>(sim, ltp.size());
     auto* d_ltd = salloc<float>(sim, ltd.size());
+    // (behind the others: between them it moved the fire bitmap's buffers, and
+    // k_fire_list took 20.9 us instead of 18.3 at 100,000 neurons)
+    e.parts = salloc<uint32_t>(sim, parts_cap(slot_cap), BufKind::kScratch);
 
     cudaStream_t st = sim->stream;
     auto h2d = [&](void* dst, const void* src, size_t bytes) {
