@@ -103,11 +103,12 @@ MINIMAL_BYTES = {
 }
 # Bytes of this engine's own layout (snncuda_gb300/csrc/engine.h) per
 # synaptic event, external event and touched target:
-#   k_events   bucketed entry (16), synapse record read + write (2 x 64);
-#              externals: entry; per target its parameters (64), neuron
+#   k_events   bucketed entry (16), synapse record read + write (2 x 64),
+#              its fields before the event (16, Engine::ev_a0); externals:
+#              entry; per target its parameters (64), neuron
 #              record and temporal bookkeeping, read + write (2 x 64 + 2 x 32)
 LAYOUT_BYTES = {
-    "k_events": (16 + 64 + 64, 16, 64 + 2 * 64 + 2 * 32),
+    "k_events": (16 + 64 + 64 + 16, 16, 64 + 2 * 64 + 2 * 32),
 }
 # DRAM bytes (read + write) per synaptic event of a kernel, from one ncu
 # capture (dram__bytes_read.sum + dram__bytes_write.sum) of the 80 k_events

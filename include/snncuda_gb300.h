@@ -381,7 +381,9 @@ int snncuda_sim_estimate_bytes(const snncuda_network* network, const snncuda_con
  * No counterpart in the reference (which times the whole tick loop on the
  * host clock, spike_throughput_benchmark.cpp:137-140).  Processes ticks like
  * snncuda_sim_run_until, but launches one tick at a time from a graph whose
- * event nodes bracket every kernel, and accumulates device time per kernel
+ * event nodes bracket every kernel (on networks whose ordinary runs take whole
+ * ticks in one kernel, too: it times the launched kernels, which such runs take
+ * for their busy ticks only), and accumulates device time per kernel
  * plus the work counters of the profiled ticks into *out (zero it first). */
 #define SNNCUDA_KERNEL_COUNT 10
 typedef struct snncuda_profile {

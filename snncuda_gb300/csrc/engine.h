@@ -180,8 +180,7 @@ struct TickState {
     uint32_t far_ticks;       // entries of far_idx minus one (0 = none)
     int32_t stdp_enabled;     // StdpRule::enabled (runtime toggle)
     int32_t temporal_enabled; // SynapseDendriteConfig::temporal_learning_enabled
-    uint32_t done_scan;       // "last block" counters
-    uint32_t done_fire_list;
+    uint32_t done_fire_list;  // "last block" counter
     uint32_t small_stop;      // not 0: k_small ended before its last tick (launch_small)
     uint32_t n_parts;         // entries of Engine::parts this tick (reset by k_bcount),
     uint32_t part_events;     // and events of a part (part_shift)
@@ -241,9 +240,10 @@ struct Engine {
     uint32_t* slot_count;                  // [W]
 
     // per-tick scratch: grouping by target.  Targets are bucketed by
-    // bucket_shift (2^bucket_shift consecutive targets per bucket, at most
-    // kMaxBuckets buckets); grid_bucket blocks each count and place one
-    // contiguous chunk of the due list.
+    // bucket_shift (2^bucket_shift consecutive targets per bucket: tick_bucket_shift,
+    // at most kMaxTickBuckets buckets; bucket_shift_for, at most kMaxBuckets, in
+    // grouping calls); grid_bucket blocks each count and place one contiguous chunk
+    // of the due list.
     uint32_t bucket_shift;
     uint32_t nbuckets;
     uint32_t grid_bucket;
@@ -292,7 +292,6 @@ struct Engine {
     // picks grid_events, grid_bucket and grid_process)
     uint32_t grid_wide;
     uint32_t grid_process;  // k_temporal blocks
-    uint32_t grid_walk;     // (a tuning field without effect: k_events walks its own targets)
     uint32_t grid_fire;
     uint32_t grid_events;   // k_events blocks at most (one per bucket)
 };
@@ -405,12 +404,12 @@ constexpr uint32_t kMaxClasses = 256;    // distinct delivery delays
 // `marks` (optional) holds 2 * kKernelCount events recorded around every
 // kernel (before, after) for profiling graphs.
 constexpr int kKernelCount = 8;
-// The streams of a tick: k_temporal and k_post run on `side`, forked from
-// `main` with ev[0] / ev[2] and joined back with ev[1] / ev[3].
+// The streams of a tick: k_post and k_temporal run on `side`, forked from
+// `main` with ev[0] and joined back with ev[1].
 struct TickStreams {
     cudaStream_t main;
     cudaStream_t side;
-    cudaEvent_t ev[4];
+    cudaEvent_t ev[2];
 };
 void launch_tick(const Engine& e, const TickStreams& s, cudaEvent_t* marks = nullptr);
 const char* kernel_name(int index);

@@ -37,8 +37,9 @@
 //
 // Every wait is a kernel boundary (a programmatic dependent's grid
 // dependency wait included), a "last block" hand-off (an atomic counter, no
-// spinning) or the time-bounded mbarrier wait of a staging copy, so no kernel
-// here can hang.
+// spinning), the time-bounded mbarrier wait of a staging copy, or, in k_small, the
+// hardware barrier of its cluster, whose blocks all reach it or have exited (which
+// counts), so no kernel here can hang.
 // Float arithmetic uses explicitly rounded intrinsics so nothing is
 // contracted into an FMA: each operation rounds exactly as the reference's
 // separately evaluated float expressions.
@@ -1376,7 +1377,7 @@ __global__ void k_group_init(const __grid_constant__ Engine e, uint32_t count) {
 // against the last post spike, last_pre, the pre-spike count, and the
 // spike-code pattern (:318-365).  None of it depends on the target's neuron
 // state; only the STDP part depends on whether the target fired earlier in the
-// tick, which the walk handles by redoing it (walk_fired_targets).
+// tick, which the walk handles by redoing it (walk_after_fire).
 template <bool kInline>
 __device__ __forceinline__ void pre_event(SynAB& r, const TargetParam& p, uint32_t t, uint16_t* lc,
                                           const Engine& e, int stdp, int temporal, bool inl) {
@@ -1475,8 +1476,8 @@ __device__ __forceinline__ void store_record(SynAB* p, const SynAB& r) {
                  : "memory");
 }
 
-// The parameters of a bucket's targets: in shared memory, or (buckets wider
-// than kSharedParams targets: networks beyond 2^22 neurons) in the first 16
+// The parameters of a block's targets: in shared memory, or (k_small, and buckets
+// wider than kSharedParams targets: networks beyond 2^23 neurons) in the first 16
 // bytes of each NeuronParam.
 constexpr uint32_t kSharedParams = 256;
 

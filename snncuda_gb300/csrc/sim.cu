@@ -202,10 +202,11 @@ struct snncuda_sim {
     cudaEvent_t marks[2 * kKernelCount]{};
     uint32_t ticks_per_graph{16};  // ticks captured in graph_many
     uint32_t sms{1};
+    uint32_t grid_walk{1};         // snncuda_tuning::grid_walk (without effect)
 
     // second stream of the tick graphs and its fork/join events
     cudaStream_t side{nullptr};
-    cudaEvent_t tick_ev[4]{};
+    cudaEvent_t tick_ev[2]{};
     // eviction: the device state held in host memory (evict_impl / restore_impl)
     bool evicted{false};
     std::vector<std::vector<unsigned char>> evicted_data;  // per owned buffer
@@ -268,7 +269,7 @@ struct snncuda_sim {
         if (profiled && marks[0] == nullptr)
             for (cudaEvent_t& ev : marks) check(cudaEventCreate(&ev), "event");
         check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-        const TickStreams ts{stream, side, {tick_ev[0], tick_ev[1], tick_ev[2], tick_ev[3]}};
+        const TickStreams ts{stream, side, {tick_ev[0], tick_ev[1]}};
         for (int i = 0; i < ticks; ++i) launch_tick(e, ts, profiled ? marks : nullptr);
         check(cudaStreamEndCapture(stream, &g), "end capture");
         cudaGraphExec_t exec = nullptr;
@@ -562,7 +563,7 @@ void create_impl(const snncuda_network* net, const snncuda_config& cfg, snncuda_
     e.grid_events = e.grid_wide * 8;
     sim->sms = static_cast<uint32_t>(std::max(1, sms));
     e.grid_process = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((N + 255) / 256, sms * 8ull)));
-    e.grid_walk = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((N + 63) / 64, sms * 8ull)));
+    sim->grid_walk = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((N + 63) / 64, sms * 8ull)));
     e.grid_fire = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(fire_tiles, sms * 8ull)));
     // Post-spike STDP beside the fire ordering or in tick order: a tick of
     // 7e7 synapses takes 124 us beside and 130 in order, of 2e8 334 and 348,
@@ -880,7 +881,7 @@ void autotune_impl(snncuda_sim* sim, uint64_t probe_ticks, snncuda_tuning* out) 
     ++probes;
     if (out) {
         out->grid_events = e.grid_events;
-        out->grid_walk = e.grid_walk;
+        out->grid_walk = sim->grid_walk;
         out->grid_bucket = e.grid_bucket;
         out->scatter_pass_events = e.scatter_pass_events;
         out->side_serial = e.side_serial;
@@ -911,7 +912,7 @@ void apply_tuning_impl(snncuda_sim* sim, const snncuda_tuning& t) {
         t.side_serial > 1 || (t.block_threads != 0 && t.block_threads != 256))
         throw_fail(SNNCUDA_ERR_INVALID_ARGUMENT, "tuning field outside the autotuner's ranges");
     e.grid_events = t.grid_events;
-    e.grid_walk = t.grid_walk;
+    sim->grid_walk = t.grid_walk;
     e.grid_bucket = t.grid_bucket;
     e.grid_process = t.grid_temporal;
     e.scatter_pass_events = t.scatter_pass_events;
