@@ -3180,9 +3180,8 @@ __global__ void k_range_counts(Engine e, uint32_t nb, uint32_t ne, unsigned long
         code_matches += e.syn[i].b.code_matches;
     }
     // the wheel: every block has all slots' counts at once (one after the other
-    // they were W waits; a slot shared out to some blocks only took 91 us where this
-    // takes 71, 40,000 events in 32 slots); wheels of more slots than a block has
-    // threads are shared out by slots
+    // they were W waits); wheels of more slots than a block has threads are shared
+    // out by slots
     auto count_events = [&](uint32_t slot, uint32_t cnt, unsigned long long from, unsigned long long step) {
         const unsigned long long* ev = e.wheel + static_cast<size_t>(slot) * e.slot_cap;
         for (unsigned long long i = from; i < cnt; i += step) {
@@ -3194,17 +3193,31 @@ __global__ void k_range_counts(Engine e, uint32_t nb, uint32_t ne, unsigned long
     if (e.W <= kThreads) {
         if (threadIdx.x < e.W) s_count[threadIdx.x] = e.slot_count[threadIdx.x];
         __syncthreads();
-        for (uint32_t slot = 0; slot < e.W; ++slot) count_events(slot, s_count[slot], first, stride);
+        // (a slot's first events go to another block each time: few events would
+        // otherwise be the first blocks' work, slot after slot)
+        const uint32_t turn = gridDim.x / e.W;
+        for (uint32_t slot = 0; slot < e.W; ++slot) {
+            const uint32_t at = blockIdx.x + slot * turn, b = at < gridDim.x ? at : at - gridDim.x;
+            count_events(slot, s_count[slot], b * blockDim.x + threadIdx.x, stride);
+        }
     } else {
         const uint32_t parts = gridDim.x > e.W ? gridDim.x / e.W : 1u;
         for (uint32_t task = blockIdx.x; task < e.W * parts; task += gridDim.x)
             count_events(task % e.W, e.slot_count[task % e.W], task / e.W * blockDim.x + threadIdx.x, parts * blockDim.x);
     }
-    if (spikes) atomicAdd(out, spikes);
-    if (pre) atomicAdd(out + 1, pre);
-    if (wheel) atomicAdd(out + 2, wheel);
-    if (matches) atomicAdd(out + 3, matches);
-    if (code_matches) atomicAdd(out + 4, code_matches);
+    // one atomic a block and sum (a thread each, they took longer than the reads)
+    __shared__ unsigned long long s_sum[5];
+    __syncthreads();
+    if (threadIdx.x < 5) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned long long sums[5] = {spikes, pre, wheel, matches, code_matches};
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        for (int d = 16; d > 0; d >>= 1) sums[k] += __shfl_down_sync(0xffffffffu, sums[k], d);
+        if ((threadIdx.x & 31) == 0 && sums[k]) atomicAdd(&s_sum[k], sums[k]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 5 && s_sum[threadIdx.x]) atomicAdd(out + threadIdx.x, s_sum[threadIdx.x]);
 }
 
 // Readers: a thread per neuron or synapse; the outputs are coalesced, the
