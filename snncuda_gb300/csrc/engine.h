@@ -426,7 +426,8 @@ constexpr uint32_t kSmallSlots = 1024;
 // event of the fire with the most (one warp copies them: 32 in 0.5 us), a fire
 // and delay class (190 fires x 250 classes: 54 us, launched 46), an event above
 // kSmallEven where the blocks have more targets than threads (8,000 neurons: 4,000
-// events 31 us, launched 33, 7,000 43 and 38; 16,000: 32 and 32, 44 and 35).  A
+// events 31 us, launched 33, 6,000 39 and 37, 7,000 43 and 38; 16,000: 4,000 both
+// 32, 7,000 44 and 35).  A
 // quiet tick gains kSmallGain (1,000 neurons: 500 events 18 us, launched 28;
 // 1,452 neurons, fires of 650 events: 43 and 49) less N / 4 and, as the launched
 // kernels count the fires by class, kSmallClassGain per class more.  Once a
@@ -434,7 +435,7 @@ constexpr uint32_t kSmallSlots = 1024;
 // take over: rare heavy ticks do not do that, a layer of 100 output neurons with
 // 30,000 inputs each that fires all the time (4,700 us a tick here, 126 launched)
 // does in a few.
-constexpr uint32_t kSmallRow = 2, kSmallCopy = 16, kSmallClass10 = 5, kSmallEvent = 4, kSmallEven = 4096;
+constexpr uint32_t kSmallRow = 2, kSmallCopy = 16, kSmallClass10 = 5, kSmallEvent = 6, kSmallEven = 4096;
 constexpr uint32_t kSmallGain = 12000, kSmallClassGain = 32;
 constexpr uint32_t kSmallDebt = 1u << 20;
 static_assert(sizeof(TickState::small_debt) == kSmallBlocks * sizeof(uint32_t), "a block's debt");
